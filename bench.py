@@ -119,6 +119,9 @@ SOLVER = dict(method=14, lam=50.0, theta=0.33, tau=0.25, alpha_proj=60.0, lambda
 # duhat(2),uproj(2),X1,Y1,Z1 = 7; B reads duhat(2),p(4),X1(3),sk(2),u,v,uproj(2)
 # = 15, writes p(4),X,Y,Z,sk(2) = 9.
 ALG_BYTES = {"recon_a": 25 * 4, "recon_b": 24 * 4}
+# the batch's large levels (k_batch_a2 / k_batch_b2): A also updates and writes
+# sk (9 written), B reads duhat(2),p(4),X1(3) and writes p(4),X,Y,Z
+ALG_BYTES_BATCH = {"recon_a": 27 * 4, "recon_b": 16 * 4}
 # compulsory bytes of one inner iteration per pixel (both kernels together)
 ITER_BYTES = 31 * 4
 L2_FLUSH_BYTES = 512 << 20
@@ -1822,8 +1825,9 @@ def roofline_of(ms, px, batched=False):
     """Roofline entry of the dominant level-0 kernel from per-launch times
     (`px` pixels per launch; `batched`: the batched solver's kernels)."""
     names = ["recon_a", "recon_b"]
+    alg = ALG_BYTES_BATCH if batched else ALG_BYTES
     dom = 0 if ms[0] >= ms[1] else 1
-    achieved = ALG_BYTES[names[dom]] * px / (ms[dom] * 1e-3) / 1e9
+    achieved = alg[names[dom]] * px / (ms[dom] * 1e-3) / 1e9
     peak, peak_kind = load_peaks()
     traffic = None
     tpath = os.path.join(ROOT, "profiles",
@@ -1835,13 +1839,13 @@ def roofline_of(ms, px, batched=False):
         # the capture's DRAM bytes per launch scaled by pixels (traffic grows
         # with the pixel count: one pass over every field per launch)
         traffic = None if per is None else per * px / tr["pixels"]
-    return {"bound": "hbm", "kernel": ("k_batch<OpReconA>" if dom == 0 else "k_batch<OpReconB>")
+    return {"bound": "hbm", "kernel": ("k_batch_a2" if dom == 0 else "k_batch_b2")
             if batched else ("k_recon_a" if dom == 0 else "k_recon_b"),
             "achieved": achieved, "peak": peak,
             "peak_kind": peak_kind, "unit": "GB/s", "frac": achieved / peak, "traffic": traffic,
-            "alg_bytes_per_launch": ALG_BYTES[names[dom]] * px,
+            "alg_bytes_per_launch": alg[names[dom]] * px,
             "launch_ms": {names[0]: ms[0], names[1]: ms[1]},
-            "frac_each": {names[k]: ALG_BYTES[names[k]] * px / (ms[k] * 1e-3) / 1e9 / peak
+            "frac_each": {names[k]: alg[names[k]] * px / (ms[k] * 1e-3) / 1e9 / peak
                           for k in range(2)},
             "iteration": iteration_roofline(ms, px, peak),
             "issue": issue_roofline(ms, px, tr.get("warp_instructions_per_32px")

@@ -31,6 +31,7 @@
 #include "rf_nvtx.h"
 #include "rf_kernels.cuh"
 #include "rf_ops.cuh"
+#include "rf_pair.cuh"
 
 using namespace rf;
 
@@ -42,6 +43,13 @@ constexpr int BX = 32;
 constexpr int BY = 8;
 constexpr int kMaxTile = 256;
 constexpr int kMaxLevels = 16;
+// Levels of at least this many pixels (all pairs together) run the two-pixel
+// half-steps: below, a launch is shorter than the chain of one pixel's
+// instructions and the one-pixel kernels' is the shorter chain.  Measured, 2 / 4
+// learned 720p pairs (levels 0.46 and 1.84 / 0.92 and 3.7 million pixels): from
+// 0.4 million 2.00 / 3.21 ms, from 1.5 million 2.06 / 3.53, never 2.13 / 3.65;
+// from 0.05 million the mixed batch loses 1%.
+constexpr long long kPairMinPixels = 400000;
 
 struct BatchPair {
     LevelDims dims[kMaxLevels];
@@ -122,6 +130,61 @@ __global__ void __launch_bounds__(kMaxTile) k_batch_rows2(BatchCtx ctx, int leve
     const int ix = t.x0 + (int)threadIdx.x, iy = t.y0 + 2 * (int)threadIdx.y;
     if (ix >= d.w || iy >= d.h) return;
     op.two(t, d, ix, iy);
+}
+
+// The two-pixel half-steps (rf_pair.cuh): one block = one tile of kPairW x
+// kPairRows pixels of the level's pair-tile table, a warp per row.
+//
+// A is bound by instruction issue and the latency of its first loads (461
+// warp instructions per 32 pixels at 54% issue, 20 warps per SM; DRAM at 60%),
+// B by the min / max pipe and its copies (346 at 69%): per launch of 64 720p
+// pairs (58 982 400 pixels) 1.28 and 0.79 ms against 1.40 and 1.11 ms for the
+// one-pixel kernels, 108 and 64 bytes per pixel.  Measured on 32 learned 720p
+// pairs (whole call, one-pixel kernels 24.8 ms): 5 / 10 blocks per SM of 4 rows
+// 20.4 ms; 8 rows 23.5 (waits at the block's barrier), 2 rows 21.3; A at 4
+// blocks (128 registers) 22.5, at 6 (80, spilling) 20.6; A from staged copies
+// as B 21.4 (573 instructions); several rows per warp 20.6 .. 22.8; L2
+// prefetch of half a wave ahead 20.4, none 21.1, one wave 20.5.
+constexpr int kPairThreads = 32 * kPairRows;
+constexpr int kPairBlocksA = 5, kPairBlocksB = 10;
+
+// Ask L2 for what A reads of the tile ctx.prefetch blocks on: a lane per
+// 128-byte line of the warp's row (a few instructions per warp; a request per
+// pixel and field cost the one-pixel A more than it saved).
+__device__ __forceinline__ void prefetch_rows(const BatchCtx& ctx, int level, const ReconFields& f) {
+    const int b = (int)blockIdx.x + ctx.prefetch;
+    if (ctx.prefetch <= 0 || b >= (int)gridDim.x) return;
+    const TileEntry t = ctx.tiles[b];
+    const LevelDims d = ctx.pairs[t.pair].dims[level];
+    const int y = t.y0 + (int)(threadIdx.x >> 5);
+    if (y >= d.h) return;
+    for (int k = threadIdx.x & 31; k < 2 * kReconReads; k += 32) {
+        const int x = t.x0 + 32 * (k & 1);
+        if (x < d.w) prefetch_l2(recon_read(f, k >> 1) + t.off + x + y * d.s);
+    }
+}
+
+__global__ void __launch_bounds__(kPairThreads, kPairBlocksA)
+    k_batch_a2(BatchCtx ctx, int level, const __grid_constant__ ReconFields f,
+               const __grid_constant__ Weights wt, int first, int ucb) {
+    __shared__ float2 sc[kCount];
+    const TileEntry t = ctx.tiles[blockIdx.x];
+    const LevelDims d = ctx.pairs[t.pair].dims[level];
+    const LevelConsts* lc = ctx.consts + t.pair * ctx.L + level;
+    pair_consts(lc, wt, sc, threadIdx.x, kPairThreads);
+    if (!first) prefetch_rows(ctx, level, f);
+    const int x = t.x0 + 2 * (int)(threadIdx.x & 31), y = t.y0 + (int)(threadIdx.x >> 5);
+    recon_a_pair<0>(f, lc, sc, wt, d, t.off, x, y, x < d.w && y < d.h, first != 0, ucb != 0);
+}
+
+template <bool LAST>
+__global__ void __launch_bounds__(kPairThreads, kPairBlocksB)
+    k_batch_b2(BatchCtx ctx, int level, const __grid_constant__ ReconFields f,
+               const __grid_constant__ Weights wt, int first) {
+    __shared__ __align__(16) float sm[StageB::FLOATS];
+    const TileEntry t = ctx.tiles[blockIdx.x];
+    recon_b_tile<LAST>(f, wt, sm, ctx.pairs[t.pair].dims[level], t.off, t.x0, t.y0,
+                                  first != 0);
 }
 
 // Level-0 row copies (the staging gathers): one warp per row of a pair's
@@ -502,6 +565,10 @@ struct rf_batch {
     size_t tiles_cap = 0;                 // entries allocated at d_tiles
     std::vector<size_t> tile_start;       // first entry of each level
     std::vector<int> prefix;  // [level][n + 1] tile prefix sums
+    // the two-pixel half-steps' tile tables, behind the others: first entry
+    // and blocks of each level; 0 blocks: the level runs the one-pixel kernels
+    std::vector<size_t> pair_start;
+    std::vector<int> pair_blocks;
     std::vector<int> tile_w, tile_h;  // tile shape of each level
     LevelConsts* d_consts = nullptr;
     LevelConsts* h_consts = nullptr;
@@ -578,6 +645,23 @@ cudaError_t fill_tiles(rf_batch* b) {
             b->prefix[l * (b->n + 1) + i + 1] = b->prefix[l * (b->n + 1) + i] + nx * ny;
         }
     }
+    b->pair_start.assign(b->L, 0);
+    b->pair_blocks.assign(b->L, 0);
+    for (int l = 0; l < b->L; l++) {
+        b->pair_start[l] = tab.size();
+        bool fits = pair_weights(solver_weights(&b->p));
+        long long px = 0;
+        for (int i = 0; i < b->n; i++) {
+            fits = fits && pair_stride(b->dims[i][l]);
+            px += (long long)b->dims[i][l].w * b->dims[i][l].h;
+        }
+        if (!fits || px < kPairMinPixels) continue;
+        for (int i = 0; i < b->n; i++)
+            for (int y = 0; y < b->dims[i][l].h; y += kPairRows)
+                for (int x = 0; x < b->dims[i][l].w; x += kPairW)
+                    tab.push_back(TileEntry{i, x, y, (int)b->base_off[i]});
+        b->pair_blocks[l] = (int)(tab.size() - b->pair_start[l]);
+    }
     if (tab.size() > b->tiles_cap) {
         if (b->d_tiles) cudaFree(b->d_tiles);
         b->d_tiles = nullptr;
@@ -630,6 +714,30 @@ int launch_op(rf_batch* b, int level, const Op& op) {
     if (tiles <= 0) return 0;
     const dim3 block(b->tile_w[level], b->tile_h[level]);
     k_batch<Op><<<tiles, block, 0, b->stream>>>(ctx_of(b, level), level, op);
+    b->enq++;
+    return rf::launch_status();
+}
+
+// A (data step) and B (dual step) of an inner iteration over the level's
+// pixel pairs (rf_pair.cuh); `last`: the warp's last B
+int launch_a2(rf_batch* b, int level, const ReconFields& f, const Weights& wt, bool first,
+              bool ucb) {
+    BatchCtx c = ctx_of(b, level);
+    c.tiles = b->d_tiles + b->pair_start[level];
+    c.prefetch = b->prefetch / 16 * kPairBlocksA / 2;  // half a wave of these blocks
+    k_batch_a2<<<b->pair_blocks[level], kPairThreads, 0, b->stream>>>(c, level, f, wt, first, ucb);
+    b->enq++;
+    return rf::launch_status();
+}
+
+int launch_b2(rf_batch* b, int level, const ReconFields& f, const Weights& wt, bool first,
+              bool last) {
+    BatchCtx c = ctx_of(b, level);
+    c.tiles = b->d_tiles + b->pair_start[level];
+    if (last)
+        k_batch_b2<true><<<b->pair_blocks[level], kPairThreads, 0, b->stream>>>(c, level, f, wt, first);
+    else
+        k_batch_b2<false><<<b->pair_blocks[level], kPairThreads, 0, b->stream>>>(c, level, f, wt, first);
     b->enq++;
     return rf::launch_status();
 }
@@ -785,7 +893,11 @@ rf_status enqueue_batch(rf_batch* b, int kind) {
             }
             for (int iter = 0; iter < n_iters && !(recon && b->split > 0); iter++) {
                 const int first = iter == 0;
-                if (recon) {
+                if (recon && b->pair_blocks[level] > 0) {
+                    BL(launch_a2(b, level, r, wt, first, ucb));
+                    BL(launch_b2(b, level, r, wt, first, iter + 1 == n_iters));
+                    ucb = false;
+                } else if (recon) {
                     BL(launch_op(b, level, OpReconA{r, wt, first, ucb ? 1 : 0}));
                     BL(launch_op(b, level, OpReconB{r, wt, first}));
                     ucb = false;
@@ -1200,8 +1312,12 @@ rf_status rf_batch_profile_level(rf_batch* b, int level, int n_iters, float* ms)
         BC(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
         int bad = 0;
         for (int i = 0; i < n_iters && !bad; i++)
-            bad = k == 0 ? launch_op(b, level, OpReconA{r, wt, 0, 0})
-                         : launch_op(b, level, OpReconB{r, wt, 0});
+            if (b->pair_blocks[level] > 0)
+                bad = k == 0 ? launch_a2(b, level, r, wt, false, false)
+                             : launch_b2(b, level, r, wt, false, false);
+            else
+                bad = k == 0 ? launch_op(b, level, OpReconA{r, wt, 0, 0})
+                             : launch_op(b, level, OpReconB{r, wt, 0});
         cudaError_t ce = cudaStreamEndCapture(b->stream, &g);
         if (bad || ce != cudaSuccess) {
             if (g) cudaGraphDestroy(g);

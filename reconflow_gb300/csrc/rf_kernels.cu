@@ -25,6 +25,7 @@
 #include "rf_alloc.h"
 #include "rf_kernels.cuh"
 #include "rf_ops.cuh"
+#include "rf_pair.cuh"
 
 namespace {
 
@@ -223,6 +224,28 @@ __global__ void __launch_bounds__(BX* BY, RF_MINB_B) k_recon_b(ReconFields f, We
     int iy = blockIdx.y * blockDim.y + threadIdx.y;
     if (ix >= d.w || iy >= d.h) return;
     recon_b_px(f, wt, d, ix, iy, first);
+}
+
+// The two-pixel half-steps (rf_pair.cuh; registers and tile as in the batch)
+template <int PRIOR>
+__global__ void __launch_bounds__(32 * kPairRows, 5)
+    k_recon_a2(const __grid_constant__ ReconFields f, const LevelConsts* __restrict__ lcp,
+               const __grid_constant__ Weights wt, LevelDims d, int first, int uc_from_buffer) {
+    __shared__ float2 sc[kCount];
+    const int x = 2 * (int)(blockIdx.x * 32 + (threadIdx.x & 31));
+    const int y = blockIdx.y * kPairRows + (threadIdx.x >> 5);
+    pair_consts(lcp, wt, sc, threadIdx.x, 32 * kPairRows);
+    recon_a_pair<PRIOR>(f, lcp, sc, wt, d, 0, x, y, x < d.w && y < d.h, first != 0,
+                        uc_from_buffer != 0);
+}
+
+template <bool LAST>
+__global__ void __launch_bounds__(32 * kPairRows, 10)
+    k_recon_b2(const __grid_constant__ ReconFields f, const __grid_constant__ Weights wt,
+               LevelDims d, int first) {
+    __shared__ __align__(16) float sm[StageB::FLOATS];
+    recon_b_tile<LAST>(f, wt, sm, d, 0, blockIdx.x * kPairW, blockIdx.y * kPairRows,
+                                  first != 0);
 }
 
 // ---------------------------------------------------------------------------
@@ -682,6 +705,39 @@ int launch_recon_b(const ReconFields& f, const Weights& wt, LevelDims d, bool fi
                    cudaStream_t st, dim3 b) {
     dim3 g((d.w + b.x - 1) / b.x, (d.h + b.y - 1) / b.y);
     return launch_pdl(k_recon_b, g, b, st, f, wt, d, first ? 1 : 0);
+}
+
+bool pair_weights(const Weights& wt) {
+    // divisors in the range of the packed quotients, the dual step's not below 1
+    auto divisor = [](float a) { return a >= 0x1p-50f && a <= 0x1p120f; };
+    return divisor(wt.A) && divisor(wt.proj_den) && divisor(wt.lambdams) && wt.fac >= 0.0f && wt.alpha_tv >= 0.0f &&
+           wt.alpha_proj >= 0.0f && wt.alpha_fn >= 0.0f;
+}
+
+bool use_pairs(const Weights& wt, LevelDims d) {
+    // A 720p pair's level 0 (0.92 million pixels, under two waves of blocks, its
+    // state in L2) takes as long either way (37.2 against 37.0 ms a solve), a
+    // 1080p pair's (2.1 million) is faster by pairs (67.5 against 73.0 ms).
+    constexpr long long kMinPixels = 1500000;
+    return pair_stride(d) && (long long)d.w * d.h >= kMinPixels && pair_weights(wt);
+}
+
+int launch_recon_a2(const ReconFields& f, const LevelConsts* lc, const Weights& wt, LevelDims d,
+                    bool first, bool uc_from_buffer, int prior, cudaStream_t st) {
+    const dim3 g((d.w + kPairW - 1) / kPairW, (d.h + kPairRows - 1) / kPairRows);
+    const int n = 32 * kPairRows, fi = first ? 1 : 0, ub = uc_from_buffer ? 1 : 0;
+    if (prior == 1) k_recon_a2<1><<<g, n, 0, st>>>(f, lc, wt, d, fi, ub);
+    else if (prior == 2) k_recon_a2<2><<<g, n, 0, st>>>(f, lc, wt, d, fi, ub);
+    else k_recon_a2<0><<<g, n, 0, st>>>(f, lc, wt, d, fi, ub);
+    return check_launch();
+}
+
+int launch_recon_b2(const ReconFields& f, const Weights& wt, LevelDims d, bool first, bool last,
+                    cudaStream_t st) {
+    const dim3 g((d.w + kPairW - 1) / kPairW, (d.h + kPairRows - 1) / kPairRows);
+    if (last) k_recon_b2<true><<<g, 32 * kPairRows, 0, st>>>(f, wt, d, first ? 1 : 0);
+    else k_recon_b2<false><<<g, 32 * kPairRows, 0, st>>>(f, wt, d, first ? 1 : 0);
+    return check_launch();
 }
 
 #ifdef RF_BOUNDS_CHECK

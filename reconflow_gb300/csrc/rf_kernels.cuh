@@ -146,6 +146,15 @@ int launch_recon_a(const ReconFields& f, const LevelConsts* lc, const Weights& w
                    dim3 block = dim3(32, 8));
 int launch_recon_b(const ReconFields& f, const Weights& wt, LevelDims d, bool first,
                    cudaStream_t st, dim3 block = dim3(32, 8));
+// The two-pixel half-steps (rf_pair.cuh) of levels where use_pairs(): A, and
+// B (`last`: a warp's last).  The multiplier update belongs to the A that
+// follows, so the two kinds of half-step do not mix within a warp.
+bool pair_weights(const Weights& wt);  // whether the weights fit them
+bool use_pairs(const Weights& wt, LevelDims d);
+int launch_recon_a2(const ReconFields& f, const LevelConsts* lc, const Weights& wt, LevelDims d,
+                    bool first, bool uc_from_buffer, int prior, cudaStream_t st);
+int launch_recon_b2(const ReconFields& f, const Weights& wt, LevelDims d, bool first, bool last,
+                    cudaStream_t st);
 int launch_plain_data(float* duhat, float* dvhat, const float* pu1, const float* pu2,
                       const float* pv1, const float* pv2, const float* Ix, const float* Iy,
                       const float* Iz, const Weights& wt, LevelDims d, bool first,

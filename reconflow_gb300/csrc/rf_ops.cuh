@@ -31,8 +31,10 @@ __device__ __forceinline__ float deriv5(float m2, float m1, float p1, float p2) 
 }
 
 // `base`: element of the level's pixel (0, 0) in every field (0 for a
-// single pair; a pair's offset in the batched solver's planes).
-template <int PRIOR>
+// single pair; a pair's offset in the batched solver's planes).  SK: the
+// multiplier update of the previous iteration's dual step (solveUcSk.cu:94-95)
+// is made here first (rf_pair.cuh).
+template <int PRIOR, bool SK = false>
 __device__ __forceinline__ void recon_a_px(const ReconFields& f, const LevelConsts& c,
                                            const Weights& wt, LevelDims d, int ix, int iy,
                                            int first, int uc_from_buffer, int base = 0) {
@@ -103,6 +105,11 @@ __device__ __forceinline__ void recon_a_px(const ReconFields& f, const LevelCons
         if (PRIOR == 2) mk = RF_AT(f, mask, pos);
     }
 
+    if (SK && !first) {
+        sku = sku + u + duhat - uproj;
+        skv = skv + v + dvhat - vproj;
+    }
+
     // --- data step (solveReconDataL1.cu:24-100) ---
     float A, dusub, dvsub;
     if (PRIOR == 0) {
@@ -137,6 +144,10 @@ __device__ __forceinline__ void recon_a_px(const ReconFields& f, const LevelCons
     float Xo, Yo, Zo;
     solve3d_pixel(c, uproj1, vproj1, ix, iy, Xn, Yn, Zn, wt.lambdaf, wt.lambdams, Xo, Yo, Zo);
 
+    if (SK && !first) {
+        RF_AT(f, sku, pos) = sku;
+        RF_AT(f, skv, pos) = skv;
+    }
     RF_AT(f, duhat, pos) = duhat1;
     RF_AT(f, dvhat, pos) = dvhat1;
     RF_AT(f, uproj, pos) = uproj1;

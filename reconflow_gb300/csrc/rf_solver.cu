@@ -355,6 +355,12 @@ rf_status enqueue_recon(rf_handle* h, float** res_u, float** res_v, bool warm = 
                 uc_in_buffer = false;
             }
             for (int iter = 0; iter < n_iters && !use_cluster_at(h, d); iter++) {
+                if (use_pairs(wt, d)) {
+                    RF_LAUNCH(launch_recon_a2(f, lc, wt, d, iter == 0, uc_in_buffer, prior, st));
+                    RF_LAUNCH(launch_recon_b2(f, wt, d, iter == 0, iter + 1 == n_iters, st));
+                    uc_in_buffer = false;
+                    continue;
+                }
                 const dim3 tile(h->tile_w[level], h->tile_h[level]);
                 RF_LAUNCH(launch_recon_a(f, lc, wt, d, iter == 0, uc_in_buffer, prior, st, tile));
                 RF_LAUNCH(launch_recon_b(f, wt, d, iter == 0, st, tile));
@@ -1055,7 +1061,10 @@ rf_status rf_profile_iterations(rf_handle* h, int level, int n_iters, float* ms)
         RF_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
         int bad = 0;
         for (int i = 0; i < n_iters && !bad; i++) {
-            if (recon)
+            if (recon && use_pairs(wt, d))
+                bad = k == 0 ? launch_recon_a2(f, h->d_consts + level, wt, d, false, false, prior, st)
+                             : launch_recon_b2(f, wt, d, false, false, st);
+            else if (recon)
                 bad = k == 0 ? launch_recon_a(f, h->d_consts + level, wt, d, false, false, prior, st,
                                               dim3(h->tile_w[level], h->tile_h[level]))
                              : launch_recon_b(f, wt, d, false, st,
