@@ -51,87 +51,80 @@ struct Shape {
     int B, H, W, C;  // NHWC
 };
 
-// ---- tcgen05 GEMM operands: 8 consecutive K elements of one row ----------
+// ---- tcgen05 GEMM operands: 8 consecutive K elements of one row (rf_tc.cuh) ----
 __device__ __forceinline__ uint4 pack8(const bf16 (&v)[8]) {
     return make_uint4(pack2(v[0], v[1]), pack2(v[2], v[3]), pack2(v[4], v[5]), pack2(v[6], v[7]));
 }
 
 // forward A: im2col row of output pixel m, k = (ky*3 + kx)*Cin + ci (Cin % 8 == 0)
 struct TcConvIn {
-    static constexpr bool kAsync = true;
     const bf16* x;
     int B, H, W, C, Ho, Wo, stride;
+    struct Row {
+        long long off;  // element of tap (0, 0), channel 0 (outside the image at its edges)
+        int y, x;       // that tap's pixel; y < -2: no row
+    };
+    struct Pos {
+        int off, ky, kx;
+    };
     __device__ const void* base() const { return x; }
-    __device__ const void* src(int m, int k) const {
-        int ci = k % C, t = k / C, kx = t % 3, ky = t / 3;
-        int xo = m % Wo, r = m / Wo, yo = r % Ho, b = r / Ho;
-        int y = yo * stride + ky - 1, xx = xo * stride + kx - 1;
-        if (y < 0 || y >= H || xx < 0 || xx >= W) return nullptr;
-        return x + (((size_t)b * H + y) * W + xx) * C + ci;
+    __device__ Row row(int m, int M) const {
+        const int xo = m % Wo, r = m / Wo, yo = r % Ho, b = r / Ho;
+        const int y = yo * stride - 1, xx = xo * stride - 1;
+        return Row{(((long long)b * H + y) * W + xx) * C, m < M ? y : -8, xx};
+    }
+    __device__ Pos kpos(int k) const {
+        const int ci = k % C, t = k / C, kx = t % 3, ky = t / 3;
+        return Pos{(ky * W + kx) * C + ci, ky, kx};
+    }
+    __device__ const void* at(const Row& r, const Pos& k) const {
+        if ((unsigned)(r.y + k.ky) >= (unsigned)H || (unsigned)(r.x + k.kx) >= (unsigned)W)
+            return nullptr;
+        return x + r.off + k.off;
     }
 };
 
 // K-major matrix rows: w[n][k], K % 8 == 0
 struct TcRows {
-    static constexpr bool kAsync = true;
     const bf16* w;
     int K;
+    typedef const bf16* Row;
     __device__ const void* base() const { return w; }
-    __device__ const void* src(int n, int k) const { return w + (size_t)n * K + k; }
+    __device__ Row row(int n, int N) const { return n < N ? w + (size_t)n * K : nullptr; }
+    __device__ int kpos(int k) const { return k; }
+    __device__ const void* at(Row r, int k) const { return r ? r + k : nullptr; }
 };
 
 // input-gradient A: input pixel m, k = (ky*3 + kx)*Cout + co -> dy at the
 // output pixel that tap (ky, kx) of m feeds (Cout % 8 == 0)
 struct TcDataGradA {
-    static constexpr bool kAsync = true;
     const bf16* dy;
     int H, W, Ho, Wo, Cout, stride;
+    struct Row {
+        int img, y, x;  // the image's first output row; input pixel + 1 (y < 0: no row)
+    };
+    struct Pos {
+        int co, ky, kx;
+    };
     __device__ const void* base() const { return dy; }
-    __device__ const void* src(int m, int k) const {
-        int co = k % Cout, t = k / Cout, kx = t % 3, ky = t / 3;
-        int xx = m % W, r = m / W, y = r % H, b = r / H;
-        int ty = y + 1 - ky, tx = xx + 1 - kx;
-        if (ty < 0 || tx < 0 || ty % stride || tx % stride) return nullptr;
-        int yo = ty / stride, xo = tx / stride;
-        if (yo >= Ho || xo >= Wo) return nullptr;
-        return dy + (((size_t)b * Ho + yo) * Wo + xo) * Cout + co;
+    __device__ Row row(int m, int M) const {
+        const int xx = m % W, r = m / W, y = r % H, b = r / H;
+        return Row{b * Ho, m < M ? y + 1 : -8, xx + 1};
     }
-};
-
-// weight-gradient A: row m = (ky*3 + kx)*Cin + ci of im2col^T, k = output pixel
-struct TcWGradA {
-    static constexpr bool kAsync = false;
-    const bf16* x;
-    int H, W, C, Ho, Wo, stride;
-    __device__ uint4 operator()(int m, int k, int k_end) const {
-        int ci = m % C, t = m / C, kx = t % 3, ky = t / 3;
-        bf16 v[8];
-#pragma unroll
-        for (int e = 0; e < 8; e++) {
-            int p = k + e;
-            v[e] = __float2bfloat16(0.f);
-            if (p < k_end) {
-                int xo = p % Wo, r = p / Wo, yo = r % Ho, b = r / Ho;
-                int y = yo * stride + ky - 1, xx = xo * stride + kx - 1;
-                if (y >= 0 && y < H && xx >= 0 && xx < W)
-                    v[e] = x[(((size_t)b * H + y) * W + xx) * C + ci];
-            }
+    __device__ Pos kpos(int k) const {
+        const int co = k % Cout, t = k / Cout, kx = t % 3, ky = t / 3;
+        return Pos{co, ky, kx};
+    }
+    __device__ const void* at(const Row& r, const Pos& k) const {
+        int ty = r.y - k.ky, tx = r.x - k.kx;
+        if (ty < 0 || tx < 0) return nullptr;
+        if (stride == 2) {
+            if ((ty | tx) & 1) return nullptr;
+            ty >>= 1;
+            tx >>= 1;
         }
-        return pack8(v);
-    }
-};
-
-// weight-gradient B: row n = co, k = output pixel -> dy[pixel][co]
-struct TcWGradB {
-    static constexpr bool kAsync = false;
-    const bf16* dy;
-    int Cout;
-    __device__ uint4 operator()(int n, int k, int k_end) const {
-        bf16 v[8];
-#pragma unroll
-        for (int e = 0; e < 8; e++)
-            v[e] = k + e < k_end ? dy[(size_t)(k + e) * Cout + n] : __float2bfloat16(0.f);
-        return pack8(v);
+        if (ty >= Ho || tx >= Wo) return nullptr;
+        return dy + ((size_t)(r.img + ty) * Wo + tx) * Cout + k.co;
     }
 };
 
@@ -153,26 +146,45 @@ __global__ void k_transpose_w(const bf16* w, int cin, int cout, bf16* wt) {
     wt[((size_t)ci * 9 + t) * cout + co] = w[i];
 }
 
+__device__ __forceinline__ void store8(float* p, const float (&v)[8]) {
+    reinterpret_cast<float4*>(p)[0] = make_float4(v[0], v[1], v[2], v[3]);
+    reinterpret_cast<float4*>(p)[1] = make_float4(v[4], v[5], v[6], v[7]);
+}
+__device__ __forceinline__ uint4 pack8(const float (&v)[8]) {
+    bf16 h[8];
+#pragma unroll
+    for (int e = 0; e < 8; e++) h[e] = __float2bfloat16(v[e]);
+    return pack8(h);
+}
+// + bias, optional ReLU
+__device__ __forceinline__ void bias_relu(const float* bias, int relu, const float (&v)[8],
+                                          float (&o)[8]) {
+#pragma unroll
+    for (int e = 0; e < 8; e++) {
+        const float t = v[e] + bias[e];
+        o[e] = relu ? fmaxf(t, 0.f) : t;
+    }
+}
+
 // forward epilogue: + bias, optional ReLU; BF16 activation and/or FP32 copy
 struct ConvOut {
     const float* bias;
     bf16* y;
     float* yf;
-    int M, Cout, relu;
-    __device__ void operator()(int, int m, int n, float v) const {
-        if (m >= M || n >= Cout) return;
-        v += bias[n];
-        if (relu) v = fmaxf(v, 0.f);
-        if (y) y[(size_t)m * Cout + n] = __float2bfloat16(v);
-        if (yf) yf[(size_t)m * Cout + n] = v;
+    int Cout, relu;
+    __device__ void operator()(int m, int n, const float (&v)[8]) const {
+        float o[8];
+        bias_relu(bias + n, relu, v, o);
+        if (y) *(uint4*)(y + (size_t)m * Cout + n) = pack8(o);
+        if (yf) store8(yf + (size_t)m * Cout + n, o);
     }
 };
 
 struct StoreF32 {
     float* out;
-    int M, N;
-    __device__ void operator()(int, int m, int n, float v) const {
-        if (m < M && n < N) out[(size_t)m * N + n] = v;
+    int N;
+    __device__ void operator()(int m, int n, const float (&v)[8]) const {
+        store8(out + (size_t)m * N + n, v);
     }
 };
 
@@ -209,61 +221,89 @@ __global__ void __launch_bounds__(kBiasThreads) k_bias_partial(const float* dy, 
     }
 }
 
+// The elementwise passes take 4 (FP32) or 8 (BF16 copies) channels per thread:
+// every channel count is a multiple of 8, and one element per thread, with its
+// index divisions, ran at 0.3 - 0.4 of the HBM rate.
 __global__ void k_f32_to_bf16(const float* a, bf16* b, size_t n) {
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) b[i] = __float2bfloat16(a[i]);
 }
 
-// dy = g * [activation > 0] (ReLU backward), in place on g, and a BF16 copy
-__global__ void k_relu_grad(float* g, const bf16* act, bf16* gb, size_t n) {
-    size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    float v = __bfloat162float(act[i]) > 0.f ? g[i] : 0.f;
-    g[i] = v;
-    gb[i] = __float2bfloat16(v);
+__device__ __forceinline__ uint2 bf16x4(float4 v) {
+    return make_uint2(pack2(__float2bfloat16(v.x), __float2bfloat16(v.y)),
+                      pack2(__float2bfloat16(v.z), __float2bfloat16(v.w)));
+}
+__device__ __forceinline__ bool bf16_positive(unsigned bits) {  // > 0 (not NaN)
+    bits &= 0xFFFFu;
+    return bits != 0 && bits <= 0x7F80u;
 }
 
-// cat = [nearest 2x upsample of a (Ha x Wa x Ca), b (H x W x Cb)]
+// dy = (g + add) * [activation > 0] (ReLU backward; `add` may be null), in
+// place on g, and a BF16 copy; n a multiple of 4
+__global__ void k_relu_grad(float* g, const float* add, const bf16* act, bf16* gb, size_t n) {
+    const size_t i = 4 * ((size_t)blockIdx.x * blockDim.x + threadIdx.x);
+    if (i >= n) return;
+    float4 v = *(const float4*)(g + i);
+    if (add) {
+        const float4 t = *(const float4*)(add + i);
+        v.x += t.x;
+        v.y += t.y;
+        v.z += t.z;
+        v.w += t.w;
+    }
+    const uint2 a = *(const uint2*)(act + i);
+    if (!bf16_positive(a.x)) v.x = 0.f;
+    if (!bf16_positive(a.x >> 16)) v.y = 0.f;
+    if (!bf16_positive(a.y)) v.z = 0.f;
+    if (!bf16_positive(a.y >> 16)) v.w = 0.f;
+    *(float4*)(g + i) = v;
+    *(uint2*)(gb + i) = bf16x4(v);
+}
+
+// cat = [nearest 2x upsample of a (Ha x Wa x Ca), b (H x W x Cb)], 8 channels
+// per thread
 __global__ void k_concat_up(const bf16* a, int Ha, int Wa, int Ca, const bf16* b, int Cb,
                             int Bn, int H, int W, bf16* cat) {
-    size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    size_t n = (size_t)Bn * H * W * (Ca + Cb);
-    if (i >= n) return;
-    int C = Ca + Cb;
-    int c = i % C;
-    size_t p = i / C;
-    int x = p % W, r = p / W, y = r % H, bb = r / H;
-    if (c < Ca)
-        cat[i] = a[(((size_t)bb * Ha + y / 2) * Wa + x / 2) * Ca + c];
-    else
-        cat[i] = b[p * Cb + (c - Ca)];
+    const int C = Ca + Cb, G = C / 8;
+    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= (size_t)Bn * H * W * G) return;
+    const int c = (int)(i % G) * 8;
+    const size_t p = i / G;
+    const int x = (int)(p % W), r = (int)(p / W), y = r % H, bb = r / H;
+    *(uint4*)(cat + p * C + c) =
+        c < Ca ? *(const uint4*)(a + (((size_t)bb * Ha + y / 2) * Wa + x / 2) * Ca + c)
+               : *(const uint4*)(b + p * Cb + (c - Ca));
 }
 
-// split the concat gradient: d_a (half resolution) += sum of its 2x2
-// children; d_b (+)= the rest.  accumulate != 0 adds to the existing values.
+// split the concat gradient: d_a (half resolution) = sum of its 2x2 children
+// (in row order), d_b = the rest; 4 channels per thread
 __global__ void k_concat_up_grad(const float* dcat, int Ha, int Wa, int Ca, int Cb, int Bn,
-                                 int H, int W, float* da, float* db, int accumulate_b) {
-    size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    size_t na = (size_t)Bn * Ha * Wa * Ca;
-    size_t nb = (size_t)Bn * H * W * Cb;
-    int C = Ca + Cb;
+                                 int H, int W, float* da, float* db) {
+    const size_t i = 4 * ((size_t)blockIdx.x * blockDim.x + threadIdx.x);
+    const size_t na = (size_t)Bn * Ha * Wa * Ca;
+    const size_t nb = (size_t)Bn * H * W * Cb;
+    const int C = Ca + Cb;
     if (i < na) {
-        int c = i % Ca;
-        size_t p = i / Ca;
-        int x = p % Wa, r = p / Wa, y = r % Ha, bb = r / Ha;
-        float s = 0.f;
+        const int c = (int)(i % Ca);
+        const size_t p = i / Ca;
+        const int x = (int)(p % Wa), r = (int)(p / Wa), y = r % Ha, bb = r / Ha;
+        float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
         for (int dy = 0; dy < 2; dy++)
             for (int dx = 0; dx < 2; dx++) {
-                int yy = 2 * y + dy, xx = 2 * x + dx;
-                if (yy < H && xx < W) s += dcat[(((size_t)bb * H + yy) * W + xx) * C + c];
+                const int yy = 2 * y + dy, xx = 2 * x + dx;
+                if (yy < H && xx < W) {
+                    const float4 t = *(const float4*)(dcat + (((size_t)bb * H + yy) * W + xx) * C + c);
+                    s.x += t.x;
+                    s.y += t.y;
+                    s.z += t.z;
+                    s.w += t.w;
+                }
             }
-        da[i] += s;
+        *(float4*)(da + i) = s;
     }
     if (i < nb) {
-        int c = i % Cb;
-        size_t p = i / Cb;
-        float v = dcat[p * C + Ca + c];
-        db[i] = accumulate_b ? db[i] + v : v;
+        const int c = (int)(i % Cb);
+        *(float4*)(db + i) = *(const float4*)(dcat + i / Cb * C + Ca + c);
     }
 }
 
@@ -302,11 +342,6 @@ __global__ void k_adam(float* w, const float* g, float* m, float* v, size_t n, f
     v[i] = vi;
     float mh = mi / c1, vh = vi / c2;
     w[i] -= lr * mh / (sqrtf(vh) + eps);
-}
-
-__global__ void k_add(float* a, const float* b, size_t n) {
-    size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) a[i] += b[i];
 }
 
 inline unsigned blocks_for(size_t n, int t = 256) { return (unsigned)((n + t - 1) / t); }
@@ -402,31 +437,34 @@ struct ConvOutPadded {
     }
 };
 
-// the stride-2 layer keeps the im2col GEMM: its input and output padded
+// the stride-2 layer keeps the im2col GEMM: its input and output padded (the
+// border supplies the zeros of the padding)
 struct TcConvInPadded {
-    static constexpr bool kAsync = true;
     const bf16* x;
     int H, W, C, Ho, Wo, stride;
+    typedef const bf16* Row;
     __device__ const void* base() const { return x; }
-    __device__ const void* src(int m, int k) const {
-        int ci = k % C, t = k / C, kx = t % 3, ky = t / 3;
-        int xo = m % Wo, r = m / Wo, yo = r % Ho, b = r / Ho;
-        // padded coordinates: the border supplies the zeros of the padding
-        int y = yo * stride + ky, xx = xo * stride + kx;
-        return x + (((size_t)b * (H + 2) + y) * (W + 2) + xx) * C + ci;
+    __device__ Row row(int m, int M) const {
+        const int xo = m % Wo, r = m / Wo, yo = r % Ho, b = r / Ho;
+        return m < M ? x + (((size_t)b * (H + 2) + yo * stride) * (W + 2) + xo * stride) * C
+                     : nullptr;
     }
+    __device__ int kpos(int k) const {
+        const int ci = k % C, t = k / C, kx = t % 3, ky = t / 3;
+        return (ky * (W + 2) + kx) * C + ci;
+    }
+    __device__ const void* at(Row r, int k) const { return r ? r + k : nullptr; }
 };
 
 struct ConvOutToPadded {
     const float* bias;
     bf16* y;
-    int M, Cout, relu, Ho, Wo;
-    __device__ void operator()(int, int m, int n, float v) const {
-        if (m >= M || n >= Cout) return;
-        v += bias[n];
-        if (relu) v = fmaxf(v, 0.f);
-        int xo = m % Wo, r = m / Wo, yo = r % Ho, b = r / Ho;
-        y[pad_pos(b, yo, xo, Ho, Wo) * Cout + n] = __float2bfloat16(v);
+    int Cout, relu, Ho, Wo;
+    __device__ void operator()(int m, int n, const float (&v)[8]) const {
+        float o[8];
+        bias_relu(bias + n, relu, v, o);
+        const int xo = m % Wo, r = m / Wo, yo = r % Ho, b = r / Ho;
+        *(uint4*)(y + pad_pos(b, yo, xo, Ho, Wo) * Cout + n) = pack8(o);
     }
 };
 
@@ -488,38 +526,62 @@ rf_status cfail(rf_status st, const std::string& msg) {
 int Ho_of(int H, int s) { return s == 1 ? H : (H + 1) / 2; }
 
 template <int NT, class LA, class LB, class EP>
-rf_status tc_launch(rf_cnn* c, int M, int N, int K, int splits, LA la, LB lb, EP ep) {
-    using S = rf_tc::TcSmem<NT, rf_tc::stages_for<LA, LB>()>;
+rf_status tc_launch(rf_cnn* c, int M, int N, int K, LA la, LB lb, EP ep) {
+    using S = rf_tc::TcSmem<NT>;
     static bool attr_set = false;
     if (!attr_set) {
         CN(cudaFuncSetAttribute(rf_tc::k_tc_gemm<NT, LA, LB, EP>,
                                 cudaFuncAttributeMaxDynamicSharedMemorySize, S::kBytes));
         attr_set = true;
     }
-    int kspan = ((K + splits - 1) / splits + rf_tc::kTK - 1) / rf_tc::kTK * rf_tc::kTK;
-    splits = (K + kspan - 1) / kspan;
-    dim3 grid((M + rf_tc::kTM - 1) / rf_tc::kTM, (N + NT - 1) / NT, splits);
+    dim3 grid((M + rf_tc::kTM - 1) / rf_tc::kTM, (N + NT - 1) / NT);
     rf_tc::k_tc_gemm<NT, LA, LB, EP><<<grid, rf_tc::kThreads, S::kBytes, c->stream>>>(
-        M, N, K, kspan, la, lb, ep, c->d_status, c->test_first_wait_polls);
+        M, N, K, la, lb, ep, c->d_status, c->test_first_wait_polls);
     c->launches++;
     CN(cudaGetLastError());
     return RF_OK;
 }
 
-// D[M x N] = A[M x K] B[N x K]^T on the tensor cores; returns the number of
-// K splits actually used through *used (if not null)
+// D[M x N] = A[M x K] B[N x K]^T on the tensor cores
 template <class LA, class LB, class EP>
-rf_status tc_gemm(rf_cnn* c, int M, int N, int K, int splits, LA la, LB lb, EP ep,
-                  int* used = nullptr) {
-    if (used) {
-        int kspan = ((K + splits - 1) / splits + rf_tc::kTK - 1) / rf_tc::kTK * rf_tc::kTK;
-        *used = (K + kspan - 1) / kspan;
+rf_status tc_gemm(rf_cnn* c, int M, int N, int K, LA la, LB lb, EP ep) {
+    if (N <= 16) return tc_launch<16>(c, M, N, K, la, lb, ep);
+    if (N <= 32) return tc_launch<32>(c, M, N, K, la, lb, ep);
+    if (N <= 64) return tc_launch<64>(c, M, N, K, la, lb, ep);
+    if (N <= 96) return tc_launch<96>(c, M, N, K, la, lb, ep);
+    return tc_launch<128>(c, M, N, K, la, lb, ep);
+}
+
+template <int NT>
+rf_status wgrad_launch(rf_cnn* c, int M, int N, int K, int kspan, int splits,
+                       const rf_tc::WgradGeom& w, TcStoreWGrad ep) {
+    using S = rf_tc::WgSmem<NT>;
+    static bool attr_set = false;
+    if (!attr_set) {
+        CN(cudaFuncSetAttribute(rf_tc::k_tc_wgrad<NT, TcStoreWGrad>,
+                                cudaFuncAttributeMaxDynamicSharedMemorySize, S::kBytes));
+        attr_set = true;
     }
-    if (N <= 16) return tc_launch<16>(c, M, N, K, splits, la, lb, ep);
-    if (N <= 32) return tc_launch<32>(c, M, N, K, splits, la, lb, ep);
-    if (N <= 64) return tc_launch<64>(c, M, N, K, splits, la, lb, ep);
-    if (N <= 96) return tc_launch<96>(c, M, N, K, splits, la, lb, ep);
-    return tc_launch<128>(c, M, N, K, splits, la, lb, ep);
+    const dim3 grid((M + rf_tc::kTM - 1) / rf_tc::kTM, 1, splits);
+    rf_tc::k_tc_wgrad<NT, TcStoreWGrad><<<grid, rf_tc::kThreads, S::kBytes, c->stream>>>(
+        M, N, K, kspan, w, ep, c->d_status, c->test_first_wait_polls);
+    c->launches++;
+    CN(cudaGetLastError());
+    return RF_OK;
+}
+
+// weight gradient of layer L over K pixels in `splits` parts; returns the
+// number of parts actually used through *used
+rf_status conv_wgrad(rf_cnn* c, const Layer& L, const rf_tc::WgradGeom& w, int K, int splits,
+                     int* used) {
+    const int M = 9 * L.cin, N = L.cout;
+    const int kspan = ((K + splits - 1) / splits + rf_tc::kTK - 1) / rf_tc::kTK * rf_tc::kTK;
+    splits = *used = (K + kspan - 1) / kspan;
+    const TcStoreWGrad ep{c->part, M, N};
+    if (N <= 16) return wgrad_launch<16>(c, M, N, K, kspan, splits, w, ep);
+    if (N <= 32) return wgrad_launch<32>(c, M, N, K, kspan, splits, w, ep);
+    if (N <= 64) return wgrad_launch<64>(c, M, N, K, kspan, splits, w, ep);
+    return wgrad_launch<96>(c, M, N, K, kspan, splits, w, ep);
 }
 
 // forward conv of layer L: x (B x H x W x cin) -> y (BF16) and/or yf (FP32)
@@ -529,8 +591,8 @@ rf_status conv_fwd(rf_cnn* c, const Layer& L, const bf16* x, int B, int H, int W
     int M = B * Ho * Wo, K = 9 * L.cin;
     TcConvIn la{x, B, H, W, L.cin, Ho, Wo, L.stride};
     TcRows lb{c->wb + L.woff, K};
-    ConvOut ep{c->w + L.boff, y, yf, M, L.cout, L.relu};
-    return tc_gemm(c, M, L.cout, K, 1, la, lb, ep);
+    ConvOut ep{c->w + L.boff, y, yf, L.cout, L.relu};
+    return tc_gemm(c, M, L.cout, K, la, lb, ep);
 }
 
 // backward of layer L given dy (FP32, already through the ReLU mask) and its
@@ -544,8 +606,8 @@ rf_status conv_bwd(rf_cnn* c, const Layer& L, const bf16* x, int B, int H, int W
     int used = 1;
     size_t need = (size_t)splits * L.cout * Mw;
     if (need > c->part_floats) return cfail(RF_ERR_STATE, "cnn: partial buffer too small");
-    rf_status rs = tc_gemm(c, Mw, L.cout, P, splits, TcWGradA{x, H, W, L.cin, Ho, Wo, L.stride},
-                           TcWGradB{dyb, L.cout}, TcStoreWGrad{c->part, Mw, L.cout}, &used);
+    rf_status rs = conv_wgrad(c, L, rf_tc::WgradGeom{x, dyb, H, W, L.cin, Ho, Wo, L.cout, L.stride},
+                              P, splits, &used);
     if (rs != RF_OK) return rs;
     k_reduce_partials<<<blocks_for((size_t)L.cout * Mw), 256, 0, c->stream>>>(
         c->part, used, L.cout * Mw, c->g + L.woff);
@@ -559,8 +621,8 @@ rf_status conv_bwd(rf_cnn* c, const Layer& L, const bf16* x, int B, int H, int W
     c->launches += 3;
     if (dx) {
         int M = B * H * W, K = 9 * L.cout;
-        rs = tc_gemm(c, M, L.cin, K, 1, TcDataGradA{dyb, H, W, Ho, Wo, L.cout, L.stride},
-                     TcRows{c->wt + L.woff, K}, StoreF32{dx, M, L.cin});
+        rs = tc_gemm(c, M, L.cin, K, TcDataGradA{dyb, H, W, Ho, Wo, L.cout, L.stride},
+                     TcRows{c->wt + L.woff, K}, StoreF32{dx, L.cin});
         if (rs != RF_OK) return rs;
     }
     CN(cudaGetLastError());
@@ -634,10 +696,10 @@ rf_status forward_direct(rf_cnn* c, const float* input, int B, int H, int W) {
     rf_status rs = conv3_direct<32>(c, 0, c->map_x, B, H, W, c->a1p, nullptr);
     if (rs == RF_OK) {
         const int M = B * H2 * W2, K = 9 * c2.cin;
-        rs = tc_gemm(c, M, c2.cout, K, 1,
+        rs = tc_gemm(c, M, c2.cout, K,
                      TcConvInPadded{c->a1p, H, W, c2.cin, H2, W2, c2.stride},
                      TcRows{c->wb + c2.woff, K},
-                     ConvOutToPadded{c->w + c2.boff, c->a2p, M, c2.cout, c2.relu, H2, W2});
+                     ConvOutToPadded{c->w + c2.boff, c->a2p, c2.cout, c2.relu, H2, W2});
     }
     if (rs == RF_OK) rs = conv3_direct<96>(c, 2, c->map_a2, B, H2, W2, c->a3p, nullptr);
     if (rs == RF_OK) rs = conv3_direct<16>(c, 3, c->map_a3, B, H2, W2, nullptr, c->o16);
@@ -665,7 +727,7 @@ rf_status forward(rf_cnn* c, const float* input, int B, int H, int W) {
     if (rs == RF_OK) rs = conv_fwd(c, h16, c->a3, B, H2, W2, nullptr, c->o16);
     if (rs != RF_OK) return rs;
     size_t ncat = (size_t)B * H * W * (c3.cout + c1.cout);
-    k_concat_up<<<blocks_for(ncat), 256, 0, c->stream>>>(c->a3, H2, W2, c3.cout, c->a1, c1.cout,
+    k_concat_up<<<blocks_for(ncat / 8), 256, 0, c->stream>>>(c->a3, H2, W2, c3.cout, c->a1, c1.cout,
                                                          B, H, W, c->cat);
     c->launches++;
     rs = conv_fwd(c, c4, c->cat, B, H, W, c->a4, nullptr);
@@ -683,35 +745,31 @@ rf_status backward(rf_cnn* c, int B, int H, int W) {
     rf_status rs = conv_bwd(c, h8, c->a4, B, H, W, c->g_o8, c->gb, c->g_a4);
     if (rs != RF_OK) return rs;
     size_t n4 = (size_t)B * H * W * c4.cout;
-    k_relu_grad<<<blocks_for(n4), 256, 0, c->stream>>>(c->g_a4, c->a4, c->gb, n4);
+    k_relu_grad<<<blocks_for(n4 / 4), 256, 0, c->stream>>>(c->g_a4, nullptr, c->a4, c->gb, n4);
     rs = conv_bwd(c, c4, c->cat, B, H, W, c->g_a4, c->gb, c->g_cat);
     if (rs != RF_OK) return rs;
     // split the concat gradient: g_a3 = up^T(g_cat[:96]), g_a1 = g_cat[96:]
     size_t n3 = (size_t)B * H2 * W2 * c3.cout;
     size_t n1 = (size_t)B * H * W * c1.cout;
-    CN(cudaMemsetAsync(c->g_a3, 0, n3 * sizeof(float), c->stream));
-    k_concat_up_grad<<<blocks_for(std::max(n3, n1)), 256, 0, c->stream>>>(
-        c->g_cat, H2, W2, c3.cout, c1.cout, B, H, W, c->g_a3, c->g_a1, 0);
+    k_concat_up_grad<<<blocks_for(std::max(n3, n1) / 4), 256, 0, c->stream>>>(
+        c->g_cat, H2, W2, c3.cout, c1.cout, B, H, W, c->g_a3, c->g_a1);
     // 1/16 head adds into g_a3
     k_f32_to_bf16<<<blocks_for(n16), 256, 0, c->stream>>>(c->g_o16, c->gb, n16);
     float* tmp = c->g_a2;  // scratch for the head's input gradient (same size as g_a3)
     rs = conv_bwd(c, h16, c->a3, B, H2, W2, c->g_o16, c->gb, tmp);
     if (rs != RF_OK) return rs;
-    // g_a3 += tmp (reuse the ReLU kernel path: add then mask)
-    k_add<<<blocks_for(n3), 256, 0, c->stream>>>(c->g_a3, tmp, n3);
-    k_relu_grad<<<blocks_for(n3), 256, 0, c->stream>>>(c->g_a3, c->a3, c->gb, n3);
+    k_relu_grad<<<blocks_for(n3 / 4), 256, 0, c->stream>>>(c->g_a3, tmp, c->a3, c->gb, n3);
     rs = conv_bwd(c, c3, c->a2, B, H2, W2, c->g_a3, c->gb, c->g_a2);
     if (rs != RF_OK) return rs;
     size_t n2 = (size_t)B * H2 * W2 * c2.cout;
-    k_relu_grad<<<blocks_for(n2), 256, 0, c->stream>>>(c->g_a2, c->a2, c->gb, n2);
+    k_relu_grad<<<blocks_for(n2 / 4), 256, 0, c->stream>>>(c->g_a2, nullptr, c->a2, c->gb, n2);
     // c2's input gradient adds into g_a1 (which holds the skip part): use tmp2
     float* tmp2 = c->g_a4;  // free now, large enough (B*H*W*64 >= B*H*W*32)
     rs = conv_bwd(c, c2, c->a1, B, H, W, c->g_a2, c->gb, tmp2);
     if (rs != RF_OK) return rs;
-    k_add<<<blocks_for(n1), 256, 0, c->stream>>>(c->g_a1, tmp2, n1);
-    k_relu_grad<<<blocks_for(n1), 256, 0, c->stream>>>(c->g_a1, c->a1, c->gb, n1);
+    k_relu_grad<<<blocks_for(n1 / 4), 256, 0, c->stream>>>(c->g_a1, tmp2, c->a1, c->gb, n1);
     rs = conv_bwd(c, c1, c->x, B, H, W, c->g_a1, c->gb, nullptr);
-    c->launches += 9;
+    c->launches += 7;
     if (rs != RF_OK) return rs;
     CN(cudaGetLastError());
     return RF_OK;

@@ -5,24 +5,33 @@
 //   D[M x N] = sum_k A(m, k) B(n, k)      (both operands K-major)
 //
 // One CTA of 128 threads computes a 128 x NT tile of D (NT = 16 .. 256, a
-// multiple of 16) over a range of K (split-K over gridDim.z).  For each
-// K-chunk of 64 the 128 threads gather the A tile (128 x 64) and the B tile
+// multiple of 16).  For each
+// K-chunk of 64 the 128 threads copy the A tile (128 x 64) and the B tile
 // (NT x 64) into shared memory in the canonical no-swizzle K-major layout
 // (8 x 16-byte core matrices: rows of a core matrix 16 bytes apart, core
-// matrices 128 bytes apart along K and 1024 bytes apart along M / N), make
-// the writes visible to the tensor core (fence.proxy.async), and one thread
-// issues four 128 x NT x 16 MMAs and commits them to an mbarrier.  kStages
-// chunk buffers form a ring: the copies of chunks c+1 .. c+kStages-1 are in
-// flight (cp.async, 16 bytes each, zero-filled outside the operand) while
-// the MMAs of chunk c run.  The epilogue reads the accumulator with
-// tcgen05.ld: warp w owns TMEM lanes (= rows of D) 32w .. 32w + 31.
+// matrices kLbo bytes apart along K and kSbo along M / N), make the writes
+// visible to the tensor core (fence.proxy.async), and one thread issues four
+// 128 x NT x 16 MMAs and commits them to an mbarrier.  kStages chunk buffers
+// form a ring: the copies of chunks c+1 .. c+kStages-1 are in flight (cp.async,
+// 16 bytes each, zero-filled outside the operand) while the MMAs of chunk c
+// run.  The epilogue reads the accumulator with tcgen05.ld: warp w owns TMEM
+// lanes (= rows of D) 32w .. 32w + 31.
 //
-// A loader functor gives the 8 consecutive K elements of one row: an
-// asynchronous loader (kAsync = true) their 16-byte-aligned global address
-// (src(), null for zeros), a gathering loader (kAsync = false) their value as
-// a uint4 (operator(), zeros outside the operand), which the threads store
-// into the ring themselves.  The epilogue functor receives (split, m, n,
-// value).
+// What bounds it is feeding the copies.  kLbo is 144 and not 128 so that the
+// eight copies of a row (K groups g = 0 .. 7, issued by neighbouring threads,
+// 128 contiguous bytes of global memory) land in different banks: at 128 they
+// shared four banks and a chunk took 8 times as long to write.  And an operand
+// hands out what its address computation can reuse: row(r) once per thread and
+// row before the loop, kpos(k) once per thread and chunk, at(row, kpos) per
+// copy (null for zeros); with all of it per copy, the integer divisions of the
+// im2col index took longer than the copies.  On 64 images of 160 x 120 the
+// 128 -> 64 layer takes 1.12 ms forward and 0.86 ms for its input gradient
+// (1.71 and 1.83 before), its tile traffic (4.1 GB through L2) and one barrier
+// per chunk bounding it now.
+//
+// The epilogue functor receives a row's eight consecutive columns (m, n, v[8]; N
+// a multiple of 8) and stores them as vectors: a thread has a row, so scalar
+// stores were 32 sectors an instruction.
 #pragma once
 
 #include <cstdint>
@@ -139,9 +148,11 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8]) {
     for (int i = 0; i < 8; i++) v[i] = __uint_as_float(r[i]);
 }
 
+// a chunk tile in shared memory: core matrices along K and along M / N
+constexpr int kLbo = 144, kSbo = kTK / 8 * kLbo;
 // byte offset of element row r, k-group g (8 elements) in a chunk tile
 __device__ __forceinline__ uint32_t tile_off(int r, int g) {
-    return (uint32_t)(((r >> 3) * (kTK / 8) + g) * 128 + (r & 7) * 16);
+    return (uint32_t)((r >> 3) * kSbo + g * kLbo + (r & 7) * 16);
 }
 
 __device__ __forceinline__ void cp_async16(void* smem_dst, const void* gsrc, int src_bytes) {
@@ -157,28 +168,20 @@ __device__ __forceinline__ void cp_async_wait() {
     asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
-// chunk buffers in the ring: three when a loader copies asynchronously (two
-// chunks in flight during an MMA), two when both gather through registers
-// (their stores finish before the chunk's barrier anyway; less shared
-// memory keeps more CTAs resident)
-template <class LA, class LB>
-constexpr int stages_for() {
-    return (LA::kAsync || LB::kAsync) ? 3 : 2;
-}
+constexpr int kStages = 3;  // chunk buffers in the ring: two chunks in flight during an MMA
 
-template <int NT, int kStages>
+template <int NT>
 struct TcSmem {
     static_assert(NT % 16 == 0 && NT >= 16 && NT <= 256, "N tile");
     static_assert((NT * 8) % 128 == 0, "B tile rows split evenly over the CTA's threads");
-    static constexpr int kA = kTM * kTK * 2;  // bytes of one A chunk
-    static constexpr int kB = NT * kTK * 2;
+    static constexpr int kA = kTM / 8 * kSbo;  // bytes of one A chunk
+    static constexpr int kB = NT / 8 * kSbo;
     // the chunk ring, barriers, alignment slack
     static constexpr int kBytes = kStages * (kA + kB) + 2048;
     static constexpr uint32_t kCols = NT <= 32 ? 32 : (NT <= 64 ? 64 : (NT <= 128 ? 128 : 256));
 };
 
-// grid: x = M tiles, y = N tiles, z = K splits (each `kspan` long, a multiple
-// of kTK).  `status` (device int) is set to 1 if a wait gave up; the launch's
+// grid: x = M tiles, y = N tiles.  `status` (device int) is set to 1 if a wait gave up; the launch's
 // outputs are then not written.  A thread whose wait for a ring slot gives up
 // writes no further chunks (an MMA may still be reading that slot); the MMA
 // thread keeps issuing and committing, and every thread drains the last
@@ -188,12 +191,10 @@ struct TcSmem {
 // 0 makes it give up at once while the MMAs still complete); -1 = the
 // normal limit.
 template <int NT, class LA, class LB, class EP>
-__global__ void __launch_bounds__(kThreads) k_tc_gemm(int M, int N, int K, int kspan, LA la,
-                                                     LB lb, EP ep, int* status,
-                                                     int first_wait_polls) {
+__global__ void __launch_bounds__(kThreads) k_tc_gemm(int M, int N, int K, LA la, LB lb, EP ep,
+                                                     int* status, int first_wait_polls) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
-    constexpr int kStages = stages_for<LA, LB>();
-    using S = TcSmem<NT, kStages>;
+    using S = TcSmem<NT>;
     unsigned char* base = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint64_t* bars = (uint64_t*)(base + kStages * (S::kA + S::kB));  // one per ring slot
     uint32_t* tslot = (uint32_t*)(bars + kStages);
@@ -201,9 +202,7 @@ __global__ void __launch_bounds__(kThreads) k_tc_gemm(int M, int N, int K, int k
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int m0 = blockIdx.x * kTM, n0 = blockIdx.y * NT;
-    const int k_begin = blockIdx.z * kspan;
-    const int k_end = min(K, k_begin + kspan);
-    const int nchunks = (k_end - k_begin + kTK - 1) / kTK;
+    const int nchunks = (K + kTK - 1) / kTK;
 
     if (tid == 0) {
         for (int q = 0; q < kStages; q++) mbar_init(&bars[q], 1);
@@ -217,57 +216,35 @@ __global__ void __launch_bounds__(kThreads) k_tc_gemm(int M, int N, int K, int k
     const uint32_t tmem = *tslot;
     constexpr uint32_t idesc = idesc_bf16(kTM, NT);
 
-    // queue the copies (or do the gathers) of chunk c into ring slot c % kStages
+    // thread t copies K group t % 8 of rows t / 8, t / 8 + 16, ...
+    constexpr int kPerA = kTM * (kTK / 8) / kThreads;  // 8
+    constexpr int kPerB = NT * (kTK / 8) / kThreads;   // NT / 16
+    const int g = tid & 7, r0 = tid >> 3;
+    typename LA::Row ra[kPerA];
+    typename LB::Row rb[kPerB];
+#pragma unroll
+    for (int j = 0; j < kPerA; j++) ra[j] = la.row(m0 + r0 + 16 * j, M);
+#pragma unroll
+    for (int j = 0; j < kPerB; j++) rb[j] = lb.row(n0 + r0 + 16 * j, N);
+
+    // queue the copies of chunk c into ring slot c % kStages
     auto issue = [&](int c) {
         const int q = c % kStages;
-        unsigned char* tA = base + q * S::kA;
-        unsigned char* tB = base + kStages * S::kA + q * S::kB;
-        const int kc = k_begin + c * kTK;
-        constexpr int kPerA = kTM * (kTK / 8) / kThreads;  // 8
-        constexpr int kPerB = NT * (kTK / 8) / kThreads;   // NT / 16
-        if constexpr (LA::kAsync) {
+        unsigned char* tA = base + q * S::kA + tile_off(r0, g);
+        unsigned char* tB = base + kStages * S::kA + q * S::kB + tile_off(r0, g);
+        const int k = c * kTK + g * 8;
+        const bool in = k < K;
+        const auto ka = la.kpos(k);
+        const auto kb = lb.kpos(k);
 #pragma unroll
-            for (int j = 0; j < kPerA; j++) {
-                const int i = tid + j * kThreads, r = i >> 3, g = i & 7, k = kc + g * 8;
-                const void* src = (m0 + r < M && k < k_end) ? la.src(m0 + r, k) : nullptr;
-                cp_async16(tA + tile_off(r, g), src ? src : la.base(), src ? 16 : 0);
-            }
-        } else {
-            // all of a thread's loads are issued before its stores (the stores go
-            // through a generic pointer the compiler cannot tell from global memory)
-            uint4 va[kPerA];
-#pragma unroll
-            for (int j = 0; j < kPerA; j++) {
-                const int i = tid + j * kThreads, r = i >> 3, g = i & 7, k = kc + g * 8;
-                va[j] = make_uint4(0, 0, 0, 0);
-                if (m0 + r < M && k < k_end) va[j] = la(m0 + r, k, k_end);
-            }
-#pragma unroll
-            for (int j = 0; j < kPerA; j++) {
-                const int i = tid + j * kThreads;
-                *(uint4*)(tA + tile_off(i >> 3, i & 7)) = va[j];
-            }
+        for (int j = 0; j < kPerA; j++) {
+            const void* src = in ? la.at(ra[j], ka) : nullptr;
+            cp_async16(tA + 2 * j * kSbo, src ? src : la.base(), src ? 16 : 0);
         }
-        if constexpr (LB::kAsync) {
 #pragma unroll
-            for (int j = 0; j < kPerB; j++) {
-                const int i = tid + j * kThreads, r = i >> 3, g = i & 7, k = kc + g * 8;
-                const void* src = (n0 + r < N && k < k_end) ? lb.src(n0 + r, k) : nullptr;
-                cp_async16(tB + tile_off(r, g), src ? src : lb.base(), src ? 16 : 0);
-            }
-        } else {
-            uint4 vb[kPerB];
-#pragma unroll
-            for (int j = 0; j < kPerB; j++) {
-                const int i = tid + j * kThreads, r = i >> 3, g = i & 7, k = kc + g * 8;
-                vb[j] = make_uint4(0, 0, 0, 0);
-                if (n0 + r < N && k < k_end) vb[j] = lb(n0 + r, k, k_end);
-            }
-#pragma unroll
-            for (int j = 0; j < kPerB; j++) {
-                const int i = tid + j * kThreads;
-                *(uint4*)(tB + tile_off(i >> 3, i & 7)) = vb[j];
-            }
+        for (int j = 0; j < kPerB; j++) {
+            const void* src = in ? lb.at(rb[j], kb) : nullptr;
+            cp_async16(tB + 2 * j * kSbo, src ? src : lb.base(), src ? 16 : 0);
         }
     };
 
@@ -289,8 +266,8 @@ __global__ void __launch_bounds__(kThreads) k_tc_gemm(int M, int N, int K, int k
             const uint32_t b0 = smem_u32(base + kStages * S::kA + q * S::kB);
 #pragma unroll
             for (int kk = 0; kk < kTK / 16; kk++) {
-                const uint64_t da = smem_desc(a0 + kk * 256, 128, 1024);
-                const uint64_t db = smem_desc(b0 + kk * 256, 128, 1024);
+                const uint64_t da = smem_desc(a0 + kk * 2 * kLbo, kLbo, kSbo);
+                const uint64_t db = smem_desc(b0 + kk * 2 * kLbo, kLbo, kSbo);
                 mma_bf16(tmem, da, db, idesc, (c > 0 || kk > 0) ? 1u : 0u);
             }
             mma_commit(&bars[q]);
@@ -328,10 +305,183 @@ __global__ void __launch_bounds__(kThreads) k_tc_gemm(int M, int N, int K, int k
         for (int j = 0; j < NT; j += 8) {
             float v[8];
             tmem_ld8(lane_addr + (uint32_t)j, v);
+            if (m < M && n0 + j < N) ep(m, n0 + j, v);
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 0) tmem_dealloc(tmem, S::kCols);
+}
+
+// ---------------------------------------------------------------------------
+// Weight gradient of a 3x3 convolution
+// ---------------------------------------------------------------------------
+// D[m][n] = sum over output pixels p of x(p, m) dy(p, n), with m = tap * Cin +
+// ci and x(p, m) the input channel ci under tap `tap` of pixel p.  The reduction
+// runs over pixels, along which neither operand is contiguous, but 8 channels
+// of a pixel are: both operands go to shared memory M / N-major (core matrices
+// of 8 pixels x 8 channels, 16 bytes a pixel), so a copy is 16 bytes of an
+// activation as it lies in memory and nothing is transposed.  (Gathering them
+// K-major, 8 scalar loads per 16 bytes with a division chain each, took 6.7 of
+// a 28 ms training step for the 128 -> 64 layer alone, 64 images of 160 x 120;
+// this takes 1.04 ms of 8.1, and all six layers 2.4 instead of 17.1.)  The order of the
+// reduction is that of k_tc_gemm: pixels in order, 16 per MMA, split at the
+// same places.
+//
+// Thread t copies pixel 4 (t / 8) + t % 4 of a chunk, channel groups (t / 4) % 2
+// + 2j: eight threads read full 32-byte sectors, and with channel groups 1088
+// bytes apart (64 pixels x 16 bytes and 64 of padding) they write all 32 banks.
+constexpr int kWgGroup = kTK * 16 + 64;  // bytes from one channel group to the next
+
+struct WgradGeom {
+    const __nv_bfloat16 *x, *dy;
+    int H, W, C, Ho, Wo, Cout, stride;
+};
+
+template <int NT>
+struct WgSmem {
+    static constexpr int kA = kTM / 8 * kWgGroup, kB = NT / 8 * kWgGroup;
+    static constexpr int kBytes = kStages * (kA + kB) + 2048;
+    static constexpr uint32_t kCols = TcSmem<NT>::kCols;
+};
+
+template <int NT, class EP>
+__global__ void __launch_bounds__(kThreads) k_tc_wgrad(int M, int N, int K, int kspan, WgradGeom w,
+                                                      EP ep, int* status, int first_wait_polls) {
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    using S = WgSmem<NT>;
+    unsigned char* base = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    uint64_t* bars = (uint64_t*)(base + kStages * (S::kA + S::kB));
+    uint32_t* tslot = (uint32_t*)(bars + kStages);
+    int* fail = (int*)(tslot + 1);
+
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int m0 = blockIdx.x * kTM;
+    const int k_begin = blockIdx.z * kspan, k_end = min(K, k_begin + kspan);
+    const int nchunks = (k_end - k_begin + kTK - 1) / kTK;
+
+    if (tid == 0) {
+        for (int q = 0; q < kStages; q++) mbar_init(&bars[q], 1);
+        *fail = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 0) tmem_alloc(tslot, S::kCols);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *tslot;
+    // both operands M / N-major: bits 15 and 16
+    constexpr uint32_t idesc = idesc_bf16(kTM, NT) | (1u << 15) | (1u << 16);
+
+    // this thread's pixel, the next chunk's to be issued
+    const int pk = 4 * (tid >> 3) + (tid & 3), g0 = (tid >> 2) & 1;
+    int p = k_begin + pk, xo, yo, img;
+    {
+        xo = p % w.Wo;
+        const int r = p / w.Wo;
+        yo = r % w.Ho;
+        img = r / w.Ho;
+    }
+    constexpr int kGA = kTM / 16, kGB = NT / 16;  // channel groups per thread
+    // tap and channel of each of this thread's A groups (a tap of -1: past M)
+    int tap[kGA], coff[kGA];
+#pragma unroll
+    for (int j = 0; j < kGA; j++) {
+        const int m = m0 + 8 * (g0 + 2 * j);
+        tap[j] = m < M ? m / w.C : -1;
+        const int ky = m / w.C / 3, kx = m / w.C % 3;
+        coff[j] = ((ky - 1) * w.W + (kx - 1)) * w.C + m % w.C;
+    }
+
+    auto issue = [&](int c) {
+        const int q = c % kStages;
+        unsigned char* tA = base + q * S::kA + g0 * kWgGroup + pk * 16;
+        unsigned char* tB = base + kStages * S::kA + q * S::kB + g0 * kWgGroup + pk * 16;
+        const bool in = p < k_end;
+        const int y = yo * w.stride, x = xo * w.stride;
+        const __nv_bfloat16* xp = w.x + (((size_t)img * w.H + y) * w.W + x) * w.C;
+#pragma unroll
+        for (int j = 0; j < kGA; j++) {
+            const int ky = tap[j] / 3, kx = tap[j] - 3 * ky;
+            const bool ok = in && tap[j] >= 0 && (unsigned)(y + ky - 1) < (unsigned)w.H &&
+                            (unsigned)(x + kx - 1) < (unsigned)w.W;
+            cp_async16(tA + 2 * j * kWgGroup, ok ? xp + coff[j] : w.x, ok ? 16 : 0);
+        }
+        const __nv_bfloat16* dp = w.dy + (size_t)p * w.Cout;
+#pragma unroll
+        for (int j = 0; j < kGB; j++) {
+            const int n = 8 * (g0 + 2 * j);
+            const bool ok = in && n < N;
+            cp_async16(tB + 2 * j * kWgGroup, ok ? dp + n : w.dy, ok ? 16 : 0);
+        }
+        p += kTK;
+        xo += kTK;
+        while (xo >= w.Wo) {
+            xo -= w.Wo;
+            if (++yo == w.Ho) {
+                yo = 0;
+                img++;
+            }
+        }
+    };
+
+    for (int c = 0; c < kStages - 1; c++) {
+        if (c < nchunks) issue(c);
+        cp_async_commit();
+    }
+    bool gave_up = false;  // as in k_tc_gemm
+    for (int c = 0; c < nchunks; c++) {
+        const int q = c % kStages;
+        cp_async_wait<kStages - 2>();
+        fence_async_smem();
+        __syncthreads();
+        if (tid == 0) {
+            tc_fence_after();
+            const uint32_t a0 = smem_u32(base + q * S::kA);
+            const uint32_t b0 = smem_u32(base + kStages * S::kA + q * S::kB);
+#pragma unroll
+            for (int kk = 0; kk < kTK / 16; kk++) {
+                const uint64_t da = smem_desc(a0 + kk * 256, 128, kWgGroup);
+                const uint64_t db = smem_desc(b0 + kk * 256, 128, kWgGroup);
+                mma_bf16(tmem, da, db, idesc, (c > 0 || kk > 0) ? 1u : 0u);
+            }
+            mma_commit(&bars[q]);
+        }
+        const int nc = c + kStages - 1;
+        if (nc < nchunks && !gave_up) {
+            if (c >= 1) {
+                const int pc = c - 1;
+                const unsigned lim = (c == 1 && first_wait_polls >= 0) ? (unsigned)first_wait_polls
+                                                                       : kSpinLimit;
+                if (!mbar_wait(&bars[pc % kStages], (unsigned)(pc / kStages) & 1u, lim)) {
+                    gave_up = true;
+                    *fail = 1;
+                }
+            }
+            if (!gave_up) issue(nc);
+        }
+        cp_async_commit();
+    }
+    cp_async_wait<0>();
+    if (nchunks > 0) {
+        const int lc = nchunks - 1;
+        if (!mbar_wait(&bars[lc % kStages], (unsigned)(lc / kStages) & 1u)) *fail = 1;
+    }
+    tc_fence_after();
+    __syncthreads();
+    if (*fail) {
+        if (tid == 0) atomicExch(status, 1);
+    } else if (nchunks > 0) {
+        const int m = m0 + warp * 32 + lane;
+        const uint32_t lane_addr = tmem + ((uint32_t)(warp * 32) << 16);
+#pragma unroll 1
+        for (int j = 0; j < NT; j += 8) {
+            float v[8];
+            tmem_ld8(lane_addr + (uint32_t)j, v);
             if (m < M)
 #pragma unroll
                 for (int e = 0; e < 8; e++)
-                    if (n0 + j + e < N) ep(blockIdx.z, m, n0 + j + e, v[e]);
+                    if (j + e < N) ep(blockIdx.z, m, j + e, v[e]);
         }
     }
     tc_fence_before();
