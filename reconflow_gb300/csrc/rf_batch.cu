@@ -111,7 +111,8 @@ __device__ __forceinline__ void prefetch_ahead(const BatchCtx& ctx, const TileEn
 // One block = one tile of one pair at `level` (the level's tile shape is
 // the block shape; the tile table gives the pair and the tile's origin).
 template <class Op>
-__global__ void __launch_bounds__(kMaxTile) k_batch(BatchCtx ctx, int level, Op op) {
+__global__ void __launch_bounds__(kMaxTile) k_batch(BatchCtx ctx, int level,
+                                                    const __grid_constant__ Op op) {
     prefetch_ahead(ctx, ctx.tiles, (int)blockIdx.x + ctx.prefetch, (int)gridDim.x, level, op);
     const TileEntry t = ctx.tiles[blockIdx.x];
     const LevelDims d = ctx.pairs[t.pair].dims[level];
@@ -301,9 +302,33 @@ struct OpReconB {
     }
 };
 
+// the half-steps of rf_pair.cuh, one pixel per thread (no L2 prefetch: levels
+// this small are in L2)
+struct OpReconA1 {
+    ReconFields f;
+    Weights wt;
+    int first, ucb;
+    __device__ void operator()(const BatchCtx& ctx, const TileEntry& t, int level, LevelDims d,
+                               int ix, int iy) const {
+        recon_a_one<0>(f, ctx.consts[t.pair * ctx.L + level], wt, d, t.off, ix, iy, first != 0,
+                       ucb != 0);
+    }
+};
+
+template <bool LAST>
+struct OpReconB1 {
+    ReconFields f;
+    Weights wt;
+    int first;
+    __device__ void operator()(const BatchCtx&, const TileEntry& t, int, LevelDims d, int ix,
+                               int iy) const {
+        recon_b_one<LAST>(f, wt, d, t.off, ix, iy, first != 0);
+    }
+};
+
 struct OpPlainData {
     int duhat, dvhat, pu1, pu2, pv1, pv2, Ix, Iy, Iz;
-    Weights wt;
+    PlainWeights wt;
     int first;
     __device__ void operator()(const BatchCtx& ctx, const TileEntry& t, int, LevelDims d, int ix,
                                int iy) const {
@@ -315,7 +340,7 @@ struct OpPlainData {
 
 struct OpPlainTV {
     int duhat, dvhat, pu1, pu2, pv1, pv2;
-    Weights wt;
+    PlainWeights wt;
     int first;
     __device__ void operator()(const BatchCtx& ctx, const TileEntry& t, int, LevelDims d, int ix,
                                int iy) const {
@@ -718,10 +743,11 @@ int launch_op(rf_batch* b, int level, const Op& op) {
     return rf::launch_status();
 }
 
-// A (data step) and B (dual step) of an inner iteration over the level's
-// pixel pairs (rf_pair.cuh); `last`: the warp's last B
-int launch_a2(rf_batch* b, int level, const ReconFields& f, const Weights& wt, bool first,
-              bool ucb) {
+// A (data step) and B (dual step) of an inner iteration (rf_pair.cuh), over the
+// level's pixel pairs or pixels; `last`: the warp's last B
+int launch_half_a(rf_batch* b, int level, const ReconFields& f, const Weights& wt, bool first,
+                  bool ucb) {
+    if (b->pair_blocks[level] == 0) return launch_op(b, level, OpReconA1{f, wt, first, ucb});
     BatchCtx c = ctx_of(b, level);
     c.tiles = b->d_tiles + b->pair_start[level];
     c.prefetch = b->prefetch / 16 * kPairBlocksA / 2;  // half a wave of these blocks
@@ -730,8 +756,11 @@ int launch_a2(rf_batch* b, int level, const ReconFields& f, const Weights& wt, b
     return rf::launch_status();
 }
 
-int launch_b2(rf_batch* b, int level, const ReconFields& f, const Weights& wt, bool first,
-              bool last) {
+int launch_half_b(rf_batch* b, int level, const ReconFields& f, const Weights& wt, bool first,
+                  bool last) {
+    if (b->pair_blocks[level] == 0)
+        return last ? launch_op(b, level, OpReconB1<true>{f, wt, first})
+                    : launch_op(b, level, OpReconB1<false>{f, wt, first});
     BatchCtx c = ctx_of(b, level);
     c.tiles = b->d_tiles + b->pair_start[level];
     if (last)
@@ -893,9 +922,9 @@ rf_status enqueue_batch(rf_batch* b, int kind) {
             }
             for (int iter = 0; iter < n_iters && !(recon && b->split > 0); iter++) {
                 const int first = iter == 0;
-                if (recon && b->pair_blocks[level] > 0) {
-                    BL(launch_a2(b, level, r, wt, first, ucb));
-                    BL(launch_b2(b, level, r, wt, first, iter + 1 == n_iters));
+                if (recon && pair_weights(wt)) {
+                    BL(launch_half_a(b, level, r, wt, first, ucb));
+                    BL(launch_half_b(b, level, r, wt, first, iter + 1 == n_iters));
                     ucb = false;
                 } else if (recon) {
                     BL(launch_op(b, level, OpReconA{r, wt, first, ucb ? 1 : 0}));
@@ -1312,9 +1341,9 @@ rf_status rf_batch_profile_level(rf_batch* b, int level, int n_iters, float* ms)
         BC(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
         int bad = 0;
         for (int i = 0; i < n_iters && !bad; i++)
-            if (b->pair_blocks[level] > 0)
-                bad = k == 0 ? launch_a2(b, level, r, wt, false, false)
-                             : launch_b2(b, level, r, wt, false, false);
+            if (pair_weights(wt))
+                bad = k == 0 ? launch_half_a(b, level, r, wt, false, false)
+                             : launch_half_b(b, level, r, wt, false, false);
             else
                 bad = k == 0 ? launch_op(b, level, OpReconA{r, wt, 0, 0})
                              : launch_op(b, level, OpReconB{r, wt, 0});

@@ -226,7 +226,32 @@ __global__ void __launch_bounds__(BX* BY, RF_MINB_B) k_recon_b(ReconFields f, We
     recon_b_px(f, wt, d, ix, iy, first);
 }
 
-// The two-pixel half-steps (rf_pair.cuh; registers and tile as in the batch)
+// The half-steps of rf_pair.cuh, one pixel per thread: 632 and 371 warp
+// instructions per 32 pixels against 725 and 385 of k_recon_a / k_recon_b (a
+// plain 640x480 solve 6.49 -> 5.94 ms, 720p 37.0 -> 35.1).  Programmatic
+// dependent launches made them slower (6.17, 36.3): the launch is not what a
+// small level waits for, its longest thread is.
+template <int PRIOR>
+__global__ void __launch_bounds__(BX* BY)
+    k_recon_a1(const __grid_constant__ ReconFields f, const LevelConsts* __restrict__ lcp,
+               const __grid_constant__ Weights wt, LevelDims d, int first, int uc_from_buffer) {
+    const int ix = blockIdx.x * blockDim.x + threadIdx.x;
+    const int iy = blockIdx.y * blockDim.y + threadIdx.y;
+    if (ix >= d.w || iy >= d.h) return;
+    recon_a_one<PRIOR>(f, *lcp, wt, d, 0, ix, iy, first != 0, uc_from_buffer != 0);
+}
+
+template <bool LAST>
+__global__ void __launch_bounds__(BX* BY)
+    k_recon_b1(const __grid_constant__ ReconFields f, const __grid_constant__ Weights wt,
+               LevelDims d, int first) {
+    const int ix = blockIdx.x * blockDim.x + threadIdx.x;
+    const int iy = blockIdx.y * blockDim.y + threadIdx.y;
+    if (ix >= d.w || iy >= d.h) return;
+    recon_b_one<LAST>(f, wt, d, 0, ix, iy, first != 0);
+}
+
+// two pixels per thread (registers and tile as in the batch)
 template <int PRIOR>
 __global__ void __launch_bounds__(32 * kPairRows, 5)
     k_recon_a2(const __grid_constant__ ReconFields f, const LevelConsts* __restrict__ lcp,
@@ -290,7 +315,7 @@ __global__ void k_plain_data(float* __restrict__ duhat0, float* __restrict__ dvh
                              const float* __restrict__ pu1, const float* __restrict__ pu2,
                              const float* __restrict__ pv1, const float* __restrict__ pv2,
                              const float* __restrict__ Ix, const float* __restrict__ Iy,
-                             const float* __restrict__ Iz, Weights wt, LevelDims d, int first) {
+                             const float* __restrict__ Iz, PlainWeights wt, LevelDims d, int first) {
     int ix = blockIdx.x * blockDim.x + threadIdx.x;
     int iy = blockIdx.y * blockDim.y + threadIdx.y;
     if (ix >= d.w || iy >= d.h) return;
@@ -299,7 +324,7 @@ __global__ void k_plain_data(float* __restrict__ duhat0, float* __restrict__ dvh
 
 __global__ void k_plain_tv(const float* __restrict__ duhat, const float* __restrict__ dvhat,
                            float* __restrict__ pu1, float* __restrict__ pu2,
-                           float* __restrict__ pv1, float* __restrict__ pv2, Weights wt,
+                           float* __restrict__ pv1, float* __restrict__ pv2, PlainWeights wt,
                            LevelDims d, int first) {
     int ix = blockIdx.x * blockDim.x + threadIdx.x;
     int iy = blockIdx.y * blockDim.y + threadIdx.y;
@@ -714,29 +739,47 @@ bool pair_weights(const Weights& wt) {
            wt.alpha_proj >= 0.0f && wt.alpha_fn >= 0.0f;
 }
 
-bool use_pairs(const Weights& wt, LevelDims d) {
+namespace {
+// whether a level takes two pixels per thread
+bool use_pairs(LevelDims d) {
     // A 720p pair's level 0 (0.92 million pixels, under two waves of blocks, its
     // state in L2) takes as long either way (37.2 against 37.0 ms a solve), a
     // 1080p pair's (2.1 million) is faster by pairs (67.5 against 73.0 ms).
     constexpr long long kMinPixels = 1500000;
-    return pair_stride(d) && (long long)d.w * d.h >= kMinPixels && pair_weights(wt);
+    return pair_stride(d) && (long long)d.w * d.h >= kMinPixels;
 }
+}  // namespace
 
-int launch_recon_a2(const ReconFields& f, const LevelConsts* lc, const Weights& wt, LevelDims d,
-                    bool first, bool uc_from_buffer, int prior, cudaStream_t st) {
-    const dim3 g((d.w + kPairW - 1) / kPairW, (d.h + kPairRows - 1) / kPairRows);
-    const int n = 32 * kPairRows, fi = first ? 1 : 0, ub = uc_from_buffer ? 1 : 0;
-    if (prior == 1) k_recon_a2<1><<<g, n, 0, st>>>(f, lc, wt, d, fi, ub);
-    else if (prior == 2) k_recon_a2<2><<<g, n, 0, st>>>(f, lc, wt, d, fi, ub);
-    else k_recon_a2<0><<<g, n, 0, st>>>(f, lc, wt, d, fi, ub);
+int launch_half_a(const ReconFields& f, const LevelConsts* lc, const Weights& wt, LevelDims d,
+                  bool first, bool uc_from_buffer, int prior, cudaStream_t st, dim3 b) {
+    const int fi = first ? 1 : 0, ub = uc_from_buffer ? 1 : 0;
+    if (use_pairs(d)) {
+        const dim3 g((d.w + kPairW - 1) / kPairW, (d.h + kPairRows - 1) / kPairRows);
+        const int n = 32 * kPairRows;
+        if (prior == 1) k_recon_a2<1><<<g, n, 0, st>>>(f, lc, wt, d, fi, ub);
+        else if (prior == 2) k_recon_a2<2><<<g, n, 0, st>>>(f, lc, wt, d, fi, ub);
+        else k_recon_a2<0><<<g, n, 0, st>>>(f, lc, wt, d, fi, ub);
+    } else {
+        const dim3 g((d.w + b.x - 1) / b.x, (d.h + b.y - 1) / b.y);
+        if (prior == 1) k_recon_a1<1><<<g, b, 0, st>>>(f, lc, wt, d, fi, ub);
+        else if (prior == 2) k_recon_a1<2><<<g, b, 0, st>>>(f, lc, wt, d, fi, ub);
+        else k_recon_a1<0><<<g, b, 0, st>>>(f, lc, wt, d, fi, ub);
+    }
     return check_launch();
 }
 
-int launch_recon_b2(const ReconFields& f, const Weights& wt, LevelDims d, bool first, bool last,
-                    cudaStream_t st) {
-    const dim3 g((d.w + kPairW - 1) / kPairW, (d.h + kPairRows - 1) / kPairRows);
-    if (last) k_recon_b2<true><<<g, 32 * kPairRows, 0, st>>>(f, wt, d, first ? 1 : 0);
-    else k_recon_b2<false><<<g, 32 * kPairRows, 0, st>>>(f, wt, d, first ? 1 : 0);
+int launch_half_b(const ReconFields& f, const Weights& wt, LevelDims d, bool first, bool last,
+                  cudaStream_t st, dim3 b) {
+    const int fi = first ? 1 : 0;
+    if (use_pairs(d)) {
+        const dim3 g((d.w + kPairW - 1) / kPairW, (d.h + kPairRows - 1) / kPairRows);
+        if (last) k_recon_b2<true><<<g, 32 * kPairRows, 0, st>>>(f, wt, d, fi);
+        else k_recon_b2<false><<<g, 32 * kPairRows, 0, st>>>(f, wt, d, fi);
+    } else {
+        const dim3 g((d.w + b.x - 1) / b.x, (d.h + b.y - 1) / b.y);
+        if (last) k_recon_b1<true><<<g, b, 0, st>>>(f, wt, d, fi);
+        else k_recon_b1<false><<<g, b, 0, st>>>(f, wt, d, fi);
+    }
     return check_launch();
 }
 

@@ -25,6 +25,15 @@ struct Weights {
     float lambdaf, lambdams;
     float proj_den;   // lambdaf + alpha_proj
     float theta;      // plain TV-L1 theta
+    float nrA, nrP;   // -1 / A, -1 / proj_den
+};
+
+// What the plain TV-L1 kernels use of them (their launches are so short that
+// the size of their parameters shows: with all of Weights a 640x480 solve takes
+// 3% longer).
+struct PlainWeights {
+    float lambda, theta, fac;
+    PlainWeights(const Weights& w) : lambda(w.lambda), theta(w.theta), fac(w.fac) {}
 };
 
 // Fields of one ReconFlow inner iteration.
@@ -146,15 +155,14 @@ int launch_recon_a(const ReconFields& f, const LevelConsts* lc, const Weights& w
                    dim3 block = dim3(32, 8));
 int launch_recon_b(const ReconFields& f, const Weights& wt, LevelDims d, bool first,
                    cudaStream_t st, dim3 block = dim3(32, 8));
-// The two-pixel half-steps (rf_pair.cuh) of levels where use_pairs(): A, and
-// B (`last`: a warp's last).  The multiplier update belongs to the A that
-// follows, so the two kinds of half-step do not mix within a warp.
-bool pair_weights(const Weights& wt);  // whether the weights fit them
-bool use_pairs(const Weights& wt, LevelDims d);
-int launch_recon_a2(const ReconFields& f, const LevelConsts* lc, const Weights& wt, LevelDims d,
-                    bool first, bool uc_from_buffer, int prior, cudaStream_t st);
-int launch_recon_b2(const ReconFields& f, const Weights& wt, LevelDims d, bool first, bool last,
-                    cudaStream_t st);
+// The half-steps of rf_pair.cuh, for weights that fit them: A, and B (`last`: a
+// warp's last).  The multiplier update belongs to the A that follows, so they
+// do not mix with launch_recon_a / _b within a warp.
+bool pair_weights(const Weights& wt);
+int launch_half_a(const ReconFields& f, const LevelConsts* lc, const Weights& wt, LevelDims d,
+                  bool first, bool uc_from_buffer, int prior, cudaStream_t st, dim3 block);
+int launch_half_b(const ReconFields& f, const Weights& wt, LevelDims d, bool first, bool last,
+                  cudaStream_t st, dim3 block);
 int launch_plain_data(float* duhat, float* dvhat, const float* pu1, const float* pu2,
                       const float* pv1, const float* pv2, const float* Ix, const float* Iy,
                       const float* Iz, const Weights& wt, LevelDims d, bool first,

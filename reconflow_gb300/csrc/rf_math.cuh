@@ -151,7 +151,7 @@ struct __align__(16) LevelConsts {
     float R1[9];
     float t1[3];
     float focal, cx, cy;
-    float pad;
+    float origin;  // 1: camera 0 at the origin, P = [f 0 cx 0; 0 g cy 0; 0 0 1 0]
 };
 
 // SolveUcKernel (solveUcSk.cu:21-33).

@@ -482,7 +482,7 @@ __device__ __forceinline__ void plain_data_px(float* duhat0, float* dvhat0,
                                               const float* __restrict__ pv2,
                                               const float* __restrict__ Ix,
                                               const float* __restrict__ Iy,
-                                              const float* __restrict__ Iz, const Weights& wt,
+                                              const float* __restrict__ Iz, const PlainWeights& wt,
                                               LevelDims d, int first, int ix, int iy) {
     const int s = d.s;
     const int pos = ix + iy * s;
@@ -517,7 +517,7 @@ __device__ __forceinline__ void plain_data_px(float* duhat0, float* dvhat0,
 __device__ __forceinline__ void plain_tv_px(const float* __restrict__ duhat,
                                             const float* __restrict__ dvhat, float* pu1,
                                             float* pu2, float* pv1, float* pv2,
-                                            const Weights& wt, LevelDims d, int first, int ix,
+                                            const PlainWeights& wt, LevelDims d, int first, int ix,
                                             int iy) {
     const int s = d.s;
     const int pos = ix + iy * s;

@@ -1,24 +1,29 @@
-// The two half-steps of a ReconFlow inner iteration, two pixels per thread.
+// The two half-steps of a ReconFlow inner iteration, one or two pixels per
+// thread.
 //
 // A (data term, projection blend, point solve: recon_a_px) and B (dual
 // update, 3x3 median and clean-up of the points, multiplier update:
-// recon_b_px) were bound by instruction issue (732 and 451 warp instructions
-// per 32 pixels).  Here a thread has the pixels (x, x + 1), x even, as the two
-// halves of packed FP32 instructions (rf_packed.cuh) and loads and stores them
-// as 64-bit vectors.  The
-// multiplier update moves from B to the next iteration's A, which reads all
-// its operands anyway (sk, u, duhat and uproj before A replaces them): B then
-// reads 9 planes and writes 7 instead of 15 and 9, and an iteration moves 172
-// bytes per pixel instead of 196.  The last B of a warp makes the update
-// itself, and leaves the dual update out: the next warp's dual field starts
-// from zero and nothing else reads it.
+// recon_b_px) were bound by instruction issue on large levels (732 and 451 warp
+// instructions per 32 pixels) and by the length of a pixel's chain of
+// instructions on small ones.
+// * Quotients and roots are rf_packed.cuh's: IEEE division's own sequence,
+//   with its check and branch, was a third of A's instructions.  A guard per
+//   thread covers all of them; where it fails the thread takes IEEE division.
+// * With camera 0 at the origin most products of the normal matrix are zeros
+//   and are not formed.
+// * The multiplier update moves from B to the next iteration's A, which reads
+//   all its operands anyway (sk, u, duhat and uproj before A replaces them): B
+//   then reads 9 planes and writes 7 instead of 15 and 9, and an iteration moves
+//   172 bytes per pixel instead of 196.  The last B of a warp makes the update
+//   itself, and leaves the dual update out: the next warp's dual field starts
+//   from zero and nothing else reads it.
+// * Large levels run two pixels (x, x + 1), x even, per thread, as the two
+//   halves of packed FP32 instructions, loaded and stored as 64-bit vectors.
 //
 // Every operation and its order are those of recon_a_px / recon_b_px, so every
-// value has the same bits; the quotients and roots are rf_packed.cuh's (IEEE
-// division's own sequence with its branch and check was a third of A's
-// instructions), with a guard per pair and IEEE division where it fails.
-// Needs a row stride that is a multiple of four and ordinary weights
-// (pair_stride, pair_weights); levels without run the one-pixel kernels.
+// value has the same bits.  Needs ordinary weights (pair_weights), pixel pairs
+// a row stride that is a multiple of four (pair_stride); other weights run
+// recon_a_px / recon_b_px.
 #pragma once
 
 #include <cstddef>
@@ -134,19 +139,27 @@ __device__ __forceinline__ float nmed3(float a, float b, float c) {
 }
 
 // median9_finite of a window whose median is a zero (the exchange order
-// decides its sign) or that holds a NaN; out of line, re-reading the window
-__device__ __noinline__ float median9_slow(const float* __restrict__ a, int x, int y, LevelDims d,
-                                           int base, long long n) {
-    (void)n;
-    float m[9];
+// decides its sign) or that holds a NaN; out of line, on the taps in registers
+// (re-reading them lengthened the longest thread of a small level's launch)
+__device__ __noinline__ float median9_slow(float a, float b, float c, float d, float e, float f,
+                                           float g, float h, float i) {
+    const float m[9] = {a, b, c, d, e, f, g, h, i};
+    // zeros of one sign only (points set to the origin are +0): that zero
+    bool nan = false, pos = false, neg = false;
 #pragma unroll
-    for (int j = 0; j < 3; j++)
-#pragma unroll
-        for (int i = 0; i < 3; i++) {
-            const int at = median3_tap(x + i - 1, y + j - 1, d.w, d.h, d.s);
-            m[j * 3 + i] = at >= 0 ? RF_PT(a, base + at, n) : 0.0f;
-        }
+    for (int k = 0; k < 9; k++) {
+        const unsigned bits = __float_as_uint(m[k]);
+        nan |= isnan(m[k]);
+        pos |= bits == 0u;
+        neg |= bits == 0x80000000u;
+    }
+    if (!nan && !(pos && neg)) return neg ? -0.0f : 0.0f;
     return median9_finite(m);
+}
+template <int N>
+__device__ __forceinline__ float median9_slow(const float (&t)[3][N], int i) {
+    return median9_slow(t[0][i], t[0][i + 1], t[0][i + 2], t[1][i], t[1][i + 1], t[1][i + 2],
+                        t[2][i], t[2][i + 1], t[2][i + 2]);
 }
 
 // Where a pair's 3x3 windows lie in its level.
@@ -203,32 +216,33 @@ __device__ __forceinline__ f2 median3_pair(const float (&t)[3][4]) {
 struct PointTaps {
     float x[3][4], y[3][4], z[3][4];
 };
-__device__ __forceinline__ void points_pair(const ReconFields& f, LevelDims d, int base, int x,
-                                            int y, PairEdges e, const PointTaps& t, f2& X, f2& Y,
+__device__ __forceinline__ void points_pair(PairEdges e, const PointTaps& t, f2& X, f2& Y,
                                             f2& Z) {
     const float(&tx)[3][4] = t.x, (&ty)[3][4] = t.y, (&tz)[3][4] = t.z;
     f2 Xm = median3_pair(tx), Ym = median3_pair(ty), Zm = median3_pair(tz);
     auto sure = [](float m) { return fabsf(m) > 0.0f; };  // neither zero nor NaN
     if (!(sure(Xm.x) && sure(Ym.x) && sure(Zm.x) && sure(Xm.y) && sure(Ym.y) && sure(Zm.y))) {
-        if (!sure(Xm.x)) Xm.x = median9_slow(f.X1, x, y, d, base, f.extent);
-        if (!sure(Ym.x)) Ym.x = median9_slow(f.Y1, x, y, d, base, f.extent);
-        if (!sure(Zm.x)) Zm.x = median9_slow(f.Z1, x, y, d, base, f.extent);
-        if (e.both && !sure(Xm.y)) Xm.y = median9_slow(f.X1, x + 1, y, d, base, f.extent);
-        if (e.both && !sure(Ym.y)) Ym.y = median9_slow(f.Y1, x + 1, y, d, base, f.extent);
-        if (e.both && !sure(Zm.y)) Zm.y = median9_slow(f.Z1, x + 1, y, d, base, f.extent);
+        if (!sure(Xm.x)) Xm.x = median9_slow(tx, 0);
+        if (!sure(Ym.x)) Ym.x = median9_slow(ty, 0);
+        if (!sure(Zm.x)) Zm.x = median9_slow(tz, 0);
+        if (e.both && !sure(Xm.y)) Xm.y = median9_slow(tx, 1);
+        if (e.both && !sure(Ym.y)) Ym.y = median9_slow(ty, 1);
+        if (e.both && !sure(Zm.y)) Zm.y = median9_slow(tz, 1);
     }
     cleanup_pixel(tx[1][1], ty[1][1], tz[1][1], Xm.x, Ym.x, Zm.x, X.x, Y.x, Z.x);
     cleanup_pixel(tx[1][2], ty[1][2], tz[1][2], Xm.y, Ym.y, Zm.y, X.y, Y.y, Z.y);
 }
 
-// dual_step (solveSmoothDualTVGlobal.cu:46-60) of two pixels (fac >= 0)
-__device__ __forceinline__ void dual_step2(f2 dx, f2 dy, f2 fac, f2& p1, f2& p2,
-                                           QuotientGuard& g) {
-    const f2 mag = sqrt2(dx * dx + dy * dy);
-    const f2 den = dup2(1.0f) + fac * mag;
-    const f2 nr = neg_recip2(den);
-    p1 = -neg_quot2(p1 + fac * dx, den, nr);
-    p2 = -neg_quot2(p2 + fac * dy, den, nr);
+// dual_step (solveSmoothDualTVGlobal.cu:46-60; fac >= 0)
+template <class V>
+__device__ __forceinline__ void dual_step_v(V dx, V dy, float facs, V& p1, V& p2,
+                                            QuotientGuard& g) {
+    const V fac = splat<V>(facs);
+    const V mag = sqrt_rn(dx * dx + dy * dy);
+    const V den = splat<V>(1.0f) + fac * mag;
+    const V nr = neg_recip(den);
+    p1 = -neg_quot(p1 + fac * dx, den, nr);
+    p2 = -neg_quot(p2 + fac * dy, den, nr);
     g.quot(mag);
     g.at_most(den);
     g.quot(p1);
@@ -261,8 +275,8 @@ __device__ __forceinline__ void dual_update(DualIn& in, float fac, PairEdges e) 
     if (!e.down) uy = vy = zero;
     QuotientGuard g;
     f2 pu1 = in.pu1, pu2 = in.pu2, pv1 = in.pv1, pv2 = in.pv2;
-    dual_step2(ux, uy, dup2(fac), pu1, pu2, g);
-    dual_step2(vx, vy, dup2(fac), pv1, pv2, g);
+    dual_step_v(ux, uy, fac, pu1, pu2, g);
+    dual_step_v(vx, vy, fac, pv1, pv2, g);
     // (a NaN in one of the four shows in their sum)
     const f2 sum = pu1 + pu2 + pv1 + pv2;
     if (g.ok() && isfinite(sum.x) && isfinite(sum.y)) {
@@ -276,151 +290,186 @@ __device__ __forceinline__ void dual_update(DualIn& in, float fac, PairEdges e) 
     }
 }
 
-// divergence (solveReconDataL1.cu:66-97) of two pixels; only the left one can
-// be in column 0
-__device__ __forceinline__ f2 divergence2(f2 p1, f2 p1l, f2 p2, f2 p2d, bool left, bool up) {
-    f2 t = p1 - p1l;
-    if (!left) t.x = p1.x;
+// what a holds for the first pixel (the only one that can be in column 0)
+// replaced by b's unless `keep`
+__device__ __forceinline__ void first_or(float& a, float b, bool keep) { a = keep ? a : b; }
+__device__ __forceinline__ void first_or(f2& a, f2 b, bool keep) { a.x = keep ? a.x : b.x; }
+
+// divergence (solveReconDataL1.cu:66-97)
+template <class V>
+__device__ __forceinline__ V divergence_v(V p1, V p1l, V p2, V p2d, bool left, bool up) {
+    V t = p1 - p1l;
+    first_or(t, p1, left);
     t = t + p2;
-    const f2 r = t - p2d;
+    const V r = t - p2d;
     return up ? r : t;
 }
 
-// Shared memory of a block: the level's constants and the weights as pairs of
-// equal floats, so that one 64-bit read gives a packed operand.
+// The level's constants and the weights by number, a value or an operand of
+// two.  For pixel pairs a block has them in shared memory as pairs of equal
+// floats, so that one 64-bit read gives a packed operand.
 enum {
     kCP = 0, kCQ = 12, kCR = 24, kCt = 33, kCf = 36, kCcx = 37, kCcy = 38, kCtv = 39, kCproj = 40,
     kCA = 41, kCpden = 42, kClf = 43, kClms = 44, kCfn = 45, kCHalf = 46, kClam = 47, kCnrA = 48,
     kCnrP = 49,
     // camera 0 at the origin (P = [f 0 cx 0; 0 g cy 0; 0 0 1 0]): f^2, g^2, and
-    // in kCorigin whether it is
+    // in kCorigin whether it is (LevelConsts::origin)
     kCff = 50, kCgg = 51, kCorigin = 52, kCount = 53
 };
 
+struct OneConsts {
+    const LevelConsts& c;
+    const Weights& wt;
+    __device__ __forceinline__ float operator()(int i) const {
+        if (i < kCQ) return c.P[i];
+        if (i < kCR) return c.Q[i - kCQ];
+        if (i < kCt) return c.R1[i - kCR];
+        if (i < kCf) return c.t1[i - kCt];
+        switch (i) {
+            case kCf: return c.focal;
+            case kCcx: return c.cx;
+            case kCcy: return c.cy;
+            case kCtv: return wt.alpha_tv;
+            case kCproj: return wt.alpha_proj;
+            case kCA: return wt.A;
+            case kCpden: return wt.proj_den;
+            case kClf: return wt.lambdaf;
+            case kClms: return wt.lambdams;
+            case kCfn: return wt.alpha_fn;
+            case kClam: return wt.lambda;
+            case kCnrA: return wt.nrA;
+            case kCnrP: return wt.nrP;
+            case kCff: return c.P[0] * c.P[0];
+            case kCgg: return c.P[5] * c.P[5];
+            case kCorigin: return c.origin;
+            default: return 0.5f;
+        }
+    }
+    __device__ __forceinline__ bool origin() const { return c.origin != 0.0f; }
+};
+
+struct PairConsts {
+    const float2* sc;
+    __device__ __forceinline__ f2 operator()(int i) const {
+        const float2 t = sc[i];
+        return f2{t.x, t.y};
+    }
+    __device__ __forceinline__ bool origin() const { return sc[kCorigin].x != 0.0f; }
+};
+
 __device__ __forceinline__ void pair_consts(const LevelConsts* __restrict__ lc, const Weights& wt,
-                                             float2* sc, int tid, int nthr) {
+                                            float2* sc, int tid, int nthr) {
+    const OneConsts c{*lc, wt};
     for (int i = tid; i < kCount; i += nthr) {
-        float v;
-        if (i < 39) v = reinterpret_cast<const float*>(lc)[i];  // P, Q, R1, t1, focal, cx, cy
-        else if (i == kCtv) v = wt.alpha_tv;
-        else if (i == kCproj) v = wt.alpha_proj;
-        else if (i == kCA) v = wt.A;
-        else if (i == kCpden) v = wt.proj_den;
-        else if (i == kClf) v = wt.lambdaf;
-        else if (i == kClms) v = wt.lambdams;
-        else if (i == kCfn) v = wt.alpha_fn;
-        else if (i == kClam) v = wt.lambda;
-        else if (i == kCnrA) v = -1.0f / wt.A;
-        else if (i == kCnrP) v = -1.0f / wt.proj_den;
-        else if (i == kCff) v = lc->P[0] * lc->P[0];
-        else if (i == kCgg) v = lc->P[5] * lc->P[5];
-        else if (i == kCorigin) {
-            bool o = lc->P[10] == 1.0f;
-            for (int k : {1, 3, 4, 7, 8, 9, 11}) o = o && __float_as_uint(lc->P[k]) == 0u;
-            v = o ? 1.0f : 0.0f;
-        } else v = 0.5f;
+        const float v = i < kCtv ? reinterpret_cast<const float*>(lc)[i] : c(i);
         sc[i] = make_float2(v, v);
     }
 }
 
-__device__ __forceinline__ f2 cst(const float2* sc, int i) {
-    const float2 t = sc[i];
-    return f2{t.x, t.y};
-}
-
-// project_uc (solveUcSk.cu:21-33) of two pixels
-__device__ __forceinline__ void project_uc2(const float2* sc, f2 X, f2 Y, f2 Z, f2 fx, f2 fy,
-                                            f2& uc, f2& vc, QuotientGuard& g) {
-    const f2 X2 = cst(sc, kCR + 0) * X + cst(sc, kCR + 1) * Y + cst(sc, kCR + 2) * Z + cst(sc, kCt + 0);
-    const f2 Y2 = cst(sc, kCR + 3) * X + cst(sc, kCR + 4) * Y + cst(sc, kCR + 5) * Z + cst(sc, kCt + 1);
-    const f2 Z2 = cst(sc, kCR + 6) * X + cst(sc, kCR + 7) * Y + cst(sc, kCR + 8) * Z + cst(sc, kCt + 2);
-    const f2 nr = neg_recip2(Z2);
-    const f2 nu = neg_quot2(cst(sc, kCf) * X2, Z2, nr), nv = neg_quot2(cst(sc, kCf) * Y2, Z2, nr);
+// project_uc (solveUcSk.cu:21-33)
+template <class V, class C>
+__device__ __forceinline__ void project_uc_v(const C& c, V X, V Y, V Z, V fx, V fy, V& uc, V& vc,
+                                             QuotientGuard& g) {
+    const V X2 = c(kCR + 0) * X + c(kCR + 1) * Y + c(kCR + 2) * Z + c(kCt + 0);
+    const V Y2 = c(kCR + 3) * X + c(kCR + 4) * Y + c(kCR + 5) * Z + c(kCt + 1);
+    const V Z2 = c(kCR + 6) * X + c(kCR + 7) * Y + c(kCR + 8) * Z + c(kCt + 2);
+    const V nr = neg_recip(Z2);
+    const V nu = neg_quot<V>(c(kCf) * X2, Z2, nr), nv = neg_quot<V>(c(kCf) * Y2, Z2, nr);
     g.div(Z2);
     g.quot_nonzero(nu);
     g.quot_nonzero(nv);
-    uc = cst(sc, kCcx) - nu - fx;
-    vc = cst(sc, kCcy) - nv - fy;
+    uc = c(kCcx) - nu - fx;
+    vc = c(kCcy) - nv - fy;
 }
 
-// l1_threshold (solveReconDataL1.cu:36-63) of two pixels
-__device__ __forceinline__ void l1_threshold2(f2 dusub, f2 dvsub, f2 dix, f2 diy, f2 dit, f2 lambda,
-                                              f2 A, f2 nrA, f2& du, f2& dv, QuotientGuard& g) {
-    const f2 rho = dix * dusub + diy * dvsub + dit;
-    const f2 magi = dix * dix + diy * diy;
-    const f2 nupper = neg_quot2(lambda * magi, A, nrA);  // = lower
+// l1_threshold (solveReconDataL1.cu:36-63): the branch's factor, with the sign
+// of its step, and its divisor; whether it steps at all (a NaN rho does not)
+__device__ __forceinline__ bool l1_branch(float rho, float nupper, float magi, float A, float lambda,
+                                          float& fac, float& den) {
+    const bool inside = rho <= -nupper && rho >= nupper;
+    const bool step = inside ? magi != 0.0f : (rho < nupper || rho > -nupper);
+    fac = inside ? rho : (rho < nupper ? -lambda : lambda);
+    den = step ? (inside ? magi : A) : 1.0f;
+    return step;
+}
+struct Steps {
+    bool x, y;
+};
+__device__ __forceinline__ bool l1_branches(float rho, float nupper, float magi, float A,
+                                            float lambda, float& fac, float& den) {
+    return l1_branch(rho, nupper, magi, A, lambda, fac, den);
+}
+__device__ __forceinline__ Steps l1_branches(f2 rho, f2 nupper, f2 magi, f2 A, f2 lambda, f2& fac,
+                                             f2& den) {
+    return Steps{l1_branch(rho.x, nupper.x, magi.x, A.x, lambda.x, fac.x, den.x),
+                 l1_branch(rho.y, nupper.y, magi.y, A.y, lambda.y, fac.y, den.y)};
+}
+__device__ __forceinline__ float choose(bool s, float a, float b) { return s ? a : b; }
+__device__ __forceinline__ f2 choose(Steps s, f2 a, f2 b) {
+    return f2{s.x ? a.x : b.x, s.y ? a.y : b.y};
+}
+template <class V>
+__device__ __forceinline__ void l1_threshold_v(V dusub, V dvsub, V dix, V diy, V dit, V lambda,
+                                               V A, V nrA, V& du, V& dv, QuotientGuard& g) {
+    const V rho = dix * dusub + diy * dvsub + dit;
+    const V magi = dix * dix + diy * diy;
+    const V nupper = neg_quot<V>(lambda * magi, A, nrA);  // = lower
     g.quot(nupper);
     g.at_most(nupper);
-    // the branch's factor, with the sign of its step, and divisor
-    auto branch = [&](float r, float nup, float m, float a, float lam, float& fac, float& den) {
-        const bool inside = r <= -nup && r >= nup;
-        const bool step = inside ? m != 0.0f : (r < nup || r > -nup);  // NaN rho: no step
-        fac = inside ? r : (r < nup ? -lam : lam);
-        den = step ? (inside ? m : a) : 1.0f;
-        return step;
-    };
-    f2 fac, den;
-    const bool sx = branch(rho.x, nupper.x, magi.x, A.x, lambda.x, fac.x, den.x);
-    const bool sy = branch(rho.y, nupper.y, magi.y, A.y, lambda.y, fac.y, den.y);
-    const f2 nr = neg_recip2(den);
-    const f2 nu = neg_quot2(fac * dix, den, nr), nv = neg_quot2(fac * diy, den, nr);
+    V fac, den;
+    const auto step = l1_branches(rho, nupper, magi, A, lambda, fac, den);
+    const V nr = neg_recip(den);
+    const V nu = neg_quot<V>(fac * dix, den, nr), nv = neg_quot<V>(fac * diy, den, nr);
     g.div(den);
     g.quot(nu);
     g.quot(nv);
-    du = dusub + nu;
-    dv = dvsub + nv;
-    if (!sx) {
-        du.x = dusub.x;
-        dv.x = dvsub.x;
-    }
-    if (!sy) {
-        du.y = dusub.y;
-        dv.y = dvsub.y;
-    }
+    du = choose(step, dusub + nu, dusub);
+    dv = choose(step, dvsub + nv, dvsub);
 }
 
-// solve3d_pixel (solve3dMinimalArea.cu:23-184) of two pixels (its operations
-// in its order; the symmetric entries of the normal matrix, whose products
-// commute bit for bit, are formed once)
-__device__ __forceinline__ void solve3d_pair(const float2* sc, f2 uproj, f2 vproj, f2 x1, f2 y1,
-                                             bool left, bool up, const f2 (&Xn)[5],
-                                             const f2 (&Yn)[5], const f2 (&Zn)[5], f2& Xo, f2& Yo,
-                                             f2& Zo, QuotientGuard& g) {
-    const f2 x2 = x1 + uproj, y2 = y1 + vproj;
-    f2 ax, bx, cx, dx, by, cy, dy, cz, dz;
+// solve3d_pixel (solve3dMinimalArea.cu:23-184; its operations in its order, the
+// symmetric entries of the normal matrix, whose products commute bit for bit,
+// formed once)
+template <class V, class C>
+__device__ __forceinline__ void solve3d_v(const C& c, V uproj, V vproj, V x1, V y1, bool left,
+                                          bool up, const V (&Xn)[5], const V (&Yn)[5],
+                                          const V (&Zn)[5], V& Xo, V& Yo, V& Zo,
+                                          QuotientGuard& g) {
+    const V x2 = x1 + uproj, y2 = y1 + vproj;
+    V ax, bx, cx, dx, by, cy, dy, cz, dz;
     {
-        f2 c8 = cst(sc, kCQ + 8), c9 = cst(sc, kCQ + 9), c10 = cst(sc, kCQ + 10),
-           c11 = cst(sc, kCQ + 11);
-        const f2 r1 = x2 * c8 - cst(sc, kCQ + 0), r2 = x2 * c9 - cst(sc, kCQ + 1),
-                 r3 = x2 * c10 - cst(sc, kCQ + 2), r4 = x2 * c11 - cst(sc, kCQ + 3);
-        const f2 s1 = y2 * c8 - cst(sc, kCQ + 4), s2 = y2 * c9 - cst(sc, kCQ + 5),
-                 s3 = y2 * c10 - cst(sc, kCQ + 6), s4 = y2 * c11 - cst(sc, kCQ + 7);
-        const f2 lf = cst(sc, kClf);
-        if (sc[kCorigin].x != 0.0f) {
+        V c8 = c(kCQ + 8), c9 = c(kCQ + 9), c10 = c(kCQ + 10),
+           c11 = c(kCQ + 11);
+        const V r1 = x2 * c8 - c(kCQ + 0), r2 = x2 * c9 - c(kCQ + 1),
+                 r3 = x2 * c10 - c(kCQ + 2), r4 = x2 * c11 - c(kCQ + 3);
+        const V s1 = y2 * c8 - c(kCQ + 4), s2 = y2 * c9 - c(kCQ + 5),
+                 s3 = y2 * c10 - c(kCQ + 6), s4 = y2 * c11 - c(kCQ + 7);
+        const V lf = c(kClf);
+        if (c.origin()) {
             // camera 0 at the origin: p = (-f, 0, x - cx, 0), q = (0, -g, y - cy, 0)
             // and most of their products are zeros, which leave the sums as they
             // are (but for the sign of a zero, which no point that is not zero
             // itself depends on; a zero point takes the slow path)
-            const f2 p3 = x1 - cst(sc, kCP + 2), q3 = y1 - cst(sc, kCP + 6);
-            const f2 nf = cst(sc, kCP + 0), ng = cst(sc, kCP + 5);
-            ax = lf * (cst(sc, kCff) + r1 * r1 + s1 * s1);
+            const V p3 = x1 - c(kCP + 2), q3 = y1 - c(kCP + 6);
+            const V nf = c(kCP + 0), ng = c(kCP + 5);
+            ax = lf * (c(kCff) + r1 * r1 + s1 * s1);
             bx = lf * (r1 * r2 + s1 * s2);
             cx = lf * (r1 * r3 - nf * p3 + s1 * s3);
             dx = lf * (r1 * r4 + s1 * s4);
-            by = lf * (cst(sc, kCgg) + r2 * r2 + s2 * s2);
+            by = lf * (c(kCgg) + r2 * r2 + s2 * s2);
             cy = lf * (r2 * r3 - ng * q3 + s2 * s3);
             dy = lf * (r2 * r4 + s2 * s4);
             cz = lf * (p3 * p3 + q3 * q3 + r3 * r3 + s3 * s3);
             dz = lf * (r3 * r4 + s3 * s4);
         } else {
-            c8 = cst(sc, kCP + 8);
-            c9 = cst(sc, kCP + 9);
-            c10 = cst(sc, kCP + 10);
-            c11 = cst(sc, kCP + 11);
-            const f2 p1 = x1 * c8 - cst(sc, kCP + 0), p2 = x1 * c9 - cst(sc, kCP + 1),
-                     p3 = x1 * c10 - cst(sc, kCP + 2), p4 = x1 * c11 - cst(sc, kCP + 3);
-            const f2 q1 = y1 * c8 - cst(sc, kCP + 4), q2 = y1 * c9 - cst(sc, kCP + 5),
-                     q3 = y1 * c10 - cst(sc, kCP + 6), q4 = y1 * c11 - cst(sc, kCP + 7);
+            c8 = c(kCP + 8);
+            c9 = c(kCP + 9);
+            c10 = c(kCP + 10);
+            c11 = c(kCP + 11);
+            const V p1 = x1 * c8 - c(kCP + 0), p2 = x1 * c9 - c(kCP + 1),
+                     p3 = x1 * c10 - c(kCP + 2), p4 = x1 * c11 - c(kCP + 3);
+            const V q1 = y1 * c8 - c(kCP + 4), q2 = y1 * c9 - c(kCP + 5),
+                     q3 = y1 * c10 - c(kCP + 6), q4 = y1 * c11 - c(kCP + 7);
             ax = lf * (p1 * p1 + q1 * q1 + r1 * r1 + s1 * s1);
             bx = lf * (p1 * p2 + q1 * q2 + r1 * r2 + s1 * s2);
             cx = lf * (p1 * p3 + q1 * q3 + r1 * r3 + s1 * s3);
@@ -433,26 +482,24 @@ __device__ __forceinline__ void solve3d_pair(const float2* sc, f2 uproj, f2 vpro
         }
     }
 
-    const f2 Xx = Xn[1] - Xn[0], Yx = Yn[1] - Yn[0], Zx = Zn[1] - Zn[0];
-    const f2 Xy = Xn[2] - Xn[0], Yy = Yn[2] - Yn[0], Zy = Zn[2] - Zn[0];
+    const V Xx = Xn[1] - Xn[0], Yx = Yn[1] - Yn[0], Zx = Zn[1] - Zn[0];
+    const V Xy = Xn[2] - Xn[0], Yy = Yn[2] - Yn[0], Zy = Zn[2] - Zn[0];
 
-    const f2 na = Yx * Zy - Zx * Yy, nb = Zx * Xy - Xx * Zy, nc = Xx * Yy - Yx * Xy;
-    const f2 area = na * na + nb * nb + nc * nc + dup2(0.001f);
-    const f2 root = sqrt2(area);  // at least sqrt(0.001)
+    const V na = Yx * Zy - Zx * Yy, nb = Zx * Xy - Xx * Zy, nc = Xx * Yy - Yx * Xy;
+    const V area = na * na + nb * nb + nc * nc + splat<V>(0.001f);
+    const V root = sqrt_rn(area);  // at least sqrt(0.001)
     // -lambdams / sqrt(area), and below everything it enters with the sign
     // turned: the quotients at the end turn it back
-    const f2 nlms = neg_quot2(cst(sc, kClms), root, neg_recip2(root));
+    const V nlms = neg_quot<V>(c(kClms), root, neg_recip(root));
     g.quot_nonzero(nlms);
 
-    const f2 half = cst(sc, kCHalf);
-    f2 Xi = half * Xn[3] + half * Xn[1], Yi = half * Yn[3] + half * Yn[1],
+    const V half = c(kCHalf);
+    V Xi = half * Xn[3] + half * Xn[1], Yi = half * Yn[3] + half * Yn[1],
        Zi = half * Zn[3] + half * Zn[1];
-    if (!left) {
-        Xi.x = Xn[1].x;
-        Yi.x = Yn[1].x;
-        Zi.x = Zn[1].x;
-    }
-    f2 Xj = half * Xn[4] + half * Xn[2], Yj = half * Yn[4] + half * Yn[2],
+    first_or(Xi, Xn[1], left);
+    first_or(Yi, Yn[1], left);
+    first_or(Zi, Zn[1], left);
+    V Xj = half * Xn[4] + half * Xn[2], Yj = half * Yn[4] + half * Yn[2],
        Zj = half * Zn[4] + half * Zn[2];
     if (!up) {
         Xj = Xn[2];
@@ -460,42 +507,42 @@ __device__ __forceinline__ void solve3d_pair(const float2* sc, f2 uproj, f2 vpro
         Zj = Zn[2];
     }
 
-    const f2 Xxx = Xx * Xx, Yxx = Yx * Yx, Zxx = Zx * Zx;
-    const f2 Xyy = Xy * Xy, Yyy = Yy * Yy, Zyy = Zy * Zy;
-    const f2 XYx = Xx * Yx, XYy = Xy * Yy, XZx = Xx * Zx, XZy = Xy * Zy, YZx = Yx * Zx,
+    const V Xxx = Xx * Xx, Yxx = Yx * Yx, Zxx = Zx * Zx;
+    const V Xyy = Xy * Xy, Yyy = Yy * Yy, Zyy = Zy * Zy;
+    const V XYx = Xx * Yx, XYy = Xy * Yy, XZx = Xx * Zx, XZy = Xy * Zy, YZx = Yx * Zx,
              YZy = Yy * Zy;
 
-    const f2 a11 = ax - nlms * (Yxx + Zxx + Yyy + Zyy);
-    const f2 a12 = bx + nlms * (XYx + XYy);
-    const f2 a13 = cx + nlms * (XZx + XZy);
-    const f2 a22 = by - nlms * (Xxx + Zxx + Xyy + Zyy);
-    const f2 a23 = cy + nlms * (YZx + YZy);
-    const f2 a33 = cz - nlms * (Xxx + Yxx + Xyy + Yyy);
+    const V a11 = ax - nlms * (Yxx + Zxx + Yyy + Zyy);
+    const V a12 = bx + nlms * (XYx + XYy);
+    const V a13 = cx + nlms * (XZx + XZy);
+    const V a22 = by - nlms * (Xxx + Zxx + Xyy + Zyy);
+    const V a23 = cy + nlms * (YZx + YZy);
+    const V a33 = cz - nlms * (Xxx + Yxx + Xyy + Yyy);
 
     // cofactors; with a21 = a12, a31 = a13, a32 = a23 the reference's E12, E13
     // and E23 are the same expressions as E21, E31 and E32
-    const f2 m2233 = a22 * a33, m2323 = a23 * a23, m1233 = a12 * a33, m2313 = a23 * a13,
+    const V m2233 = a22 * a33, m2323 = a23 * a23, m1233 = a12 * a33, m2313 = a23 * a13,
              m1223 = a12 * a23, m2213 = a22 * a13;
-    const f2 E11 = m2233 - m2323;
-    const f2 E12 = m2313 - m1233;
-    const f2 E13 = m1223 - m2213;
-    const f2 E22 = a11 * a33 - a13 * a13;
-    const f2 E23 = a13 * a12 - a11 * a23;
-    const f2 E33 = a11 * a22 - a12 * a12;
-    const f2 detA = a11 * E11 - a12 * (m1233 - m2313) + a13 * (m1223 - m2213);
+    const V E11 = m2233 - m2323;
+    const V E12 = m2313 - m1233;
+    const V E13 = m1223 - m2213;
+    const V E22 = a11 * a33 - a13 * a13;
+    const V E23 = a13 * a12 - a11 * a23;
+    const V E33 = a11 * a22 - a12 * a12;
+    const V detA = a11 * E11 - a12 * (m1233 - m2313) + a13 * (m1223 - m2213);
 
-    const f2 nXYy = -XYy, nXZy = -XZy;
-    const f2 nb1 = nlms * ((Zyy + Yyy) * Xi + (Zxx + Yxx) * Xj - XYy * Yi - XYx * Yj - XZy * Zi -
+    const V nXYy = -XYy, nXZy = -XZy;
+    const V nb1 = nlms * ((Zyy + Yyy) * Xi + (Zxx + Yxx) * Xj - XYy * Yi - XYx * Yj - XZy * Zi -
                          XZx * Zj) + dx;
-    const f2 nb2 = nlms * (nXYy * Xi - XYx * Xj + (Xyy + Zyy) * Yi + (Xxx + Zxx) * Yj - YZy * Zi -
+    const V nb2 = nlms * (nXYy * Xi - XYx * Xj + (Xyy + Zyy) * Yi + (Xxx + Zxx) * Yj - YZy * Zi -
                          YZx * Zj) + dy;
-    const f2 nb3 = nlms * (nXZy * Xi - XZx * Xj - YZy * Yi - YZx * Yj + (Xyy + Yyy) * Zi +
+    const V nb3 = nlms * (nXZy * Xi - XZx * Xj - YZy * Yi - YZx * Yj + (Xyy + Yyy) * Zi +
                          (Xxx + Yxx) * Zj) + dz;
 
-    const f2 nr = neg_recip2(detA);
-    Xo = neg_quot2(E11 * nb1 + E12 * nb2 + E13 * nb3, detA, nr);
-    Yo = neg_quot2(E12 * nb1 + E22 * nb2 + E23 * nb3, detA, nr);
-    Zo = neg_quot2(E13 * nb1 + E23 * nb2 + E33 * nb3, detA, nr);
+    const V nr = neg_recip(detA);
+    Xo = neg_quot<V>(E11 * nb1 + E12 * nb2 + E13 * nb3, detA, nr);
+    Yo = neg_quot<V>(E12 * nb1 + E22 * nb2 + E23 * nb3, detA, nr);
+    Zo = neg_quot<V>(E13 * nb1 + E23 * nb2 + E33 * nb3, detA, nr);
     g.div(detA);
     g.quot_nonzero(Xo);
     g.quot_nonzero(Yo);
@@ -574,40 +621,41 @@ __device__ __forceinline__ void recon_a_pair(const ReconFields& f, const LevelCo
     }
     __syncthreads();
     if (!inside) return;
+    const PairConsts c{sc};
     f2 divu = zero, divv = zero;  // of a zero dual field: +0
     if (!first) {
         // multiplier update of the previous B (solveUcSk.cu:94-95)
         sku = sku + u + duhat - uproj;
         skv = skv + v + dvhat - vproj;
-        divu = divergence2(pu1, mk2(pu1l, pu1.x), pu2, pu2d, left, up);
-        divv = divergence2(pv1, mk2(pv1l, pv1.x), pv2, pv2d, left, up);
+        divu = divergence_v(pu1, mk2(pu1l, pu1.x), pu2, pu2d, left, up);
+        divv = divergence_v(pv1, mk2(pv1l, pv1.x), pv2, pv2d, left, up);
     }
 
     // --- data step (solveReconDataL1.cu:24-100) ---
-    const f2 atv = cst(sc, kCtv), aproj = cst(sc, kCproj);
+    const f2 atv = c(kCtv), aproj = c(kCproj);
     QuotientGuard g;
     f2 A, nrA, nu, nv;
     const f2 ru = uproj - u - sku, rv = vproj - v - skv;
     if (PRIOR == 0) {
-        A = cst(sc, kCA);
-        nrA = cst(sc, kCnrA);
-        nu = neg_quot2(atv * duhat + aproj * ru, A, nrA);
-        nv = neg_quot2(atv * dvhat + aproj * rv, A, nrA);
+        A = c(kCA);
+        nrA = c(kCnrA);
+        nu = neg_quot<f2>(atv * duhat + aproj * ru, A, nrA);
+        nv = neg_quot<f2>(atv * dvhat + aproj * rv, A, nrA);
     } else {
-        f2 afn = cst(sc, kCfn);
+        f2 afn = c(kCfn);
         if (PRIOR == 2) afn = afn * RF_LD2(f, mask, pos);
         A = atv + aproj + afn;
-        nrA = neg_recip2(A);
+        nrA = neg_recip(A);
         g.div(A);
         const f2 ufn = RF_LD2(f, ufn, pos), vfn = RF_LD2(f, vfn, pos);
-        nu = neg_quot2(afn * (ufn - u) + atv * duhat + aproj * ru, A, nrA);
-        nv = neg_quot2(afn * (vfn - v) + atv * dvhat + aproj * rv, A, nrA);
+        nu = neg_quot<f2>(afn * (ufn - u) + atv * duhat + aproj * ru, A, nrA);
+        nv = neg_quot<f2>(afn * (vfn - v) + atv * dvhat + aproj * rv, A, nrA);
     }
     g.quot(nu);
     g.quot(nv);
     f2 du, dv;
-    l1_threshold2(-nu, -nv, dix, diy, dit, cst(sc, kClam), A, nrA, du, dv, g);
-    const f2 ndu = neg_quot2(divu, A, nrA), ndv = neg_quot2(divv, A, nrA);
+    l1_threshold_v(-nu, -nv, dix, diy, dit, c(kClam), A, nrA, du, dv, g);
+    const f2 ndu = neg_quot<f2>(divu, A, nrA), ndv = neg_quot<f2>(divv, A, nrA);
     g.quot(ndu);
     g.quot(ndv);
     const f2 duhat1 = du - ndu, dvhat1 = dv - ndv;
@@ -619,17 +667,17 @@ __device__ __forceinline__ void recon_a_pair(const ReconFields& f, const LevelCo
         uc = RF_LD2(f, uc, pos);
         vc = RF_LD2(f, vc, pos);
     } else {
-        project_uc2(sc, Xn[0], Yn[0], Zn[0], fx, fy, uc, vc, g);
+        project_uc_v(c, Xn[0], Yn[0], Zn[0], fx, fy, uc, vc, g);
     }
-    const f2 lf = cst(sc, kClf), pden = cst(sc, kCpden), nrP = cst(sc, kCnrP);
-    uproj = -neg_quot2(lf * uc + aproj * (u + duhat1 + sku), pden, nrP);
-    vproj = -neg_quot2(lf * vc + aproj * (v + dvhat1 + skv), pden, nrP);
+    const f2 lf = c(kClf), pden = c(kCpden), nrP = c(kCnrP);
+    uproj = -neg_quot<f2>(lf * uc + aproj * (u + duhat1 + sku), pden, nrP);
+    vproj = -neg_quot<f2>(lf * vc + aproj * (v + dvhat1 + skv), pden, nrP);
     g.quot_nonzero(uproj);
     g.quot_nonzero(vproj);
 
     // --- triangulation with minimal-area smoothing ---
     f2 Xo, Yo, Zo;
-    solve3d_pair(sc, uproj, vproj, fx, fy, left, up, Xn, Yn, Zn, Xo, Yo, Zo, g);
+    solve3d_v(c, uproj, vproj, fx, fy, left, up, Xn, Yn, Zn, Xo, Yo, Zo, g);
     // any quotient that is not sure, or anything that is not finite (it
     // reaches the points): the pixels with IEEE divisions
     if (!(g.ok() && finite3(Xo.x, Yo.x, Zo.x) && finite3(Xo.y, Yo.y, Zo.y))) {
@@ -727,7 +775,7 @@ __device__ __forceinline__ void recon_b_tile(const ReconFields& f, const Weights
     load_taps(my + S::off(1), e, t.y);
     load_taps(my + S::off(2), e, t.z);
     f2 X, Y, Z;
-    points_pair(f, d, base, x, y, e, t, X, Y, Z);
+    points_pair(e, t, X, Y, Z);
     if (LAST) {
         const f2 u = RF_LD2(f, u, pos), v = RF_LD2(f, v, pos);
         const f2 uproj = RF_LD2(f, uproj, pos), vproj = RF_LD2(f, vproj, pos);
@@ -756,6 +804,217 @@ __device__ __forceinline__ void recon_b_tile(const ReconFields& f, const Weights
     RF_ST2(f, X, pos, X, e.both);
     RF_ST2(f, Y, pos, Y, e.both);
     RF_ST2(f, Z, pos, Z, e.both);
+}
+
+// ---- one pixel per thread ---------------------------------------------------
+// A at a pixel (recon_a_px with the multiplier update first and the quotients
+// above).
+template <int PRIOR>
+__device__ __forceinline__ void recon_a_one(const ReconFields& f, const LevelConsts& lc,
+                                            const Weights& wt, LevelDims d, int base, int x, int y,
+                                            bool first, bool uc_from_buffer) {
+    const int s = d.s, pos = base + x + y * s;
+    const bool left = x > 0, up = y > 0;
+    // every load before any arithmetic, as in recon_a_px
+    const float u = RF_AT(f, u, pos), v = RF_AT(f, v, pos);
+    const float dix = RF_AT(f, Ix, pos), diy = RF_AT(f, Iy, pos), dit = RF_AT(f, Iz, pos);
+    float uproj = RF_AT(f, uproj, pos), vproj = RF_AT(f, vproj, pos);
+    float sku = RF_AT(f, sku, pos), skv = RF_AT(f, skv, pos);
+    float duhat = 0.0f, dvhat = 0.0f, pu1 = 0.0f, pu2 = 0.0f, pv1 = 0.0f, pv2 = 0.0f;
+    float pu1l = 0.0f, pv1l = 0.0f, pu2d = 0.0f, pv2d = 0.0f;
+    if (!first) {
+        duhat = RF_AT(f, duhat, pos);
+        dvhat = RF_AT(f, dvhat, pos);
+        pu1 = RF_AT(f, pu1, pos);
+        pu2 = RF_AT(f, pu2, pos);
+        pv1 = RF_AT(f, pv1, pos);
+        pv2 = RF_AT(f, pv2, pos);
+        if (left) {
+            pu1l = RF_AT(f, pu1, pos - 1);
+            pv1l = RF_AT(f, pv1, pos - 1);
+        }
+        if (up) {
+            pu2d = RF_AT(f, pu2, pos - s);
+            pv2d = RF_AT(f, pv2, pos - s);
+        }
+    }
+    float Xn[5], Yn[5], Zn[5];
+    auto around = [&](const float* a, float (&n)[5]) {
+        n[0] = RF_PT(a, pos, f.extent);
+        n[1] = RF_PT(a, pos + 1, f.extent);
+        n[2] = RF_PT(a, pos + s, f.extent);
+        n[3] = left ? RF_PT(a, pos - 1, f.extent) : 0.0f;
+        n[4] = up ? RF_PT(a, pos - s, f.extent) : 0.0f;
+    };
+    around(f.X, Xn);
+    around(f.Y, Yn);
+    around(f.Z, Zn);
+    float uc = 0.0f, vc = 0.0f, ufn = 0.0f, vfn = 0.0f, mk = 1.0f;
+    if (uc_from_buffer) {
+        uc = RF_AT(f, uc, pos);
+        vc = RF_AT(f, vc, pos);
+    }
+    if (PRIOR != 0) {
+        ufn = RF_AT(f, ufn, pos);
+        vfn = RF_AT(f, vfn, pos);
+        if (PRIOR == 2) mk = RF_AT(f, mask, pos);
+    }
+
+    const OneConsts c{lc, wt};
+    float divu = 0.0f, divv = 0.0f;
+    if (!first) {
+        sku = sku + u + duhat - uproj;
+        skv = skv + v + dvhat - vproj;
+        divu = divergence_v(pu1, pu1l, pu2, pu2d, left, up);
+        divv = divergence_v(pv1, pv1l, pv2, pv2d, left, up);
+    }
+    QuotientGuard g;
+    float A, nrA, nu, nv;
+    const float ru = uproj - u - sku, rv = vproj - v - skv;
+    if (PRIOR == 0) {
+        A = wt.A;
+        nrA = wt.nrA;
+        nu = neg_quot(wt.alpha_tv * duhat + wt.alpha_proj * ru, A, nrA);
+        nv = neg_quot(wt.alpha_tv * dvhat + wt.alpha_proj * rv, A, nrA);
+    } else {
+        const float afn = PRIOR == 2 ? wt.alpha_fn * mk : wt.alpha_fn;
+        A = wt.alpha_tv + wt.alpha_proj + afn;
+        nrA = neg_recip(A);
+        g.div(A);
+        nu = neg_quot(afn * (ufn - u) + wt.alpha_tv * duhat + wt.alpha_proj * ru, A, nrA);
+        nv = neg_quot(afn * (vfn - v) + wt.alpha_tv * dvhat + wt.alpha_proj * rv, A, nrA);
+    }
+    g.quot(nu);
+    g.quot(nv);
+    float du, dv;
+    l1_threshold_v(-nu, -nv, dix, diy, dit, wt.lambda, A, nrA, du, dv, g);
+    const float ndu = neg_quot(divu, A, nrA), ndv = neg_quot(divv, A, nrA);
+    g.quot(ndu);
+    g.quot(ndv);
+    duhat = du - ndu;
+    dvhat = dv - ndv;
+    const float fx = (float)x, fy = (float)y;
+    if (!uc_from_buffer) project_uc_v(c, Xn[0], Yn[0], Zn[0], fx, fy, uc, vc, g);
+    uproj = -neg_quot(wt.lambdaf * uc + wt.alpha_proj * (u + duhat + sku), wt.proj_den, wt.nrP);
+    vproj = -neg_quot(wt.lambdaf * vc + wt.alpha_proj * (v + dvhat + skv), wt.proj_den, wt.nrP);
+    g.quot_nonzero(uproj);
+    g.quot_nonzero(vproj);
+    float Xo, Yo, Zo;
+    solve3d_v(c, uproj, vproj, fx, fy, left, up, Xn, Yn, Zn, Xo, Yo, Zo, g);
+    if (!(g.ok() && finite3(Xo, Yo, Zo))) {
+        recon_a_slow<PRIOR>(f, &lc, wt, d, base, x, y, first, uc_from_buffer);
+        return;
+    }
+    if (!first) {
+        RF_AT(f, sku, pos) = sku;
+        RF_AT(f, skv, pos) = skv;
+    }
+    RF_AT(f, duhat, pos) = duhat;
+    RF_AT(f, dvhat, pos) = dvhat;
+    RF_AT(f, uproj, pos) = uproj;
+    RF_AT(f, vproj, pos) = vproj;
+    RF_AT(f, X1, pos) = Xo;
+    RF_AT(f, Y1, pos) = Yo;
+    RF_AT(f, Z1, pos) = Zo;
+}
+
+// the 3x3 taps of a pixel, border rules as load_taps
+__device__ __forceinline__ void load_taps_one(const float* a, int p, int s, long long n,
+                                              PairEdges e, float (&t)[3][3]) {
+#pragma unroll
+    for (int j = 0; j < 3; j++) {
+        const int q = j == 0 ? (e.up ? p - s : p) : (j == 1 ? p : p + s);
+        const bool in = j != 2 || e.down;
+        const float c = in ? RF_PT(a, q, n) : 0.0f;
+        t[j][0] = !in ? 0.0f : (e.left ? RF_PT(a, q - 1, n) : (j != 0 || e.up ? c : 0.0f));
+        t[j][1] = c;
+        t[j][2] = in && e.both ? RF_PT(a, q + 1, n) : 0.0f;
+    }
+}
+__device__ __forceinline__ float median3_one(const float (&t)[3][3]) {
+    float lo[3], mid[3], hi[3];
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+        const float s = nmin(t[0][i], t[1][i]), g = nmax(t[0][i], t[1][i]);
+        lo[i] = nmin(s, t[2][i]);
+        hi[i] = nmax(g, t[2][i]);
+        mid[i] = nmax(s, nmin(g, t[2][i]));
+    }
+    return nmed3(nmax3(lo[0], lo[1], lo[2]), nmed3(mid[0], mid[1], mid[2]),
+                 nmin3(hi[0], hi[1], hi[2]));
+}
+
+// B at a pixel (recon_b_px without the multiplier update); LAST as
+// recon_b_tile.
+template <bool LAST>
+__device__ __forceinline__ void recon_b_one(const ReconFields& f, const Weights& wt, LevelDims d,
+                                            int base, int x, int y, bool first) {
+    const int s = d.s, pos = base + x + y * s;
+    // `both`, `right`: x + 1 < w
+    const PairEdges e{x > 0, x + 1 < d.w, x + 1 < d.w, y > 0, y + 1 < d.h};
+    float tx[3][3], ty[3][3], tz[3][3];
+    load_taps_one(f.X1, pos, s, f.extent, e, tx);
+    load_taps_one(f.Y1, pos, s, f.extent, e, ty);
+    load_taps_one(f.Z1, pos, s, f.extent, e, tz);
+    const float duhat = RF_AT(f, duhat, pos), dvhat = RF_AT(f, dvhat, pos);
+    float a[6] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+    float ux = 0.0f, uy = 0.0f, vx = 0.0f, vy = 0.0f;
+    if (LAST) {
+        a[0] = RF_AT(f, u, pos);
+        a[1] = RF_AT(f, v, pos);
+        a[2] = RF_AT(f, uproj, pos);
+        a[3] = RF_AT(f, vproj, pos);
+        a[4] = RF_AT(f, sku, pos);
+        a[5] = RF_AT(f, skv, pos);
+    } else {
+        if (!first) {
+            a[0] = RF_AT(f, pu1, pos);
+            a[1] = RF_AT(f, pu2, pos);
+            a[2] = RF_AT(f, pv1, pos);
+            a[3] = RF_AT(f, pv2, pos);
+        }
+        if (e.both) {
+            ux = RF_AT(f, duhat, pos + 1) - duhat;
+            vx = RF_AT(f, dvhat, pos + 1) - dvhat;
+        }
+        if (e.down) {
+            uy = RF_AT(f, duhat, pos + s) - duhat;
+            vy = RF_AT(f, dvhat, pos + s) - dvhat;
+        }
+    }
+    float Xm = median3_one(tx), Ym = median3_one(ty), Zm = median3_one(tz);
+    auto sure = [](float m) { return fabsf(m) > 0.0f; };
+    if (!(sure(Xm) && sure(Ym) && sure(Zm))) {
+        if (!sure(Xm)) Xm = median9_slow(tx, 0);
+        if (!sure(Ym)) Ym = median9_slow(ty, 0);
+        if (!sure(Zm)) Zm = median9_slow(tz, 0);
+    }
+    float X, Y, Z;
+    cleanup_pixel(tx[1][1], ty[1][1], tz[1][1], Xm, Ym, Zm, X, Y, Z);
+    if (LAST) {
+        RF_AT(f, sku, pos) = a[4] + a[0] + duhat - a[2];
+        RF_AT(f, skv, pos) = a[5] + a[1] + dvhat - a[3];
+    } else {
+        QuotientGuard g;
+        float pu1 = a[0], pu2 = a[1], pv1 = a[2], pv2 = a[3];
+        dual_step_v(ux, uy, wt.fac, pu1, pu2, g);
+        dual_step_v(vx, vy, wt.fac, pv1, pv2, g);
+        if (!(g.ok() && isfinite(pu1 + pu2 + pv1 + pv2))) {
+            const float2 pu = dual_step_slow(ux, uy, wt.fac, a[0], a[1]);
+            const float2 pv = dual_step_slow(vx, vy, wt.fac, a[2], a[3]);
+            pu1 = pu.x;
+            pu2 = pu.y;
+            pv1 = pv.x;
+            pv2 = pv.y;
+        }
+        RF_AT(f, pu1, pos) = pu1;
+        RF_AT(f, pu2, pos) = pu2;
+        RF_AT(f, pv1, pos) = pv1;
+        RF_AT(f, pv2, pos) = pv2;
+    }
+    RF_AT(f, X, pos) = X;
+    RF_AT(f, Y, pos) = Y;
+    RF_AT(f, Z, pos) = Z;
 }
 
 }  // namespace

@@ -163,6 +163,8 @@ Weights make_weights(const rf_params& p) {
     w.lambdams = p.lambdams;
     w.proj_den = p.lambdaf + p.alpha_proj;
     w.theta = p.theta;
+    w.nrA = -1.0f / w.A;
+    w.nrP = -1.0f / w.proj_den;
     if (p.method == RF_METHOD_TVL1) {
         w.fac = p.tau / p.theta;
     } else {
@@ -222,7 +224,9 @@ void rf::camera_level_consts(const double* K0in, const double* K1in, int L, floa
         c.focal = (float)K1[0];
         c.cx = (float)K1[2];
         c.cy = (float)K1[5];
-        c.pad = 0.0f;
+        bool origin = c.P[10] == 1.0f;
+        for (int k : {1, 3, 4, 7, 8, 9, 11}) origin = origin && c.P[k] == 0.0f && !std::signbit(c.P[k]);
+        c.origin = origin ? 1.0f : 0.0f;
     }
 }
 
@@ -355,13 +359,13 @@ rf_status enqueue_recon(rf_handle* h, float** res_u, float** res_v, bool warm = 
                 uc_in_buffer = false;
             }
             for (int iter = 0; iter < n_iters && !use_cluster_at(h, d); iter++) {
-                if (use_pairs(wt, d)) {
-                    RF_LAUNCH(launch_recon_a2(f, lc, wt, d, iter == 0, uc_in_buffer, prior, st));
-                    RF_LAUNCH(launch_recon_b2(f, wt, d, iter == 0, iter + 1 == n_iters, st));
+                const dim3 tile(h->tile_w[level], h->tile_h[level]);
+                if (pair_weights(wt)) {
+                    RF_LAUNCH(launch_half_a(f, lc, wt, d, iter == 0, uc_in_buffer, prior, st, tile));
+                    RF_LAUNCH(launch_half_b(f, wt, d, iter == 0, iter + 1 == n_iters, st, tile));
                     uc_in_buffer = false;
                     continue;
                 }
-                const dim3 tile(h->tile_w[level], h->tile_h[level]);
                 RF_LAUNCH(launch_recon_a(f, lc, wt, d, iter == 0, uc_in_buffer, prior, st, tile));
                 RF_LAUNCH(launch_recon_b(f, wt, d, iter == 0, st, tile));
                 uc_in_buffer = false;
@@ -1061,14 +1065,15 @@ rf_status rf_profile_iterations(rf_handle* h, int level, int n_iters, float* ms)
         RF_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
         int bad = 0;
         for (int i = 0; i < n_iters && !bad; i++) {
-            if (recon && use_pairs(wt, d))
-                bad = k == 0 ? launch_recon_a2(f, h->d_consts + level, wt, d, false, false, prior, st)
-                             : launch_recon_b2(f, wt, d, false, false, st);
+            const dim3 tile(h->tile_w[level], h->tile_h[level]);
+            if (recon && pair_weights(wt))
+                bad = k == 0 ? launch_half_a(f, h->d_consts + level, wt, d, false, false, prior, st,
+                                             tile)
+                             : launch_half_b(f, wt, d, false, false, st, tile);
             else if (recon)
                 bad = k == 0 ? launch_recon_a(f, h->d_consts + level, wt, d, false, false, prior, st,
-                                              dim3(h->tile_w[level], h->tile_h[level]))
-                             : launch_recon_b(f, wt, d, false, st,
-                                              dim3(h->tile_w[level], h->tile_h[level]));
+                                              tile)
+                             : launch_recon_b(f, wt, d, false, st, tile);
             else
                 bad = k == 0 ? launch_plain_data(h->duhat, h->dvhat, h->pu1, h->pu2, h->pv1,
                                                  h->pv2, h->Ix, h->Iy, h->Iz, wt, d, false, st)
