@@ -236,7 +236,8 @@ RF_API rf_status rf_host_free(void* ptr);
  * graph as the solve captures them, the graph replay timed with CUDA events;
  * returns the mean time per launch in milliseconds (ms[0] = data /
  * projection / triangulation kernel, ms[1] = dual / median / clean-up
- * kernel; plain TV-L1: data, dual).  Changes the solver state; results of
+ * kernel; plain TV-L1: data, dual as launches of their own, where its solve
+ * runs several iterations per launch).  Changes the solver state; results of
  * the last solve are no longer valid afterwards. */
 RF_API rf_status rf_profile_iterations(rf_handle* h, int level, int n_iters, float* ms);
 

@@ -26,6 +26,7 @@
 #include "rf_kernels.cuh"
 #include "rf_ops.cuh"
 #include "rf_pair.cuh"
+#include "rf_plain.cuh"
 
 namespace {
 
@@ -861,6 +862,40 @@ bool cluster_supported() {
         cudaGetLastError();
     }
     return v == 1;
+}
+
+namespace {
+template <int R, int WARPS, int K>
+int plain_tiles(PlainState a, PlainState b, const float* Ix, const float* Iy, const float* Iz,
+                const Weights& wt, LevelDims d, int n_iters, cudaStream_t st, int* in_b) {
+    using T = PlainTile<R, WARPS, K>;
+    const dim3 g((d.w + T::W - 1) / T::W, (d.h + T::H - 1) / T::H);
+    int launches = 0;
+    for (int done = 0; done < n_iters; done += K, launches++) {
+        const int n = n_iters - done < K ? n_iters - done : K;
+        k_plain_tile<R, WARPS, K><<<g, T::THREADS, 0, st>>>(
+            launches & 1 ? a : b, launches & 1 ? b : a, Ix, Iy, Iz, wt, d, n, done == 0,
+            done + n == n_iters);
+        if (check_launch() != 0) return -1;
+    }
+    *in_b = launches & 1 ? 0 : 1;
+    return launches;
+}
+}  // namespace
+
+int launch_plain_warp(PlainState a, PlainState b, const float* Ix, const float* Iy,
+                      const float* Iz, const Weights& wt, LevelDims d, int n_iters,
+                      cudaStream_t st, int* in_b) {
+    // Large levels are bound by the work, which the ring adds to (24 x 24 of a
+    // region of 32 x 32; K = 3 and 5, 8 and 10 warps, 3 or 4 rows are 2-10% slower
+    // at 640x480 and 720p).  On small ones a block's own time per launch counts:
+    // fewer pixels per block, more iterations per launch (solve of 64x48, all
+    // five levels small: 0.90 ms against 1.22; K = 4, 5 and 8: 0.94, 1.00, 0.91).
+    // Between them, 320x240 within a 640x480 solve: 1.49 ms as a large level, 1.67
+    // as a small one; 200x150: 0.98 as a small one, 1.27 as a large one.
+    if ((long long)d.w * d.h >= 60000)
+        return plain_tiles<2, 16, 4>(a, b, Ix, Iy, Iz, wt, d, n_iters, st, in_b);
+    return plain_tiles<1, 20, 6>(a, b, Ix, Iy, Iz, wt, d, n_iters, st, in_b);
 }
 
 int launch_plain_data(float* duhat, float* dvhat, const float* pu1, const float* pu2,

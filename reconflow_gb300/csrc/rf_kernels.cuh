@@ -163,6 +163,13 @@ int launch_half_a(const ReconFields& f, const LevelConsts* lc, const Weights& wt
                   bool first, bool uc_from_buffer, int prior, cudaStream_t st, dim3 block);
 int launch_half_b(const ReconFields& f, const Weights& wt, LevelDims d, bool first, bool last,
                   cudaStream_t st, dim3 block);
+// All inner iterations of a plain TV-L1 warp, several per launch (rf_plain.cuh;
+// wt.fac >= 0, n_iters > 0), between the state planes `a` and `b` of which
+// nothing is read before it is written; *in_b: whether the final duhat is b's.  Returns the number of launches, < 0 if one failed.
+struct PlainState;
+int launch_plain_warp(PlainState a, PlainState b, const float* Ix, const float* Iy,
+                      const float* Iz, const Weights& wt, LevelDims d, int n_iters,
+                      cudaStream_t st, int* in_b);
 int launch_plain_data(float* duhat, float* dvhat, const float* pu1, const float* pu2,
                       const float* pv1, const float* pv2, const float* Ix, const float* Iy,
                       const float* Iz, const Weights& wt, LevelDims d, bool first,

@@ -21,6 +21,7 @@
 #include "rf_alloc.h"
 #include "rf_nvtx.h"
 #include "rf_kernels.cuh"
+#include "rf_plain.cuh"
 
 using namespace rf;
 
@@ -443,7 +444,23 @@ rf_status enqueue_plain(rf_handle* h, float** res_u, float** res_v, bool warm = 
             NvtxRange warp_range("level %d warp %d", level, warp);
             RF_LAUNCH(launch_warp_deriv(h->I0[level], h->I1[level], u, v, d, h->Ix, h->Iy,
                                         h->Iz, st));
-            for (int iter = 0; iter < n_iters; iter++) {
+            const float *duhat = h->duhat, *dvhat = h->dvhat;  // the last iteration's
+            const bool tiled = n_iters > 0 && wt.fac >= 0.0f;
+            if (tiled) {
+                // the second state in planes that hold nothing while a level's
+                // iterations run (warm[2..4] are only read by ReconFlow solves)
+                const PlainState a{h->duhat, h->dvhat, h->pu1, h->pu2, h->pv1, h->pv2};
+                const PlainState b{us, vs, h->i1w, h->scratch, h->warm[2], h->warm[3]};
+                int in_b = 0;
+                const int k = launch_plain_warp(a, b, h->Ix, h->Iy, h->Iz, wt, d, n_iters, st, &in_b);
+                if (k < 0) return cuda_fail(rf::last_launch_error(), "kernel launch plain iterations");
+                h->enqueue_launches += k;
+                if (in_b) {
+                    duhat = b.du;
+                    dvhat = b.dv;
+                }
+            }
+            for (int iter = 0; iter < n_iters && !tiled; iter++) {
                 RF_LAUNCH(launch_plain_data(h->duhat, h->dvhat, h->pu1, h->pu2, h->pv1, h->pv2,
                                             h->Ix, h->Iy, h->Iz, wt, d, iter == 0, st));
                 RF_LAUNCH(launch_plain_tv(h->duhat, h->dvhat, h->pu1, h->pu2, h->pv1, h->pv2, wt,
@@ -454,7 +471,7 @@ rf_status enqueue_plain(rf_handle* h, float** res_u, float** res_v, bool warm = 
                 RF_CUDA(cudaMemsetAsync(h->dvhat, 0, plane_bytes, st));
             }
             // Cudaflow.cu:580-587: median of duhat, u += it (no median of u)
-            RF_LAUNCH(launch_median_add(h->duhat, h->dvhat, u, v, u, v, d, st));
+            RF_LAUNCH(launch_median_add(duhat, dvhat, u, v, u, v, d, st));
         }
         if (level > 0) {
             LevelDims fd{h->W[level - 1], h->H[level - 1], h->S[level - 1]};
