@@ -27,6 +27,7 @@
 #include "rf_ops.cuh"
 #include "rf_pair.cuh"
 #include "rf_plain.cuh"
+#include "rf_tile.cuh"
 
 namespace {
 
@@ -784,6 +785,73 @@ int launch_half_b(const ReconFields& f, const Weights& wt, LevelDims d, bool fir
     return check_launch();
 }
 
+namespace {
+template <int ROWS, int K>
+long long tile_blocks(LevelDims d) {
+    using T = ReconTile<ROWS, K>;
+    return (long long)((d.w + T::W - 1) / T::W) * ((d.h + T::H - 1) / T::H);
+}
+
+template <int ROWS, int K>
+int recon_tiles(const ReconFields& f, const ReconState& b, const LevelConsts* lc, const Weights& wt,
+                LevelDims d, int n_iters, bool uc_from_buffer, int prior, cudaStream_t st) {
+    using T = ReconTile<ROWS, K>;
+    const ReconState a{f.duhat, f.dvhat, f.pu1, f.pu2, f.pv1, f.pv2, f.uproj,
+                       f.vproj, f.sku,   f.skv, f.X,   f.Y,   f.Z};
+    const dim3 g((d.w + T::W - 1) / T::W, (d.h + T::H - 1) / T::H);
+    // an even number, so that the last one writes f's planes
+    const int launches = 2 * ((n_iters + 2 * K - 1) / (2 * K));
+    const int each = n_iters / launches, more = n_iters % launches;
+    auto kernel = prior == 1   ? k_recon_tile<1, ROWS, K>
+                  : prior == 2 ? k_recon_tile<2, ROWS, K>
+                               : k_recon_tile<0, ROWS, K>;
+    for (int i = 0; i < launches; i++) {
+        kernel<<<g, T::THREADS, 0, st>>>(f, i & 1 ? b : a, i & 1 ? a : b, lc, wt, d,
+                                         each + (i < more ? 1 : 0), i == 0, i + 1 == launches,
+                                         i == 0 && uc_from_buffer);
+        if (check_launch() != 0) return -1;
+    }
+    return launches;
+}
+
+// Which tile a level takes, 0 for none: the first of those below with no more
+// than a block per SM.
+int recon_tile_kind(LevelDims d) {
+    // An iteration of a block is bound by the instructions of its warps, so the
+    // smallest tile is the fastest while every block has an SM to itself; two
+    // blocks on one take twice as long.  Solves of 96x72 .. 640x480, the level in
+    // question with one tile and the next larger: 80x60 with 24 x 2 (10 rows) and
+    // 24 x 8 (16): 2.44 and 2.56 ms (of a 160x120 solve); 112x83 with 24 x 4 and
+    // 20 x 8: 3.74 and 3.82 (451x333); 160x120 with 20 x 8, three iterations, and
+    // 24 x 12, two: 2.42 and 2.51; 225x166 with 24 x 12 and with two launches per
+    // iteration: 3.52 and 3.75.  320x240, 280 blocks of 24 x 12, is as fast by two
+    // launches per iteration (4.95 against 5.01, 640x480).
+    constexpr int kSms = 152;
+    if (tile_blocks<10, 2>(d) <= kSms) return 1;
+    if (tile_blocks<12, 2>(d) <= kSms) return 2;
+    if (tile_blocks<20, 3>(d) <= kSms) return 3;
+    if (tile_blocks<20, 2>(d) <= kSms) return 4;
+    return 0;
+}
+}  // namespace
+
+bool use_recon_tiles(const Weights& wt, LevelDims d, int n_iters) {
+    // (a row that ends where the next begins has that one's first pixels to its
+    // right: a tile's region must not reach a second row)
+    return n_iters >= 2 && pair_weights(wt) && (d.s > d.w || d.w >= kTileW) && recon_tile_kind(d);
+}
+
+int launch_recon_tiles(const ReconFields& f, const ReconState& b, const LevelConsts* lc,
+                       const Weights& wt, LevelDims d, int n_iters, bool uc_from_buffer, int prior,
+                       cudaStream_t st) {
+    switch (recon_tile_kind(d)) {
+        case 1: return recon_tiles<10, 2>(f, b, lc, wt, d, n_iters, uc_from_buffer, prior, st);
+        case 2: return recon_tiles<12, 2>(f, b, lc, wt, d, n_iters, uc_from_buffer, prior, st);
+        case 3: return recon_tiles<20, 3>(f, b, lc, wt, d, n_iters, uc_from_buffer, prior, st);
+        default: return recon_tiles<20, 2>(f, b, lc, wt, d, n_iters, uc_from_buffer, prior, st);
+    }
+}
+
 #ifdef RF_BOUNDS_CHECK
 __global__ void k_oob_selftest(ReconFields f) { RF_AT(f, duhat, f.extent) += 0.0f; }
 #endif
@@ -865,7 +933,7 @@ bool cluster_supported() {
 }
 
 namespace {
-template <int R, int WARPS, int K>
+template <int R, int WARPS, int K, bool SKIP>
 int plain_tiles(PlainState a, PlainState b, const float* Ix, const float* Iy, const float* Iz,
                 const Weights& wt, LevelDims d, int n_iters, cudaStream_t st, int* in_b) {
     using T = PlainTile<R, WARPS, K>;
@@ -873,7 +941,7 @@ int plain_tiles(PlainState a, PlainState b, const float* Ix, const float* Iy, co
     int launches = 0;
     for (int done = 0; done < n_iters; done += K, launches++) {
         const int n = n_iters - done < K ? n_iters - done : K;
-        k_plain_tile<R, WARPS, K><<<g, T::THREADS, 0, st>>>(
+        k_plain_tile<R, WARPS, K, SKIP><<<g, T::THREADS, 0, st>>>(
             launches & 1 ? a : b, launches & 1 ? b : a, Ix, Iy, Iz, wt, d, n, done == 0,
             done + n == n_iters);
         if (check_launch() != 0) return -1;
@@ -890,12 +958,13 @@ int launch_plain_warp(PlainState a, PlainState b, const float* Ix, const float* 
     // region of 32 x 32; K = 3 and 5, 8 and 10 warps, 3 or 4 rows are 2-10% slower
     // at 640x480 and 720p).  On small ones a block's own time per launch counts:
     // fewer pixels per block, more iterations per launch (solve of 64x48, all
-    // five levels small: 0.90 ms against 1.22; K = 4, 5 and 8: 0.94, 1.00, 0.91).
+    // five levels small: 0.90 ms against 1.22; K = 4, 5 and 8: 0.94, 1.00, 0.91;
+    // 0.81 with used-up rows sitting out).
     // Between them, 320x240 within a 640x480 solve: 1.49 ms as a large level, 1.67
     // as a small one; 200x150: 0.98 as a small one, 1.27 as a large one.
     if ((long long)d.w * d.h >= 60000)
-        return plain_tiles<2, 16, 4>(a, b, Ix, Iy, Iz, wt, d, n_iters, st, in_b);
-    return plain_tiles<1, 20, 6>(a, b, Ix, Iy, Iz, wt, d, n_iters, st, in_b);
+        return plain_tiles<2, 16, 4, false>(a, b, Ix, Iy, Iz, wt, d, n_iters, st, in_b);
+    return plain_tiles<1, 20, 6, true>(a, b, Ix, Iy, Iz, wt, d, n_iters, st, in_b);
 }
 
 int launch_plain_data(float* duhat, float* dvhat, const float* pu1, const float* pu2,

@@ -163,6 +163,14 @@ int launch_half_a(const ReconFields& f, const LevelConsts* lc, const Weights& wt
                   bool first, bool uc_from_buffer, int prior, cudaStream_t st, dim3 block);
 int launch_half_b(const ReconFields& f, const Weights& wt, LevelDims d, bool first, bool last,
                   cudaStream_t st, dim3 block);
+// All inner iterations of a ReconFlow warp, several per launch (rf_tile.cuh),
+// between f's state and `b`, f's at the end.  Whether a level takes them
+// (`n_iters` of them), and the launches; returns their number, < 0 if one failed.
+struct ReconState;
+bool use_recon_tiles(const Weights& wt, LevelDims d, int n_iters);
+int launch_recon_tiles(const ReconFields& f, const ReconState& b, const LevelConsts* lc,
+                       const Weights& wt, LevelDims d, int n_iters, bool uc_from_buffer, int prior,
+                       cudaStream_t st);
 // All inner iterations of a plain TV-L1 warp, several per launch (rf_plain.cuh;
 // wt.fac >= 0, n_iters > 0), between the state planes `a` and `b` of which
 // nothing is read before it is written; *in_b: whether the final duhat is b's.  Returns the number of launches, < 0 if one failed.

@@ -30,6 +30,152 @@ __device__ __forceinline__ float deriv5(float m2, float m1, float p1, float p2) 
     return t;
 }
 
+// What part A reads at a pixel; its results replace the values it updates.
+struct APoint {
+    float u, v, dix, diy, dit, uproj, vproj, sku, skv, duhat, dvhat;
+    float pu1, pu2, pv1, pv2, pu1l, pv1l, pu2d, pv2d;  // p, left and above
+    // X0, Y0, Z0 at: 0 = pos, 1 = x+1 (flat pos+1), 2 = y+1 (flat pos+s),
+    // 3 = x-1, 4 = y-1.  x+1 / y+1 are read at flat pos+1 / pos+s even on the
+    // last column / row (solve3dMinimalArea.cu:65,76).
+    float Xn[5], Yn[5], Zn[5];
+    float uc, vc;  // read only when uc_from_buffer
+    float ufn, vfn, mk;
+    float Xo, Yo, Zo;  // the triangulated point
+};
+
+// Every load of the pixel is issued before any arithmetic or store, so a
+// thread waits for memory once.  Part A writes only duhat, uproj, sk and X1 at
+// its own pixel, and reads none of those at another pixel, so the order of
+// loads and stores does not change any value.
+template <int PRIOR>
+__device__ __forceinline__ void load_a(const ReconFields& f, LevelDims d, int pos, int ix, int iy,
+                                       int first, int uc_from_buffer, APoint& a) {
+    const int s = d.s;
+    const bool left = ix > 0, up = iy > 0;
+    a.u = RF_AT(f, u, pos);
+    a.v = RF_AT(f, v, pos);
+    a.dix = RF_AT(f, Ix, pos);
+    a.diy = RF_AT(f, Iy, pos);
+    a.dit = RF_AT(f, Iz, pos);
+    a.uproj = RF_AT(f, uproj, pos);
+    a.vproj = RF_AT(f, vproj, pos);
+    a.sku = RF_AT(f, sku, pos);
+    a.skv = RF_AT(f, skv, pos);
+    a.duhat = a.dvhat = a.pu1 = a.pu2 = a.pv1 = a.pv2 = 0.0f;
+    a.pu1l = a.pv1l = a.pu2d = a.pv2d = 0.0f;
+    if (!first) {
+        a.duhat = RF_AT(f, duhat, pos);
+        a.dvhat = RF_AT(f, dvhat, pos);
+        a.pu1 = RF_AT(f, pu1, pos);
+        a.pu2 = RF_AT(f, pu2, pos);
+        a.pv1 = RF_AT(f, pv1, pos);
+        a.pv2 = RF_AT(f, pv2, pos);
+        if (left) {
+            a.pu1l = RF_AT(f, pu1, pos - 1);
+            a.pv1l = RF_AT(f, pv1, pos - 1);
+        }
+        if (up) {
+            a.pu2d = RF_AT(f, pu2, pos - s);
+            a.pv2d = RF_AT(f, pv2, pos - s);
+        }
+    }
+    a.Xn[0] = RF_AT(f, X, pos);
+    a.Yn[0] = RF_AT(f, Y, pos);
+    a.Zn[0] = RF_AT(f, Z, pos);
+    a.Xn[1] = RF_AT(f, X, pos + 1);
+    a.Yn[1] = RF_AT(f, Y, pos + 1);
+    a.Zn[1] = RF_AT(f, Z, pos + 1);
+    a.Xn[2] = RF_AT(f, X, pos + s);
+    a.Yn[2] = RF_AT(f, Y, pos + s);
+    a.Zn[2] = RF_AT(f, Z, pos + s);
+    a.Xn[3] = a.Yn[3] = a.Zn[3] = 0.0f;
+    a.Xn[4] = a.Yn[4] = a.Zn[4] = 0.0f;
+    if (left) {
+        a.Xn[3] = RF_AT(f, X, pos - 1);
+        a.Yn[3] = RF_AT(f, Y, pos - 1);
+        a.Zn[3] = RF_AT(f, Z, pos - 1);
+    }
+    if (up) {
+        a.Xn[4] = RF_AT(f, X, pos - s);
+        a.Yn[4] = RF_AT(f, Y, pos - s);
+        a.Zn[4] = RF_AT(f, Z, pos - s);
+    }
+    a.uc = a.vc = 0.0f;
+    if (uc_from_buffer) {
+        a.uc = RF_AT(f, uc, pos);
+        a.vc = RF_AT(f, vc, pos);
+    }
+    a.ufn = a.vfn = 0.0f;
+    a.mk = 1.0f;
+    if (PRIOR != 0) {
+        a.ufn = RF_AT(f, ufn, pos);
+        a.vfn = RF_AT(f, vfn, pos);
+        if (PRIOR == 2) a.mk = RF_AT(f, mask, pos);
+    }
+}
+template <bool SK>
+__device__ __forceinline__ void store_a(const ReconFields& f, int pos, int first, const APoint& a) {
+    if (SK && !first) {
+        RF_AT(f, sku, pos) = a.sku;
+        RF_AT(f, skv, pos) = a.skv;
+    }
+    RF_AT(f, duhat, pos) = a.duhat;
+    RF_AT(f, dvhat, pos) = a.dvhat;
+    RF_AT(f, uproj, pos) = a.uproj;
+    RF_AT(f, vproj, pos) = a.vproj;
+    RF_AT(f, X1, pos) = a.Xo;
+    RF_AT(f, Y1, pos) = a.Yo;
+    RF_AT(f, Z1, pos) = a.Zo;
+}
+
+// Part A's arithmetic at (ix, iy).  SK as recon_a_px.
+template <int PRIOR, bool SK>
+__device__ __forceinline__ void recon_a_point(APoint& a, const LevelConsts& c, const Weights& wt,
+                                              int ix, int iy, int first, int uc_from_buffer) {
+    if (SK && !first) {
+        a.sku = a.sku + a.u + a.duhat - a.uproj;
+        a.skv = a.skv + a.v + a.dvhat - a.vproj;
+    }
+
+    // --- data step (solveReconDataL1.cu:24-100) ---
+    float A, dusub, dvsub;
+    if (PRIOR == 0) {
+        A = wt.A;
+        dusub = (wt.alpha_tv * a.duhat + wt.alpha_proj * (a.uproj - a.u - a.sku)) / A;
+        dvsub = (wt.alpha_tv * a.dvhat + wt.alpha_proj * (a.vproj - a.v - a.skv)) / A;
+    } else {
+        float alphaFn = PRIOR == 2 ? wt.alpha_fn * a.mk : wt.alpha_fn;
+        A = wt.alpha_tv + wt.alpha_proj + alphaFn;
+        dusub = (alphaFn * (a.ufn - a.u) + wt.alpha_tv * a.duhat + wt.alpha_proj * (a.uproj - a.u - a.sku)) / A;
+        dvsub = (alphaFn * (a.vfn - a.v) + wt.alpha_tv * a.dvhat + wt.alpha_proj * (a.vproj - a.v - a.skv)) / A;
+    }
+    float du, dv;
+    l1_threshold(dusub, dvsub, a.dix, a.diy, a.dit, wt.lambda, A, du, dv);
+    float divpu = divergence(a.pu1, a.pu1l, a.pu2, a.pu2d, ix, iy);
+    float divpv = divergence(a.pv1, a.pv1l, a.pv2, a.pv2d, ix, iy);
+    float duhat1 = du + divpu / A;
+    float dvhat1 = dv + divpv / A;
+
+    // --- projection blend (solveUVProj.cu:13-21), uc from the current 3D ---
+    float uc, vc;
+    if (uc_from_buffer) {
+        uc = a.uc;
+        vc = a.vc;
+    } else {
+        project_uc(c, a.Xn[0], a.Yn[0], a.Zn[0], ix, iy, uc, vc);
+    }
+    float uproj1 = (wt.lambdaf * uc + wt.alpha_proj * (a.u + duhat1 + a.sku)) / wt.proj_den;
+    float vproj1 = (wt.lambdaf * vc + wt.alpha_proj * (a.v + dvhat1 + a.skv)) / wt.proj_den;
+
+    // --- triangulation with minimal-area smoothing (solve3dMinimalArea.cu:23-184) ---
+    solve3d_pixel(c, uproj1, vproj1, ix, iy, a.Xn, a.Yn, a.Zn, wt.lambdaf, wt.lambdams, a.Xo, a.Yo, a.Zo);
+
+    a.duhat = duhat1;
+    a.dvhat = dvhat1;
+    a.uproj = uproj1;
+    a.vproj = vproj1;
+}
+
 // `base`: element of the level's pixel (0, 0) in every field (0 for a
 // single pair; a pair's offset in the batched solver's planes).  SK: the
 // multiplier update of the previous iteration's dual step (solveUcSk.cu:94-95)
@@ -38,123 +184,11 @@ template <int PRIOR, bool SK = false>
 __device__ __forceinline__ void recon_a_px(const ReconFields& f, const LevelConsts& c,
                                            const Weights& wt, LevelDims d, int ix, int iy,
                                            int first, int uc_from_buffer, int base = 0) {
-    const int s = d.s;
-    const int pos = base + ix + iy * s;
-
-    // Every load of the pixel is issued before any arithmetic or store, so a
-    // thread waits for memory once.  The kernel writes only duhat, uproj and
-    // X1 at its own pixel, and reads none of those at another pixel, so the
-    // order of loads and stores does not change any value.
-    float u = RF_AT(f, u, pos), v = RF_AT(f, v, pos);
-    float dix = RF_AT(f, Ix, pos), diy = RF_AT(f, Iy, pos), dit = RF_AT(f, Iz, pos);
-    float uproj = RF_AT(f, uproj, pos), vproj = RF_AT(f, vproj, pos);
-    float sku = RF_AT(f, sku, pos), skv = RF_AT(f, skv, pos);
-    float duhat = 0.0f, dvhat = 0.0f;
-    float pu1 = 0.0f, pu2 = 0.0f, pv1 = 0.0f, pv2 = 0.0f;
-    float pu1l = 0.0f, pv1l = 0.0f, pu2d = 0.0f, pv2d = 0.0f;
-    if (!first) {
-        duhat = RF_AT(f, duhat, pos);
-        dvhat = RF_AT(f, dvhat, pos);
-        pu1 = RF_AT(f, pu1, pos);
-        pu2 = RF_AT(f, pu2, pos);
-        pv1 = RF_AT(f, pv1, pos);
-        pv2 = RF_AT(f, pv2, pos);
-        if (ix > 0) {
-            pu1l = RF_AT(f, pu1, pos - 1);
-            pv1l = RF_AT(f, pv1, pos - 1);
-        }
-        if (iy > 0) {
-            pu2d = RF_AT(f, pu2, pos - s);
-            pv2d = RF_AT(f, pv2, pos - s);
-        }
-    }
-    // X0, Y0, Z0 at: 0 = pos, 1 = x+1 (flat pos+1), 2 = y+1 (flat pos+s),
-    // 3 = x-1, 4 = y-1.  x+1 / y+1 are read at flat pos+1 / pos+s even on the
-    // last column / row (solve3dMinimalArea.cu:65,76).
-    float Xn[5], Yn[5], Zn[5];
-    Xn[0] = RF_AT(f, X, pos);
-    Yn[0] = RF_AT(f, Y, pos);
-    Zn[0] = RF_AT(f, Z, pos);
-    Xn[1] = RF_AT(f, X, pos + 1);
-    Yn[1] = RF_AT(f, Y, pos + 1);
-    Zn[1] = RF_AT(f, Z, pos + 1);
-    Xn[2] = RF_AT(f, X, pos + s);
-    Yn[2] = RF_AT(f, Y, pos + s);
-    Zn[2] = RF_AT(f, Z, pos + s);
-    Xn[3] = Yn[3] = Zn[3] = 0.0f;
-    Xn[4] = Yn[4] = Zn[4] = 0.0f;
-    if (ix > 0) {
-        Xn[3] = RF_AT(f, X, pos - 1);
-        Yn[3] = RF_AT(f, Y, pos - 1);
-        Zn[3] = RF_AT(f, Z, pos - 1);
-    }
-    if (iy > 0) {
-        Xn[4] = RF_AT(f, X, pos - s);
-        Yn[4] = RF_AT(f, Y, pos - s);
-        Zn[4] = RF_AT(f, Z, pos - s);
-    }
-    float ucb = 0.0f, vcb = 0.0f;
-    if (uc_from_buffer) {
-        ucb = RF_AT(f, uc, pos);
-        vcb = RF_AT(f, vc, pos);
-    }
-    float ufn = 0.0f, vfn = 0.0f, mk = 1.0f;
-    if (PRIOR != 0) {
-        ufn = RF_AT(f, ufn, pos);
-        vfn = RF_AT(f, vfn, pos);
-        if (PRIOR == 2) mk = RF_AT(f, mask, pos);
-    }
-
-    if (SK && !first) {
-        sku = sku + u + duhat - uproj;
-        skv = skv + v + dvhat - vproj;
-    }
-
-    // --- data step (solveReconDataL1.cu:24-100) ---
-    float A, dusub, dvsub;
-    if (PRIOR == 0) {
-        A = wt.A;
-        dusub = (wt.alpha_tv * duhat + wt.alpha_proj * (uproj - u - sku)) / A;
-        dvsub = (wt.alpha_tv * dvhat + wt.alpha_proj * (vproj - v - skv)) / A;
-    } else {
-        float alphaFn = PRIOR == 2 ? wt.alpha_fn * mk : wt.alpha_fn;
-        A = wt.alpha_tv + wt.alpha_proj + alphaFn;
-        dusub = (alphaFn * (ufn - u) + wt.alpha_tv * duhat + wt.alpha_proj * (uproj - u - sku)) / A;
-        dvsub = (alphaFn * (vfn - v) + wt.alpha_tv * dvhat + wt.alpha_proj * (vproj - v - skv)) / A;
-    }
-    float du, dv;
-    l1_threshold(dusub, dvsub, dix, diy, dit, wt.lambda, A, du, dv);
-    float divpu = divergence(pu1, pu1l, pu2, pu2d, ix, iy);
-    float divpv = divergence(pv1, pv1l, pv2, pv2d, ix, iy);
-    float duhat1 = du + divpu / A;
-    float dvhat1 = dv + divpv / A;
-
-    // --- projection blend (solveUVProj.cu:13-21), uc from the current 3D ---
-    float uc, vc;
-    if (uc_from_buffer) {
-        uc = ucb;
-        vc = vcb;
-    } else {
-        project_uc(c, Xn[0], Yn[0], Zn[0], ix, iy, uc, vc);
-    }
-    float uproj1 = (wt.lambdaf * uc + wt.alpha_proj * (u + duhat1 + sku)) / wt.proj_den;
-    float vproj1 = (wt.lambdaf * vc + wt.alpha_proj * (v + dvhat1 + skv)) / wt.proj_den;
-
-    // --- triangulation with minimal-area smoothing (solve3dMinimalArea.cu:23-184) ---
-    float Xo, Yo, Zo;
-    solve3d_pixel(c, uproj1, vproj1, ix, iy, Xn, Yn, Zn, wt.lambdaf, wt.lambdams, Xo, Yo, Zo);
-
-    if (SK && !first) {
-        RF_AT(f, sku, pos) = sku;
-        RF_AT(f, skv, pos) = skv;
-    }
-    RF_AT(f, duhat, pos) = duhat1;
-    RF_AT(f, dvhat, pos) = dvhat1;
-    RF_AT(f, uproj, pos) = uproj1;
-    RF_AT(f, vproj, pos) = vproj1;
-    RF_AT(f, X1, pos) = Xo;
-    RF_AT(f, Y1, pos) = Yo;
-    RF_AT(f, Z1, pos) = Zo;
+    const int pos = base + ix + iy * d.s;
+    APoint a;
+    load_a<PRIOR>(f, d, pos, ix, iy, first, uc_from_buffer, a);
+    recon_a_point<PRIOR, SK>(a, c, wt, ix, iy, first, uc_from_buffer);
+    store_a<SK>(f, pos, first, a);
 }
 
 // 3x3 tap of the reference's 3D median with its border rules

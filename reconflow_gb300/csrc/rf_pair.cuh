@@ -807,115 +807,66 @@ __device__ __forceinline__ void recon_b_tile(const ReconFields& f, const Weights
 }
 
 // ---- one pixel per thread ---------------------------------------------------
+// Part A's arithmetic at (x, y), the multiplier update first (recon_a_point
+// with the quotients above); false where they are not sure: `a` is then spoilt.
+template <int PRIOR>
+__device__ __forceinline__ bool recon_a_fast(APoint& a, const LevelConsts& lc, const Weights& wt,
+                                             int x, int y, bool first, bool uc_from_buffer) {
+    const bool left = x > 0, up = y > 0;
+    const OneConsts c{lc, wt};
+    float divu = 0.0f, divv = 0.0f;
+    if (!first) {
+        a.sku = a.sku + a.u + a.duhat - a.uproj;
+        a.skv = a.skv + a.v + a.dvhat - a.vproj;
+        divu = divergence_v(a.pu1, a.pu1l, a.pu2, a.pu2d, left, up);
+        divv = divergence_v(a.pv1, a.pv1l, a.pv2, a.pv2d, left, up);
+    }
+    QuotientGuard g;
+    float A, nrA, nu, nv;
+    const float ru = a.uproj - a.u - a.sku, rv = a.vproj - a.v - a.skv;
+    if (PRIOR == 0) {
+        A = wt.A;
+        nrA = wt.nrA;
+        nu = neg_quot(wt.alpha_tv * a.duhat + wt.alpha_proj * ru, A, nrA);
+        nv = neg_quot(wt.alpha_tv * a.dvhat + wt.alpha_proj * rv, A, nrA);
+    } else {
+        const float afn = PRIOR == 2 ? wt.alpha_fn * a.mk : wt.alpha_fn;
+        A = wt.alpha_tv + wt.alpha_proj + afn;
+        nrA = neg_recip(A);
+        g.div(A);
+        nu = neg_quot(afn * (a.ufn - a.u) + wt.alpha_tv * a.duhat + wt.alpha_proj * ru, A, nrA);
+        nv = neg_quot(afn * (a.vfn - a.v) + wt.alpha_tv * a.dvhat + wt.alpha_proj * rv, A, nrA);
+    }
+    g.quot(nu);
+    g.quot(nv);
+    float du, dv;
+    l1_threshold_v(-nu, -nv, a.dix, a.diy, a.dit, wt.lambda, A, nrA, du, dv, g);
+    const float ndu = neg_quot(divu, A, nrA), ndv = neg_quot(divv, A, nrA);
+    g.quot(ndu);
+    g.quot(ndv);
+    a.duhat = du - ndu;
+    a.dvhat = dv - ndv;
+    const float fx = (float)x, fy = (float)y;
+    if (!uc_from_buffer) project_uc_v(c, a.Xn[0], a.Yn[0], a.Zn[0], fx, fy, a.uc, a.vc, g);
+    a.uproj = -neg_quot(wt.lambdaf * a.uc + wt.alpha_proj * (a.u + a.duhat + a.sku), wt.proj_den, wt.nrP);
+    a.vproj = -neg_quot(wt.lambdaf * a.vc + wt.alpha_proj * (a.v + a.dvhat + a.skv), wt.proj_den, wt.nrP);
+    g.quot_nonzero(a.uproj);
+    g.quot_nonzero(a.vproj);
+    solve3d_v(c, a.uproj, a.vproj, fx, fy, left, up, a.Xn, a.Yn, a.Zn, a.Xo, a.Yo, a.Zo, g);
+    return g.ok() && finite3(a.Xo, a.Yo, a.Zo);
+}
+
 // A at a pixel (recon_a_px with the multiplier update first and the quotients
 // above).
 template <int PRIOR>
 __device__ __forceinline__ void recon_a_one(const ReconFields& f, const LevelConsts& lc,
                                             const Weights& wt, LevelDims d, int base, int x, int y,
                                             bool first, bool uc_from_buffer) {
-    const int s = d.s, pos = base + x + y * s;
-    const bool left = x > 0, up = y > 0;
-    // every load before any arithmetic, as in recon_a_px
-    const float u = RF_AT(f, u, pos), v = RF_AT(f, v, pos);
-    const float dix = RF_AT(f, Ix, pos), diy = RF_AT(f, Iy, pos), dit = RF_AT(f, Iz, pos);
-    float uproj = RF_AT(f, uproj, pos), vproj = RF_AT(f, vproj, pos);
-    float sku = RF_AT(f, sku, pos), skv = RF_AT(f, skv, pos);
-    float duhat = 0.0f, dvhat = 0.0f, pu1 = 0.0f, pu2 = 0.0f, pv1 = 0.0f, pv2 = 0.0f;
-    float pu1l = 0.0f, pv1l = 0.0f, pu2d = 0.0f, pv2d = 0.0f;
-    if (!first) {
-        duhat = RF_AT(f, duhat, pos);
-        dvhat = RF_AT(f, dvhat, pos);
-        pu1 = RF_AT(f, pu1, pos);
-        pu2 = RF_AT(f, pu2, pos);
-        pv1 = RF_AT(f, pv1, pos);
-        pv2 = RF_AT(f, pv2, pos);
-        if (left) {
-            pu1l = RF_AT(f, pu1, pos - 1);
-            pv1l = RF_AT(f, pv1, pos - 1);
-        }
-        if (up) {
-            pu2d = RF_AT(f, pu2, pos - s);
-            pv2d = RF_AT(f, pv2, pos - s);
-        }
-    }
-    float Xn[5], Yn[5], Zn[5];
-    auto around = [&](const float* a, float (&n)[5]) {
-        n[0] = RF_PT(a, pos, f.extent);
-        n[1] = RF_PT(a, pos + 1, f.extent);
-        n[2] = RF_PT(a, pos + s, f.extent);
-        n[3] = left ? RF_PT(a, pos - 1, f.extent) : 0.0f;
-        n[4] = up ? RF_PT(a, pos - s, f.extent) : 0.0f;
-    };
-    around(f.X, Xn);
-    around(f.Y, Yn);
-    around(f.Z, Zn);
-    float uc = 0.0f, vc = 0.0f, ufn = 0.0f, vfn = 0.0f, mk = 1.0f;
-    if (uc_from_buffer) {
-        uc = RF_AT(f, uc, pos);
-        vc = RF_AT(f, vc, pos);
-    }
-    if (PRIOR != 0) {
-        ufn = RF_AT(f, ufn, pos);
-        vfn = RF_AT(f, vfn, pos);
-        if (PRIOR == 2) mk = RF_AT(f, mask, pos);
-    }
-
-    const OneConsts c{lc, wt};
-    float divu = 0.0f, divv = 0.0f;
-    if (!first) {
-        sku = sku + u + duhat - uproj;
-        skv = skv + v + dvhat - vproj;
-        divu = divergence_v(pu1, pu1l, pu2, pu2d, left, up);
-        divv = divergence_v(pv1, pv1l, pv2, pv2d, left, up);
-    }
-    QuotientGuard g;
-    float A, nrA, nu, nv;
-    const float ru = uproj - u - sku, rv = vproj - v - skv;
-    if (PRIOR == 0) {
-        A = wt.A;
-        nrA = wt.nrA;
-        nu = neg_quot(wt.alpha_tv * duhat + wt.alpha_proj * ru, A, nrA);
-        nv = neg_quot(wt.alpha_tv * dvhat + wt.alpha_proj * rv, A, nrA);
-    } else {
-        const float afn = PRIOR == 2 ? wt.alpha_fn * mk : wt.alpha_fn;
-        A = wt.alpha_tv + wt.alpha_proj + afn;
-        nrA = neg_recip(A);
-        g.div(A);
-        nu = neg_quot(afn * (ufn - u) + wt.alpha_tv * duhat + wt.alpha_proj * ru, A, nrA);
-        nv = neg_quot(afn * (vfn - v) + wt.alpha_tv * dvhat + wt.alpha_proj * rv, A, nrA);
-    }
-    g.quot(nu);
-    g.quot(nv);
-    float du, dv;
-    l1_threshold_v(-nu, -nv, dix, diy, dit, wt.lambda, A, nrA, du, dv, g);
-    const float ndu = neg_quot(divu, A, nrA), ndv = neg_quot(divv, A, nrA);
-    g.quot(ndu);
-    g.quot(ndv);
-    duhat = du - ndu;
-    dvhat = dv - ndv;
-    const float fx = (float)x, fy = (float)y;
-    if (!uc_from_buffer) project_uc_v(c, Xn[0], Yn[0], Zn[0], fx, fy, uc, vc, g);
-    uproj = -neg_quot(wt.lambdaf * uc + wt.alpha_proj * (u + duhat + sku), wt.proj_den, wt.nrP);
-    vproj = -neg_quot(wt.lambdaf * vc + wt.alpha_proj * (v + dvhat + skv), wt.proj_den, wt.nrP);
-    g.quot_nonzero(uproj);
-    g.quot_nonzero(vproj);
-    float Xo, Yo, Zo;
-    solve3d_v(c, uproj, vproj, fx, fy, left, up, Xn, Yn, Zn, Xo, Yo, Zo, g);
-    if (!(g.ok() && finite3(Xo, Yo, Zo))) {
-        recon_a_slow<PRIOR>(f, &lc, wt, d, base, x, y, first, uc_from_buffer);
-        return;
-    }
-    if (!first) {
-        RF_AT(f, sku, pos) = sku;
-        RF_AT(f, skv, pos) = skv;
-    }
-    RF_AT(f, duhat, pos) = duhat;
-    RF_AT(f, dvhat, pos) = dvhat;
-    RF_AT(f, uproj, pos) = uproj;
-    RF_AT(f, vproj, pos) = vproj;
-    RF_AT(f, X1, pos) = Xo;
-    RF_AT(f, Y1, pos) = Yo;
-    RF_AT(f, Z1, pos) = Zo;
+    const int pos = base + x + y * d.s;
+    APoint a;
+    load_a<PRIOR>(f, d, pos, x, y, first, uc_from_buffer, a);
+    if (recon_a_fast<PRIOR>(a, lc, wt, x, y, first, uc_from_buffer)) store_a<true>(f, pos, first, a);
+    else recon_a_slow<PRIOR>(f, &lc, wt, d, base, x, y, first, uc_from_buffer);
 }
 
 // the 3x3 taps of a pixel, border rules as load_taps
@@ -942,6 +893,40 @@ __device__ __forceinline__ float median3_one(const float (&t)[3][3]) {
     }
     return nmed3(nmax3(lo[0], lo[1], lo[2]), nmed3(mid[0], mid[1], mid[2]),
                  nmin3(hi[0], hi[1], hi[2]));
+}
+
+// the point of B from the taps: medians and clean-up
+__device__ __forceinline__ void point_one(const float (&tx)[3][3], const float (&ty)[3][3],
+                                          const float (&tz)[3][3], float& X, float& Y, float& Z) {
+    float Xm = median3_one(tx), Ym = median3_one(ty), Zm = median3_one(tz);
+    auto sure = [](float m) { return fabsf(m) > 0.0f; };
+    if (!(sure(Xm) && sure(Ym) && sure(Zm))) {
+        if (!sure(Xm)) Xm = median9_slow(tx, 0);
+        if (!sure(Ym)) Ym = median9_slow(ty, 0);
+        if (!sure(Zm)) Zm = median9_slow(tz, 0);
+    }
+    cleanup_pixel(tx[1][1], ty[1][1], tz[1][1], Xm, Ym, Zm, X, Y, Z);
+}
+// the dual update of B from the differences of duhat; p = pu1, pu2, pv1, pv2
+__device__ __forceinline__ void dual_one(float ux, float uy, float vx, float vy, float fac,
+                                         float* p) {
+    QuotientGuard g;
+    float pu1 = p[0], pu2 = p[1], pv1 = p[2], pv2 = p[3];
+    dual_step_v(ux, uy, fac, pu1, pu2, g);
+    dual_step_v(vx, vy, fac, pv1, pv2, g);
+    if (g.ok() && isfinite(pu1 + pu2 + pv1 + pv2)) {
+        p[0] = pu1;
+        p[1] = pu2;
+        p[2] = pv1;
+        p[3] = pv2;
+    } else {
+        const float2 pu = dual_step_slow(ux, uy, fac, p[0], p[1]);
+        const float2 pv = dual_step_slow(vx, vy, fac, p[2], p[3]);
+        p[0] = pu.x;
+        p[1] = pu.y;
+        p[2] = pv.x;
+        p[3] = pv.y;
+    }
 }
 
 // B at a pixel (recon_b_px without the multiplier update); LAST as
@@ -982,35 +967,17 @@ __device__ __forceinline__ void recon_b_one(const ReconFields& f, const Weights&
             vy = RF_AT(f, dvhat, pos + s) - dvhat;
         }
     }
-    float Xm = median3_one(tx), Ym = median3_one(ty), Zm = median3_one(tz);
-    auto sure = [](float m) { return fabsf(m) > 0.0f; };
-    if (!(sure(Xm) && sure(Ym) && sure(Zm))) {
-        if (!sure(Xm)) Xm = median9_slow(tx, 0);
-        if (!sure(Ym)) Ym = median9_slow(ty, 0);
-        if (!sure(Zm)) Zm = median9_slow(tz, 0);
-    }
     float X, Y, Z;
-    cleanup_pixel(tx[1][1], ty[1][1], tz[1][1], Xm, Ym, Zm, X, Y, Z);
+    point_one(tx, ty, tz, X, Y, Z);
     if (LAST) {
         RF_AT(f, sku, pos) = a[4] + a[0] + duhat - a[2];
         RF_AT(f, skv, pos) = a[5] + a[1] + dvhat - a[3];
     } else {
-        QuotientGuard g;
-        float pu1 = a[0], pu2 = a[1], pv1 = a[2], pv2 = a[3];
-        dual_step_v(ux, uy, wt.fac, pu1, pu2, g);
-        dual_step_v(vx, vy, wt.fac, pv1, pv2, g);
-        if (!(g.ok() && isfinite(pu1 + pu2 + pv1 + pv2))) {
-            const float2 pu = dual_step_slow(ux, uy, wt.fac, a[0], a[1]);
-            const float2 pv = dual_step_slow(vx, vy, wt.fac, a[2], a[3]);
-            pu1 = pu.x;
-            pu2 = pu.y;
-            pv1 = pv.x;
-            pv2 = pv.y;
-        }
-        RF_AT(f, pu1, pos) = pu1;
-        RF_AT(f, pu2, pos) = pu2;
-        RF_AT(f, pv1, pos) = pv1;
-        RF_AT(f, pv2, pos) = pv2;
+        dual_one(ux, uy, vx, vy, wt.fac, a);
+        RF_AT(f, pu1, pos) = a[0];
+        RF_AT(f, pu2, pos) = a[1];
+        RF_AT(f, pv1, pos) = a[2];
+        RF_AT(f, pv2, pos) = a[3];
     }
     RF_AT(f, X, pos) = X;
     RF_AT(f, Y, pos) = Y;

@@ -108,12 +108,15 @@ __device__ __forceinline__ f2 shfl_down1(f2 a) {
 // (R WARPS - 2K) pixels
 template <int R, int WARPS, int K>
 struct PlainTile {
-    static constexpr int W = 32 - 2 * K, H = R * WARPS - 2 * K, THREADS = 32 * WARPS;
+    static constexpr int ROWS = R * WARPS, W = 32 - 2 * K, H = ROWS - 2 * K, THREADS = 32 * WARPS;
 };
 
 // `n` iterations; `first`: the state before them is zero; `last`: only duhat is
-// written (the next warp's dual field starts from zero).
-template <int R, int WARPS, int K>
+// written (the next warp's dual field starts from zero).  SKIP: warps whose rows
+// are used up or outside the level sit out (64x48 solve 0.90 -> 0.81 ms with 20
+// warps of a row; with two rows per warp the branches cost registers and more
+// time than they save: 1.49 -> 1.67 ms at 640x480).
+template <int R, int WARPS, int K, bool SKIP>
 __global__ void __launch_bounds__(32 * WARPS)
     k_plain_tile(PlainState in, PlainState out, const float* __restrict__ Ix,
                  const float* __restrict__ Iy, const float* __restrict__ Iz, PlainWeights wt,
@@ -124,6 +127,8 @@ __global__ void __launch_bounds__(32 * WARPS)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int x = (int)blockIdx.x * T::W - K + lane;
     const int y0 = (int)blockIdx.y * T::H - K + warp * R;
+    const int first_row = warp * R;
+    const bool any_y = y0 < d.h && y0 + R > 0;
     const bool in_x = x >= 0 && x < d.w;
     const int above = warp > 0 ? warp - 1 : 0, below = warp < WARPS - 1 ? warp + 1 : warp;
 
@@ -158,52 +163,59 @@ __global__ void __launch_bounds__(32 * WARPS)
     const float lt = wt.lambda * wt.theta;
 #pragma unroll 1
     for (int it = 0; it < n; it++) {
-        f2 up = s_n2[above][lane], t[R];
-        QuotientGuard g;
+        // warps with a row that is right after the half-step and in the level
+        const bool data = !SKIP || (first_row + R > it + 1 && first_row < T::ROWS - it && any_y);
+        const bool dual = !SKIP || (first_row + R > it + 1 && first_row < T::ROWS - 1 - it && any_y);
+        if (data) {
+            f2 up = s_n2[above][lane], t[R];
+            QuotientGuard g;
 #pragma unroll
-        for (int r = 0; r < R; r++) t[r] = plain_threshold(c[r], du[r], lt, g);
-        if (!g.ok()) {
+            for (int r = 0; r < R; r++) t[r] = plain_threshold(c[r], du[r], lt, g);
+            if (!g.ok()) {
+#pragma unroll
+                for (int r = 0; r < R; r++) {
+                    const float2 e = plain_threshold_slow(du[r], c[r].di, c[r].dit, wt.lambda, wt.theta);
+                    t[r] = f2{e.x, e.y};
+                }
+            }
 #pragma unroll
             for (int r = 0; r < R; r++) {
-                const float2 e = plain_threshold_slow(du[r], c[r].di, c[r].dit, wt.lambda, wt.theta);
-                t[r] = f2{e.x, e.y};
+                f2 left = shfl_up1(n1[r]);
+                // (no neighbour: minus zero, which changes nothing)
+                if (x == 0) left = dup2(-0.0f);
+                if (y0 + r == 0) up = dup2(-0.0f);
+                // divergence (solveDataL1.cu:54-85) of the negatives
+                const f2 div = left - n1[r] - n2[r] + up;
+                up = n2[r];
+                du[r] = t[r] + dup2(wt.theta) * div;
             }
+            s_du[warp][lane] = du[0];
         }
-#pragma unroll
-        for (int r = 0; r < R; r++) {
-            f2 left = shfl_up1(n1[r]);
-            // (no neighbour: minus zero, which changes nothing)
-            if (x == 0) left = dup2(-0.0f);
-            if (y0 + r == 0) up = dup2(-0.0f);
-            // divergence (solveDataL1.cu:54-85) of the negatives
-            const f2 div = left - n1[r] - n2[r] + up;
-            up = n2[r];
-            du[r] = t[r] + dup2(wt.theta) * div;
-        }
-        s_du[warp][lane] = du[0];
         __syncthreads();
-        const f2 down = s_du[below][lane];
-        f2 dx[R], dy[R], m1[R], m2[R];
-        QuotientGuard gd;
-#pragma unroll
-        for (int r = 0; r < R; r++) {
-            dx[r] = shfl_down1(du[r]) - du[r];
-            dy[r] = (r < R - 1 ? du[r < R - 1 ? r + 1 : r] : down) - du[r];
-            if (x + 1 >= d.w) dx[r] = dup2(0.0f);
-            if (y0 + r + 1 >= d.h) dy[r] = dup2(0.0f);
-            m1[r] = n1[r];
-            m2[r] = n2[r];
-            plain_dual(dx[r], dy[r], wt.fac, m1[r], m2[r], gd);
-        }
-        if (gd.ok()) {
+        if (dual) {
+            const f2 down = s_du[below][lane];
+            f2 dx[R], dy[R], m1[R], m2[R];
+            QuotientGuard gd;
 #pragma unroll
             for (int r = 0; r < R; r++) {
-                n1[r] = m1[r];
-                n2[r] = m2[r];
+                dx[r] = shfl_down1(du[r]) - du[r];
+                dy[r] = (r < R - 1 ? du[r < R - 1 ? r + 1 : r] : down) - du[r];
+                if (x + 1 >= d.w) dx[r] = dup2(0.0f);
+                if (y0 + r + 1 >= d.h) dy[r] = dup2(0.0f);
+                m1[r] = n1[r];
+                m2[r] = n2[r];
+                plain_dual(dx[r], dy[r], wt.fac, m1[r], m2[r], gd);
             }
-        } else {
+            if (gd.ok()) {
 #pragma unroll
-            for (int r = 0; r < R; r++) plain_dual_slow2(dx[r], dy[r], wt.fac, n1[r], n2[r]);
+                for (int r = 0; r < R; r++) {
+                    n1[r] = m1[r];
+                    n2[r] = m2[r];
+                }
+            } else {
+#pragma unroll
+                for (int r = 0; r < R; r++) plain_dual_slow2(dx[r], dy[r], wt.fac, n1[r], n2[r]);
+            }
         }
         s_n2[warp][lane] = n2[R - 1];
         __syncthreads();

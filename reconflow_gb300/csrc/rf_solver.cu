@@ -22,6 +22,7 @@
 #include "rf_nvtx.h"
 #include "rf_kernels.cuh"
 #include "rf_plain.cuh"
+#include "rf_tile.cuh"
 
 using namespace rf;
 
@@ -354,12 +355,24 @@ rf_status enqueue_recon(rf_handle* h, float** res_u, float** res_v, bool warm = 
             f.X = h->X; f.Y = h->Y; f.Z = h->Z; f.X1 = h->X1; f.Y1 = h->Y1; f.Z1 = h->Z1;
             f.uc = uc; f.vc = vc;
             f.ufn = h->ufn_l; f.vfn = h->vfn_l; f.mask = h->mask_l;
-            if (n_iters > 0 && use_cluster_at(h, d)) {
+            const bool cluster = n_iters > 0 && use_cluster_at(h, d);
+            const bool tiled = !cluster && use_recon_tiles(wt, d, n_iters);
+            if (tiled) {
+                // the second state in planes the upscales (eight of free_planes) leave
+                float* const* q = free_planes.data() + 8;
+                const ReconState b{q[0], q[1], q[2], q[3],  q[4],  q[5], q[6],
+                                   q[7], q[8], q[9], q[10], q[11], q[12]};
+                const int k = launch_recon_tiles(f, b, lc, wt, d, n_iters, uc_in_buffer, prior, st);
+                if (k < 0) return cuda_fail(rf::last_launch_error(), "kernel launch iterations");
+                h->enqueue_launches += k;
+                uc_in_buffer = false;
+            }
+            if (cluster) {
                 // a small level: all of the warp's iterations in one cluster launch
                 RF_LAUNCH(launch_recon_cluster(f, lc, wt, d, n_iters, uc_in_buffer, prior, st));
                 uc_in_buffer = false;
             }
-            for (int iter = 0; iter < n_iters && !use_cluster_at(h, d); iter++) {
+            for (int iter = 0; iter < n_iters && !cluster && !tiled; iter++) {
                 const dim3 tile(h->tile_w[level], h->tile_h[level]);
                 if (pair_weights(wt)) {
                     RF_LAUNCH(launch_half_a(f, lc, wt, d, iter == 0, uc_in_buffer, prior, st, tile));
