@@ -56,31 +56,26 @@ __device__ __forceinline__ uint4 pack8(const bf16 (&v)[8]) {
     return make_uint4(pack2(v[0], v[1]), pack2(v[2], v[3]), pack2(v[4], v[5]), pack2(v[6], v[7]));
 }
 
-// forward A: im2col row of output pixel m, k = (ky*3 + kx)*Cin + ci (Cin % 8 == 0)
+using rf_tc::TcPos;
+using rf_tc::TcRow;
+// (a buffer has at most 2^26 pixels of 128 channels, 2^30 units of 16 bytes)
+__device__ __forceinline__ const uint4* units(const bf16* p) {
+    return reinterpret_cast<const uint4*>(p);
+}
+
+// forward A: im2col row of output pixel m, k = (ky*3 + kx)*C + ci (C % 8 == 0)
 struct TcConvIn {
     const bf16* x;
-    int B, H, W, C, Ho, Wo, stride;
-    struct Row {
-        long long off;  // element of tap (0, 0), channel 0 (outside the image at its edges)
-        int y, x;       // that tap's pixel; y < -2: no row
-    };
-    struct Pos {
-        int off, ky, kx;
-    };
-    __device__ const void* base() const { return x; }
-    __device__ Row row(int m, int M) const {
+    int H, W, C, Ho, Wo, stride;
+    __device__ const uint4* base() const { return units(x); }
+    __device__ TcRow row(int m, int M) const {
         const int xo = m % Wo, r = m / Wo, yo = r % Ho, b = r / Ho;
         const int y = yo * stride - 1, xx = xo * stride - 1;
-        return Row{(((long long)b * H + y) * W + xx) * C, m < M ? y : -8, xx};
+        return TcRow{((b * H + y) * W + xx) * (C / 8), m < M ? rf_tc::conv_taps(y, xx, H, W) : 0u};
     }
-    __device__ Pos kpos(int k) const {
-        const int ci = k % C, t = k / C, kx = t % 3, ky = t / 3;
-        return Pos{(ky * W + kx) * C + ci, ky, kx};
-    }
-    __device__ const void* at(const Row& r, const Pos& k) const {
-        if ((unsigned)(r.y + k.ky) >= (unsigned)H || (unsigned)(r.x + k.kx) >= (unsigned)W)
-            return nullptr;
-        return x + r.off + k.off;
+    __device__ TcPos kpos(int k) const {
+        const int ci = k % C, t = k / C;
+        return TcPos{(t / 3 * W + t % 3) * (C / 8) + ci / 8, t};
     }
 };
 
@@ -88,43 +83,73 @@ struct TcConvIn {
 struct TcRows {
     const bf16* w;
     int K;
-    typedef const bf16* Row;
-    __device__ const void* base() const { return w; }
-    __device__ Row row(int n, int N) const { return n < N ? w + (size_t)n * K : nullptr; }
-    __device__ int kpos(int k) const { return k; }
-    __device__ const void* at(Row r, int k) const { return r ? r + k : nullptr; }
+    __device__ const uint4* base() const { return units(w); }
+    __device__ TcRow row(int n, int N) const { return TcRow{n * (K / 8), n < N ? 1u : 0u}; }
+    __device__ TcPos kpos(int k) const { return TcPos{k / 8, 0}; }
 };
 
-// input-gradient A: input pixel m, k = (ky*3 + kx)*Cout + co -> dy at the
-// output pixel that tap (ky, kx) of m feeds (Cout % 8 == 0)
+// input-gradient A (stride 1): input pixel m, k = (ky*3 + kx)*Cout + co -> dy at
+// the output pixel that tap (ky, kx) of m feeds (Cout % 8 == 0)
 struct TcDataGradA {
     const bf16* dy;
-    int H, W, Ho, Wo, Cout, stride;
-    struct Row {
-        int img, y, x;  // the image's first output row; input pixel + 1 (y < 0: no row)
-    };
-    struct Pos {
-        int co, ky, kx;
-    };
-    __device__ const void* base() const { return dy; }
-    __device__ Row row(int m, int M) const {
-        const int xx = m % W, r = m / W, y = r % H, b = r / H;
-        return Row{b * Ho, m < M ? y + 1 : -8, xx + 1};
+    int H, W, Cout;
+    __device__ const uint4* base() const { return units(dy); }
+    __device__ TcRow row(int m, int M) const {
+        const int x = m % W, r = m / W, y = r % H, b = r / H;
+        unsigned taps = 0, cols = 0;
+#pragma unroll
+        for (int i = 0; i < 3; i++) cols |= (unsigned)(x + 1 - i) < (unsigned)W ? 1u << i : 0u;
+#pragma unroll
+        for (int i = 0; i < 3; i++) taps |= (unsigned)(y + 1 - i) < (unsigned)H ? cols << 3 * i : 0u;
+        return TcRow{((b * H + y + 1) * W + x + 1) * (Cout / 8), m < M ? taps : 0u};
     }
-    __device__ Pos kpos(int k) const {
-        const int co = k % Cout, t = k / Cout, kx = t % 3, ky = t / 3;
-        return Pos{co, ky, kx};
+    __device__ TcPos kpos(int k) const {
+        const int co = k % Cout, t = k / Cout;
+        return TcPos{co / 8 - (t / 3 * W + t % 3) * (Cout / 8), t};
     }
-    __device__ const void* at(const Row& r, const Pos& k) const {
-        int ty = r.y - k.ky, tx = r.x - k.kx;
-        if (ty < 0 || tx < 0) return nullptr;
-        if (stride == 2) {
-            if ((ty | tx) & 1) return nullptr;
-            ty >>= 1;
-            tx >>= 1;
-        }
-        if (ty >= Ho || tx >= Wo) return nullptr;
-        return dy + ((size_t)(r.img + ty) * Wo + tx) * Cout + k.co;
+};
+
+// the same for a stride of 2 and the input pixels (2 yc + py, 2 xc + px): 1, 2 or
+// 4 of the nine taps reach them, k = (index among those)*Cout + co.  All pixels at
+// once spent three quarters of the K loop on zeros (0.49 ms for 64 images of
+// 160 x 120; 0.19 by parity, four launches).
+struct Parity2 {
+    int py, px;
+    __device__ int taps_x() const { return px + 1; }
+    __device__ int tap(int i) const {  // ky * 3 + kx
+        const int iy = i / taps_x(), ix = i % taps_x();
+        return (py ? 2 * iy : 1) * 3 + (px ? 2 * ix : 1);
+    }
+};
+struct TcDataGrad2A {
+    const bf16* dy;
+    int Hc, Wc, Ho, Wo, Cout;
+    Parity2 q;
+    __device__ const uint4* base() const { return units(dy); }
+    __device__ TcRow row(int m, int M) const {
+        // tap (iy, ix) of those reads output pixel (y - iy, x - ix)
+        const int xc = m % Wc, r = m / Wc, yc = r % Hc, b = r / Hc;
+        const int y = yc + q.py, x = xc + q.px;
+        unsigned taps = 0;
+        for (int iy = 0; iy <= q.py; iy++)
+            for (int ix = 0; ix <= q.px; ix++)
+                if ((unsigned)(y - iy) < (unsigned)Ho && (unsigned)(x - ix) < (unsigned)Wo)
+                    taps |= 1u << (iy * q.taps_x() + ix);
+        return TcRow{((b * Ho + y) * Wo + x) * (Cout / 8), m < M ? taps : 0u};
+    }
+    __device__ TcPos kpos(int k) const {
+        const int i = k / Cout, iy = i / q.taps_x(), ix = i % q.taps_x();
+        return TcPos{k % Cout / 8 - (iy * Wo + ix) * (Cout / 8), i};
+    }
+};
+struct TcTapRows {
+    const bf16* w;  // [n][tap][Cout]
+    int Cout;
+    Parity2 q;
+    __device__ const uint4* base() const { return units(w); }
+    __device__ TcRow row(int n, int N) const { return TcRow{n * 9 * (Cout / 8), n < N ? 1u : 0u}; }
+    __device__ TcPos kpos(int k) const {
+        return TcPos{(q.tap(k / Cout) * Cout + k % Cout) / 8, 0};
     }
 };
 
@@ -188,6 +213,16 @@ struct StoreF32 {
     }
 };
 
+struct StoreF32Parity {
+    float* out;
+    int N, H, W, Hc, Wc;
+    Parity2 q;
+    __device__ void operator()(int m, int n, const float (&v)[8]) const {
+        const int xc = m % Wc, r = m / Wc, yc = r % Hc, b = r / Hc;
+        store8(out + (((size_t)b * H + 2 * yc + q.py) * W + 2 * xc + q.px) * N + n, v);
+    }
+};
+
 __global__ void k_reduce_partials(const float* part, int chunks, int n, float* out) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -196,68 +231,95 @@ __global__ void k_reduce_partials(const float* part, int chunks, int n, float* o
     out[i] = s;
 }
 
-// bias gradient, stage 1: block b sums dy over its pixel range
-// [b * span, (b + 1) * span) for every channel; thread t takes channel t % C
-// and every R-th pixel from t / C (R = 256 / C), then the R partial sums of a
-// channel are added in a fixed order.  Stage 2 (k_reduce_partials) adds the
-// block partials in block order, so the result is deterministic.
-constexpr int kBiasThreads = 256;
-
-__global__ void __launch_bounds__(kBiasThreads) k_bias_partial(const float* dy, int P, int C,
-                                                               int span, float* part) {
-    __shared__ float red[kBiasThreads];
-    const int t = threadIdx.x, R = kBiasThreads / C;
-    const int c = t % C, r = t / C;
-    const int p0 = blockIdx.x * span, p1 = min(P, p0 + span);
-    float acc = 0.f;
-    if (r < R)
-        for (int p = p0 + r; p < p1; p += R) acc += dy[(size_t)p * C + c];
-    red[t] = acc;
-    __syncthreads();
-    if (t < C) {
-        float s = 0.f;
-        for (int k = 0; k < R; k++) s += red[t + k * C];
-        part[(size_t)blockIdx.x * C + t] = s;
-    }
-}
-
 // The elementwise passes take 4 (FP32) or 8 (BF16 copies) channels per thread:
 // every channel count is a multiple of 8, and one element per thread, with its
 // index divisions, ran at 0.3 - 0.4 of the HBM rate.
-__global__ void k_f32_to_bf16(const float* a, bf16* b, size_t n) {
-    size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) b[i] = __float2bfloat16(a[i]);
-}
-
 __device__ __forceinline__ uint2 bf16x4(float4 v) {
     return make_uint2(pack2(__float2bfloat16(v.x), __float2bfloat16(v.y)),
                       pack2(__float2bfloat16(v.z), __float2bfloat16(v.w)));
+}
+// n a multiple of 4; `a` may be the caller's, aligned as a float only
+__global__ void k_f32_to_bf16(const float* a, bf16* b, size_t n) {
+    const size_t i = 4 * ((size_t)blockIdx.x * blockDim.x + threadIdx.x);
+    if (i >= n) return;
+    const float4 v = (uintptr_t)a % 16 == 0 ? *(const float4*)(a + i)
+                                            : make_float4(a[i], a[i + 1], a[i + 2], a[i + 3]);
+    *(uint2*)(b + i) = bf16x4(v);
 }
 __device__ __forceinline__ bool bf16_positive(unsigned bits) {  // > 0 (not NaN)
     bits &= 0xFFFFu;
     return bits != 0 && bits <= 0x7F80u;
 }
 
-// dy = (g + add) * [activation > 0] (ReLU backward; `add` may be null), in
-// place on g, and a BF16 copy; n a multiple of 4
-__global__ void k_relu_grad(float* g, const float* add, const bf16* act, bf16* gb, size_t n) {
-    const size_t i = 4 * ((size_t)blockIdx.x * blockDim.x + threadIdx.x);
-    if (i >= n) return;
-    float4 v = *(const float4*)(g + i);
-    if (add) {
-        const float4 t = *(const float4*)(add + i);
-        v.x += t.x;
-        v.y += t.y;
-        v.z += t.z;
-        v.w += t.w;
+// A layer's output gradient dy = (g + add) * [act > 0] (`add` null: none; `act`
+// null: a linear layer) as BF16, and the partial sums of its bias gradient: block b
+// takes pixels [b kGradSpan, (b + 1) kGradSpan), thread t the four channels
+// 4 (t % (C / 4)) of every R-th pixel; the R sums of a channel are added in order,
+// k_reduce_bias adds the blocks' (deterministic).  One pass and no FP32 copy of dy:
+// as two passes (masked gradient in place and BF16 copy, then the sums) the
+// 64-channel layer of 64 images of 160 x 120 took 0.26 ms, now 0.09 (6.9 TB/s).
+constexpr int kGradThreads = 256, kGradSpan = 512;
+
+__global__ void __launch_bounds__(kGradThreads) k_grad_in(const float* g, const float* add,
+                                                          const bf16* act, bf16* gb, int P, int C,
+                                                          float* part) {
+    __shared__ float4 red[kGradThreads];
+    const int t = threadIdx.x, Q = C / 4, R = kGradThreads / Q;
+    const int q = t % Q, r = t / Q;
+    const int p0 = blockIdx.x * kGradSpan, p1 = min(P, p0 + kGradSpan);
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (r < R)
+#pragma unroll 4
+        for (int p = p0 + r; p < p1; p += R) {
+            const size_t i = (size_t)p * C + 4 * q;
+            float4 v = *(const float4*)(g + i);
+            if (add) {
+                const float4 a = *(const float4*)(add + i);
+                v.x += a.x;
+                v.y += a.y;
+                v.z += a.z;
+                v.w += a.w;
+            }
+            if (act) {
+                const uint2 a = *(const uint2*)(act + i);
+                if (!bf16_positive(a.x)) v.x = 0.f;
+                if (!bf16_positive(a.x >> 16)) v.y = 0.f;
+                if (!bf16_positive(a.y)) v.z = 0.f;
+                if (!bf16_positive(a.y >> 16)) v.w = 0.f;
+            }
+            *(uint2*)(gb + i) = bf16x4(v);
+            acc.x += v.x;
+            acc.y += v.y;
+            acc.z += v.z;
+            acc.w += v.w;
+        }
+    red[t] = acc;
+    __syncthreads();
+    if (t < Q) {
+        float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int k = 0; k < R; k++) {
+            const float4 v = red[t + k * Q];
+            s.x += v.x;
+            s.y += v.y;
+            s.z += v.z;
+            s.w += v.w;
+        }
+        *(float4*)(part + (size_t)blockIdx.x * C + 4 * t) = s;
     }
-    const uint2 a = *(const uint2*)(act + i);
-    if (!bf16_positive(a.x)) v.x = 0.f;
-    if (!bf16_positive(a.x >> 16)) v.y = 0.f;
-    if (!bf16_positive(a.y)) v.z = 0.f;
-    if (!bf16_positive(a.y >> 16)) v.w = 0.f;
-    *(float4*)(g + i) = v;
-    *(uint2*)(gb + i) = bf16x4(v);
+}
+
+// channel blockIdx.x of `n` blocks' partial sums
+__global__ void __launch_bounds__(kGradThreads) k_reduce_bias(const float* part, int n, int C,
+                                                              float* out) {
+    __shared__ float red[kGradThreads];
+    float s = 0.f;
+    for (int i = threadIdx.x; i < n; i += kGradThreads) s += part[(size_t)i * C + blockIdx.x];
+    red[threadIdx.x] = s;
+    for (int k = kGradThreads / 2; k > 0; k /= 2) {
+        __syncthreads();
+        if (threadIdx.x < k) red[threadIdx.x] += red[threadIdx.x + k];
+    }
+    if (threadIdx.x == 0) out[blockIdx.x] = red[0];
 }
 
 // cat = [nearest 2x upsample of a (Ha x Wa x Ca), b (H x W x Cb)], 8 channels
@@ -307,25 +369,29 @@ __global__ void k_concat_up_grad(const float* dcat, int Ha, int Wa, int Ca, int 
     }
 }
 
-// L1 loss on channels 0..2 with per-channel weights, masked; writes dL/dpred
+// L1 loss on channels 0..2 of 8 with per-channel weights, masked; writes dL/dpred
 // (already divided by the number of valid pixels) and accumulates the loss.
-__global__ void k_l1_loss(const float* pred, const float* tgt, const float* mask, int P, int C,
-                          float w0, float w1, float w2, float inv_count, float* grad,
+__global__ void k_l1_loss(const float4* pred, const float* tgt, const float* mask, int P,
+                          float w0, float w1, float w2, float inv_count, float4* grad,
                           double* loss) {
     int p = blockIdx.x * blockDim.x + threadIdx.x;
     double l = 0.0;
     if (p < P) {
-        float m = mask[p];
-        for (int c = 0; c < C; c++) {
-            float g = 0.f;
-            if (c < 3 && m > 0.f) {
-                float wc = c == 0 ? w0 : (c == 1 ? w1 : w2);
-                float d = pred[(size_t)p * C + c] - tgt[(size_t)p * C + c];
+        const float m = mask[p];
+        float4 g = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (m > 0.f) {
+            const float4 a = pred[2 * (size_t)p];
+            const float* t = tgt + 8 * (size_t)p;  // the caller's, aligned as a float only
+            auto term = [&](float wc, float d) {
                 l += (double)(wc * fabsf(d)) * inv_count;
-                g = (d > 0.f ? wc : (d < 0.f ? -wc : 0.f)) * inv_count;
-            }
-            grad[(size_t)p * C + c] = g;
+                return (d > 0.f ? wc : (d < 0.f ? -wc : 0.f)) * inv_count;
+            };
+            g.x = term(w0, a.x - t[0]);
+            g.y = term(w1, a.y - t[1]);
+            g.z = term(w2, a.z - t[2]);
         }
+        grad[2 * (size_t)p] = g;
+        grad[2 * (size_t)p + 1] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
     for (int o = 16; o > 0; o >>= 1) l += __shfl_down_sync(0xffffffffu, l, o);
     if ((threadIdx.x & 31) == 0) atomicAdd(loss, l);
@@ -442,18 +508,16 @@ struct ConvOutPadded {
 struct TcConvInPadded {
     const bf16* x;
     int H, W, C, Ho, Wo, stride;
-    typedef const bf16* Row;
-    __device__ const void* base() const { return x; }
-    __device__ Row row(int m, int M) const {
+    __device__ const uint4* base() const { return units(x); }
+    __device__ TcRow row(int m, int M) const {
         const int xo = m % Wo, r = m / Wo, yo = r % Ho, b = r / Ho;
-        return m < M ? x + (((size_t)b * (H + 2) + yo * stride) * (W + 2) + xo * stride) * C
-                     : nullptr;
+        return TcRow{((b * (H + 2) + yo * stride) * (W + 2) + xo * stride) * (C / 8),
+                     m < M ? 1u : 0u};
     }
-    __device__ int kpos(int k) const {
-        const int ci = k % C, t = k / C, kx = t % 3, ky = t / 3;
-        return (ky * (W + 2) + kx) * C + ci;
+    __device__ TcPos kpos(int k) const {
+        const int ci = k % C, t = k / C;
+        return TcPos{(t / 3 * (W + 2) + t % 3) * (C / 8) + ci / 8, 0};
     }
-    __device__ const void* at(Row r, int k) const { return r ? r + k : nullptr; }
 };
 
 struct ConvOutToPadded {
@@ -589,16 +653,29 @@ rf_status conv_fwd(rf_cnn* c, const Layer& L, const bf16* x, int B, int H, int W
                    float* yf) {
     int Ho = Ho_of(H, L.stride), Wo = Ho_of(W, L.stride);
     int M = B * Ho * Wo, K = 9 * L.cin;
-    TcConvIn la{x, B, H, W, L.cin, Ho, Wo, L.stride};
+    TcConvIn la{x, H, W, L.cin, Ho, Wo, L.stride};
     TcRows lb{c->wb + L.woff, K};
     ConvOut ep{c->w + L.boff, y, yf, L.cout, L.relu};
     return tc_gemm(c, M, L.cout, K, la, lb, ep);
 }
 
-// backward of layer L given dy (FP32, already through the ReLU mask) and its
-// BF16 copy: weight and bias gradients, and the input gradient if dx != null
-rf_status conv_bwd(rf_cnn* c, const Layer& L, const bf16* x, int B, int H, int W,
-                   const float* dy, const bf16* dyb, float* dx) {
+// the output gradient of layer L (k_grad_in) into c->gb, and its bias gradient
+rf_status grad_in(rf_cnn* c, const Layer& L, const float* g, const float* add, const bf16* act,
+                  int P) {
+    const int nblk = (P + kGradSpan - 1) / kGradSpan;
+    if ((size_t)nblk * L.cout > c->part_floats || L.cout > kGradThreads)
+        return cfail(RF_ERR_STATE, "cnn: partial buffer too small for the bias gradient");
+    k_grad_in<<<nblk, kGradThreads, 0, c->stream>>>(g, add, act, c->gb, P, L.cout, c->part);
+    k_reduce_bias<<<L.cout, kGradThreads, 0, c->stream>>>(c->part, nblk, L.cout, c->g + L.boff);
+    c->launches += 2;
+    CN(cudaGetLastError());
+    return RF_OK;
+}
+
+// backward of layer L given its output gradient in c->gb (through the ReLU mask):
+// the weight gradient, and the input gradient if dx != null
+rf_status conv_bwd(rf_cnn* c, const Layer& L, const bf16* x, int B, int H, int W, float* dx) {
+    const bf16* dyb = c->gb;
     int Ho = Ho_of(H, L.stride), Wo = Ho_of(W, L.stride);
     int P = B * Ho * Wo, Mw = 9 * L.cin;
     // weight gradient: [tap*cin + ci] x [co] over the pixels, split over K
@@ -611,26 +688,29 @@ rf_status conv_bwd(rf_cnn* c, const Layer& L, const bf16* x, int B, int H, int W
     if (rs != RF_OK) return rs;
     k_reduce_partials<<<blocks_for((size_t)L.cout * Mw), 256, 0, c->stream>>>(
         c->part, used, L.cout * Mw, c->g + L.woff);
-    // bias: the weight-gradient partials are consumed above, so their buffer is free
-    const int span = 2048, nblk = (P + span - 1) / span;
-    if ((size_t)nblk * L.cout > c->part_floats || L.cout > kBiasThreads)
-        return cfail(RF_ERR_STATE, "cnn: partial buffer too small for the bias gradient");
-    k_bias_partial<<<nblk, kBiasThreads, 0, c->stream>>>(dy, P, L.cout, span, c->part);
-    k_reduce_partials<<<blocks_for(L.cout, 64), 64, 0, c->stream>>>(c->part, nblk, L.cout,
-                                                                   c->g + L.boff);
-    c->launches += 3;
-    if (dx) {
+    c->launches++;
+    if (dx && L.stride == 1) {
         int M = B * H * W, K = 9 * L.cout;
-        rs = tc_gemm(c, M, L.cin, K, TcDataGradA{dyb, H, W, Ho, Wo, L.cout, L.stride},
+        rs = tc_gemm(c, M, L.cin, K, TcDataGradA{dyb, H, W, L.cout},
                      TcRows{c->wt + L.woff, K}, StoreF32{dx, L.cin});
-        if (rs != RF_OK) return rs;
+    } else if (dx) {
+        for (int i = 0; i < 4 && rs == RF_OK; i++) {
+            const Parity2 q{i >> 1, i & 1};
+            const int Hc = (H - q.py + 1) / 2, Wc = (W - q.px + 1) / 2;
+            const int K = (q.py + 1) * (q.px + 1) * L.cout;
+            if (Hc > 0 && Wc > 0)
+                rs = tc_gemm(c, B * Hc * Wc, L.cin, K, TcDataGrad2A{dyb, Hc, Wc, Ho, Wo, L.cout, q},
+                             TcTapRows{c->wt + L.woff, L.cout, q},
+                             StoreF32Parity{dx, L.cin, H, W, Hc, Wc, q});
+        }
     }
+    if (rs != RF_OK) return rs;
     CN(cudaGetLastError());
     return RF_OK;
 }
 
 rf_status sync_bf16_weights(rf_cnn* c) {
-    k_f32_to_bf16<<<blocks_for(c->n_params), 256, 0, c->stream>>>(c->w, c->wb, c->n_params);
+    k_f32_to_bf16<<<blocks_for(c->n_params / 4), 256, 0, c->stream>>>(c->w, c->wb, c->n_params);
     c->launches++;
     for (size_t li = 0; li < c->layers.size(); li++) {
         const Layer& L = c->layers[li];
@@ -718,7 +798,7 @@ rf_status forward(rf_cnn* c, const float* input, int B, int H, int W) {
     const Layer &c1 = c->layers[0], &c2 = c->layers[1], &c3 = c->layers[2], &h16 = c->layers[3],
                 &c4 = c->layers[4], &h8 = c->layers[5];
     size_t nin = (size_t)B * H * W * 16;
-    k_f32_to_bf16<<<blocks_for(nin), 256, 0, c->stream>>>(input, c->x, nin);
+    k_f32_to_bf16<<<blocks_for(nin / 4), 256, 0, c->stream>>>(input, c->x, nin);
     c->launches++;
     int H2 = Ho_of(H, 2), W2 = Ho_of(W, 2);
     rf_status rs = conv_fwd(c, c1, c->x, B, H, W, c->a1, nullptr);
@@ -738,38 +818,30 @@ rf_status forward(rf_cnn* c, const float* input, int B, int H, int W) {
 rf_status backward(rf_cnn* c, int B, int H, int W) {
     const Layer &c1 = c->layers[0], &c2 = c->layers[1], &c3 = c->layers[2], &h16 = c->layers[3],
                 &c4 = c->layers[4], &h8 = c->layers[5];
-    int H2 = Ho_of(H, 2), W2 = Ho_of(W, 2);
-    size_t n8 = (size_t)B * H * W * 8, n16 = (size_t)B * H2 * W2 * 8;
+    const int H2 = Ho_of(H, 2), W2 = Ho_of(W, 2), P = B * H * W, P2 = B * H2 * W2;
+    const size_t n3 = (size_t)P2 * c3.cout, n1 = (size_t)P * c1.cout;
     // heads (linear)
-    k_f32_to_bf16<<<blocks_for(n8), 256, 0, c->stream>>>(c->g_o8, c->gb, n8);
-    rf_status rs = conv_bwd(c, h8, c->a4, B, H, W, c->g_o8, c->gb, c->g_a4);
-    if (rs != RF_OK) return rs;
-    size_t n4 = (size_t)B * H * W * c4.cout;
-    k_relu_grad<<<blocks_for(n4 / 4), 256, 0, c->stream>>>(c->g_a4, nullptr, c->a4, c->gb, n4);
-    rs = conv_bwd(c, c4, c->cat, B, H, W, c->g_a4, c->gb, c->g_cat);
+    rf_status rs = grad_in(c, h8, c->g_o8, nullptr, nullptr, P);
+    if (rs == RF_OK) rs = conv_bwd(c, h8, c->a4, B, H, W, c->g_a4);
+    if (rs == RF_OK) rs = grad_in(c, c4, c->g_a4, nullptr, c->a4, P);
+    if (rs == RF_OK) rs = conv_bwd(c, c4, c->cat, B, H, W, c->g_cat);
     if (rs != RF_OK) return rs;
     // split the concat gradient: g_a3 = up^T(g_cat[:96]), g_a1 = g_cat[96:]
-    size_t n3 = (size_t)B * H2 * W2 * c3.cout;
-    size_t n1 = (size_t)B * H * W * c1.cout;
     k_concat_up_grad<<<blocks_for(std::max(n3, n1) / 4), 256, 0, c->stream>>>(
         c->g_cat, H2, W2, c3.cout, c1.cout, B, H, W, c->g_a3, c->g_a1);
+    c->launches++;
     // 1/16 head adds into g_a3
-    k_f32_to_bf16<<<blocks_for(n16), 256, 0, c->stream>>>(c->g_o16, c->gb, n16);
     float* tmp = c->g_a2;  // scratch for the head's input gradient (same size as g_a3)
-    rs = conv_bwd(c, h16, c->a3, B, H2, W2, c->g_o16, c->gb, tmp);
-    if (rs != RF_OK) return rs;
-    k_relu_grad<<<blocks_for(n3 / 4), 256, 0, c->stream>>>(c->g_a3, tmp, c->a3, c->gb, n3);
-    rs = conv_bwd(c, c3, c->a2, B, H2, W2, c->g_a3, c->gb, c->g_a2);
-    if (rs != RF_OK) return rs;
-    size_t n2 = (size_t)B * H2 * W2 * c2.cout;
-    k_relu_grad<<<blocks_for(n2 / 4), 256, 0, c->stream>>>(c->g_a2, nullptr, c->a2, c->gb, n2);
+    rs = grad_in(c, h16, c->g_o16, nullptr, nullptr, P2);
+    if (rs == RF_OK) rs = conv_bwd(c, h16, c->a3, B, H2, W2, tmp);
+    if (rs == RF_OK) rs = grad_in(c, c3, c->g_a3, tmp, c->a3, P2);
+    if (rs == RF_OK) rs = conv_bwd(c, c3, c->a2, B, H2, W2, c->g_a2);
+    if (rs == RF_OK) rs = grad_in(c, c2, c->g_a2, nullptr, c->a2, P2);
     // c2's input gradient adds into g_a1 (which holds the skip part): use tmp2
     float* tmp2 = c->g_a4;  // free now, large enough (B*H*W*64 >= B*H*W*32)
-    rs = conv_bwd(c, c2, c->a1, B, H, W, c->g_a2, c->gb, tmp2);
-    if (rs != RF_OK) return rs;
-    k_relu_grad<<<blocks_for(n1 / 4), 256, 0, c->stream>>>(c->g_a1, tmp2, c->a1, c->gb, n1);
-    rs = conv_bwd(c, c1, c->x, B, H, W, c->g_a1, c->gb, nullptr);
-    c->launches += 7;
+    if (rs == RF_OK) rs = conv_bwd(c, c2, c->a1, B, H, W, tmp2);
+    if (rs == RF_OK) rs = grad_in(c, c1, c->g_a1, tmp2, c->a1, P);
+    if (rs == RF_OK) rs = conv_bwd(c, c1, c->x, B, H, W, nullptr);
     if (rs != RF_OK) return rs;
     CN(cudaGetLastError());
     return RF_OK;
@@ -1009,12 +1081,12 @@ rf_status rf_cnn_backward(rf_cnn* c, const float* input, const float* tgt16, con
     int H2 = (H + 1) / 2, W2 = (W + 1) / 2;
     int P8 = B * H * W, P16 = B * H2 * W2;
     CN(cudaMemsetAsync(c->d_loss, 0, sizeof(double), c->stream));
-    k_l1_loss<<<blocks_for(P16), 256, 0, c->stream>>>(c->o16, tgt16, mask16, P16, 8, weights[0],
-                                                      weights[1], weights[2], 1.0f / P16,
-                                                      c->g_o16, c->d_loss);
-    k_l1_loss<<<blocks_for(P8), 256, 0, c->stream>>>(c->o8, tgt8, mask8, P8, 8, weights[0],
-                                                     weights[1], weights[2], 1.0f / P8, c->g_o8,
-                                                     c->d_loss);
+    k_l1_loss<<<blocks_for(P16), 256, 0, c->stream>>>((const float4*)c->o16, tgt16, mask16, P16,
+                                                      weights[0], weights[1], weights[2],
+                                                      1.0f / P16, (float4*)c->g_o16, c->d_loss);
+    k_l1_loss<<<blocks_for(P8), 256, 0, c->stream>>>((const float4*)c->o8, tgt8, mask8, P8,
+                                                     weights[0], weights[1], weights[2], 1.0f / P8,
+                                                     (float4*)c->g_o8, c->d_loss);
     c->launches += 2;
     rs = backward(c, B, H, W);
     if (rs != RF_OK) return rs;

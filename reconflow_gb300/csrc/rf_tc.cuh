@@ -20,14 +20,14 @@
 // What bounds it is feeding the copies.  kLbo is 144 and not 128 so that the
 // eight copies of a row (K groups g = 0 .. 7, issued by neighbouring threads,
 // 128 contiguous bytes of global memory) land in different banks: at 128 they
-// shared four banks and a chunk took 8 times as long to write.  And an operand
-// hands out what its address computation can reuse: row(r) once per thread and
-// row before the loop, kpos(k) once per thread and chunk, at(row, kpos) per
-// copy (null for zeros); with all of it per copy, the integer divisions of the
-// im2col index took longer than the copies.  On 64 images of 160 x 120 the
-// 128 -> 64 layer takes 1.12 ms forward and 0.86 ms for its input gradient
-// (1.71 and 1.83 before), its tile traffic (4.1 GB through L2) and one barrier
-// per chunk bounding it now.
+// shared four banks and a chunk took 8 times as long to write.  The copies go
+// through L1 (cp.async.ca): the three taps of a row overlap in all but one pixel,
+// and past L1 every layer waited for L2.  And a copy's address is a bit test, an
+// addition and a select (TcRow, TcPos); the integer divisions of the im2col index
+// are made once per thread and row, and once per thread and chunk.  On 64 images
+// of 160 x 120 the 128 -> 64 layer takes 0.59 ms forward (past L1 1.12) and 0.54
+// for its input gradient (0.87), bound by the latency of the copies: eight warps
+// per SM, two chunks each in flight.
 //
 // The epilogue functor receives a row's eight consecutive columns (m, n, v[8]; N
 // a multiple of 8) and stores them as vectors: a thread has a row, so scalar
@@ -148,6 +148,27 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8]) {
     for (int i = 0; i < 8; i++) v[i] = __uint_as_float(r[i]);
 }
 
+// An operand of k_tc_gemm hands out, in units of 16 bytes (8 elements) from base():
+// where a row starts and which of its taps exist (bit t of `taps`; never bit 31),
+// and where K group k lies from there and which tap it belongs to.  A copy is then
+// a bit test, an addition and a select.
+struct TcRow {
+    int off;
+    unsigned taps;
+};
+struct TcPos {
+    int off, tap;
+};
+// which taps ky * 3 + kx of a 3x3 window whose first pixel is (y, x) lie in a level
+__device__ __forceinline__ unsigned conv_taps(int y, int x, int H, int W) {
+    unsigned cols = 0, t = 0;
+#pragma unroll
+    for (int i = 0; i < 3; i++) cols |= (unsigned)(x + i) < (unsigned)W ? 1u << i : 0u;
+#pragma unroll
+    for (int i = 0; i < 3; i++) t |= (unsigned)(y + i) < (unsigned)H ? cols << 3 * i : 0u;
+    return t;
+}
+
 // a chunk tile in shared memory: core matrices along K and along M / N
 constexpr int kLbo = 144, kSbo = kTK / 8 * kLbo;
 // byte offset of element row r, k-group g (8 elements) in a chunk tile
@@ -156,7 +177,7 @@ __device__ __forceinline__ uint32_t tile_off(int r, int g) {
 }
 
 __device__ __forceinline__ void cp_async16(void* smem_dst, const void* gsrc, int src_bytes) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(smem_dst)),
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(smem_dst)),
                  "l"(gsrc), "r"(src_bytes)
                  : "memory");
 }
@@ -220,8 +241,9 @@ __global__ void __launch_bounds__(kThreads) k_tc_gemm(int M, int N, int K, LA la
     constexpr int kPerA = kTM * (kTK / 8) / kThreads;  // 8
     constexpr int kPerB = NT * (kTK / 8) / kThreads;   // NT / 16
     const int g = tid & 7, r0 = tid >> 3;
-    typename LA::Row ra[kPerA];
-    typename LB::Row rb[kPerB];
+    TcRow ra[kPerA], rb[kPerB];
+    const uint4* const base_a = la.base();
+    const uint4* const base_b = lb.base();
 #pragma unroll
     for (int j = 0; j < kPerA; j++) ra[j] = la.row(m0 + r0 + 16 * j, M);
 #pragma unroll
@@ -233,18 +255,17 @@ __global__ void __launch_bounds__(kThreads) k_tc_gemm(int M, int N, int K, LA la
         unsigned char* tA = base + q * S::kA + tile_off(r0, g);
         unsigned char* tB = base + kStages * S::kA + q * S::kB + tile_off(r0, g);
         const int k = c * kTK + g * 8;
-        const bool in = k < K;
-        const auto ka = la.kpos(k);
-        const auto kb = lb.kpos(k);
+        TcPos ka = la.kpos(k), kb = lb.kpos(k);
+        if (k >= K) ka.tap = kb.tap = 31;
 #pragma unroll
         for (int j = 0; j < kPerA; j++) {
-            const void* src = in ? la.at(ra[j], ka) : nullptr;
-            cp_async16(tA + 2 * j * kSbo, src ? src : la.base(), src ? 16 : 0);
+            const bool ok = ra[j].taps >> ka.tap & 1u;
+            cp_async16(tA + 2 * j * kSbo, base_a + (ok ? ra[j].off + ka.off : 0), ok ? 16 : 0);
         }
 #pragma unroll
         for (int j = 0; j < kPerB; j++) {
-            const void* src = in ? lb.at(rb[j], kb) : nullptr;
-            cp_async16(tB + 2 * j * kSbo, src ? src : lb.base(), src ? 16 : 0);
+            const bool ok = rb[j].taps >> kb.tap & 1u;
+            cp_async16(tB + 2 * j * kSbo, base_b + (ok ? rb[j].off + kb.off : 0), ok ? 16 : 0);
         }
     };
 
@@ -324,7 +345,7 @@ __global__ void __launch_bounds__(kThreads) k_tc_gemm(int M, int N, int K, LA la
 // activation as it lies in memory and nothing is transposed.  (Gathering them
 // K-major, 8 scalar loads per 16 bytes with a division chain each, took 6.7 of
 // a 28 ms training step for the 128 -> 64 layer alone, 64 images of 160 x 120;
-// this takes 1.04 ms of 8.1, and all six layers 2.4 instead of 17.1.)  The order of the
+// this takes 0.66, and all six layers 1.5 instead of 17.1.)  The order of the
 // reduction is that of k_tc_gemm: pixels in order, 16 per MMA, split at the
 // same places.
 //
@@ -383,15 +404,17 @@ __global__ void __launch_bounds__(kThreads) k_tc_wgrad(int M, int N, int K, int 
         img = r / w.Ho;
     }
     constexpr int kGA = kTM / 16, kGB = NT / 16;  // channel groups per thread
-    // tap and channel of each of this thread's A groups (a tap of -1: past M)
-    int tap[kGA], coff[kGA];
+    // tap of each of this thread's A groups (31: past M), and where it lies from the
+    // pixel's first channel in units of 16 bytes
+    int tap[kGA], goff[kGA];
 #pragma unroll
     for (int j = 0; j < kGA; j++) {
-        const int m = m0 + 8 * (g0 + 2 * j);
-        tap[j] = m < M ? m / w.C : -1;
-        const int ky = m / w.C / 3, kx = m / w.C % 3;
-        coff[j] = ((ky - 1) * w.W + (kx - 1)) * w.C + m % w.C;
+        const int m = m0 + 8 * (g0 + 2 * j), t = m / w.C;
+        tap[j] = m < M ? t : 31;
+        goff[j] = (((t / 3 - 1) * w.W + (t % 3 - 1)) * w.C + m % w.C) / 8;
     }
+    const uint4* const xv = reinterpret_cast<const uint4*>(w.x);
+    const uint4* const dv = reinterpret_cast<const uint4*>(w.dy);
 
     auto issue = [&](int c) {
         const int q = c % kStages;
@@ -399,20 +422,18 @@ __global__ void __launch_bounds__(kThreads) k_tc_wgrad(int M, int N, int K, int 
         unsigned char* tB = base + kStages * S::kA + q * S::kB + g0 * kWgGroup + pk * 16;
         const bool in = p < k_end;
         const int y = yo * w.stride, x = xo * w.stride;
-        const __nv_bfloat16* xp = w.x + (((size_t)img * w.H + y) * w.W + x) * w.C;
+        const int off = ((img * w.H + y) * w.W + x) * (w.C / 8);
+        const unsigned taps = in ? conv_taps(y - 1, x - 1, w.H, w.W) : 0u;
 #pragma unroll
         for (int j = 0; j < kGA; j++) {
-            const int ky = tap[j] / 3, kx = tap[j] - 3 * ky;
-            const bool ok = in && tap[j] >= 0 && (unsigned)(y + ky - 1) < (unsigned)w.H &&
-                            (unsigned)(x + kx - 1) < (unsigned)w.W;
-            cp_async16(tA + 2 * j * kWgGroup, ok ? xp + coff[j] : w.x, ok ? 16 : 0);
+            const bool ok = taps >> tap[j] & 1u;
+            cp_async16(tA + 2 * j * kWgGroup, xv + (ok ? off + goff[j] : 0), ok ? 16 : 0);
         }
-        const __nv_bfloat16* dp = w.dy + (size_t)p * w.Cout;
+        const int doff = p * (w.Cout / 8) + g0;
 #pragma unroll
         for (int j = 0; j < kGB; j++) {
-            const int n = 8 * (g0 + 2 * j);
-            const bool ok = in && n < N;
-            cp_async16(tB + 2 * j * kWgGroup, ok ? dp + n : w.dy, ok ? 16 : 0);
+            const bool ok = in && 8 * (g0 + 2 * j) < N;
+            cp_async16(tB + 2 * j * kWgGroup, dv + (ok ? doff + 2 * j : 0), ok ? 16 : 0);
         }
         p += kTK;
         xo += kTK;
