@@ -729,31 +729,52 @@ rf_status sync_bf16_weights(rf_cnn* c) {
 }
 
 // one stride-1 layer on the direct kernel: `map` covers its padded input
-template <int NT>
-rf_status conv3_direct(rf_cnn* c, int li, const CUtensorMap& map, int B, int H, int W,
-                       bf16* y, float* yf) {
+template <int NT, int MT>
+rf_status conv3_launch(rf_cnn* c, int li, const CUtensorMap& map, int B, int H, int W, bf16* y,
+                       float* yf) {
     const Layer& L = c->layers[li];
-    using S = rf_tc::ConvSmem<NT>;
+    using S = rf_tc::ConvSmem<NT, MT>;
     rf_tc::ConvGeom g;
     g.Wp = W + 2;
     g.npos = B * (H + 2) * (W + 2);
-    g.nbox = (rf_tc::kTM + 2 * (W + 3) + rf_tc::kConvBox - 1) / rf_tc::kConvBox;
+    g.nbox = S::nbox(W);
     g.stages = L.cin / 16;
     const size_t smem = S::bytes(g.nbox);
     static bool attr_set = false;
     if (!attr_set) {
-        CN(cudaFuncSetAttribute(rf_tc::k_tc_conv3<NT, ConvOutPadded>,
+        CN(cudaFuncSetAttribute(rf_tc::k_tc_conv3<NT, MT, ConvOutPadded>,
                                 cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
         attr_set = true;
     }
     if (smem > 227 * 1024) return cfail(RF_ERR_UNSUPPORTED, "cnn: row too long for the direct kernel");
     ConvOutPadded ep{c->w + L.boff, L.cout, y, L.cout, yf, L.cout, L.relu, H, W, g.npos};
-    const unsigned grid = (unsigned)((g.npos + rf_tc::kTM - 1) / rf_tc::kTM);
-    rf_tc::k_tc_conv3<NT, ConvOutPadded><<<grid, rf_tc::kThreads, smem, c->stream>>>(
-        map, c->wc[li], g, ep, c->d_status, c->test_first_wait_polls);
+    const int tile = rf_tc::kTM * MT;
+    rf_tc::k_tc_conv3<NT, MT, ConvOutPadded>
+        <<<(unsigned)((g.npos + tile - 1) / tile), rf_tc::kThreads, smem, c->stream>>>(
+            map, c->wc[li], g, ep, c->d_status, c->test_first_wait_polls);
     c->launches++;
     CN(cudaGetLastError());
     return RF_OK;
+}
+// The largest of 512, 256 and 128 positions per CTA with which every SM gets a CTA
+// and two fit on it.  Fewer, larger tiles load the weights and the two rows around a
+// tile less often (64 images of 160 x 90: 0.92 ms with 128, 0.72 with at most 256,
+// 0.71 with 512); with too few of them SMs idle (four images: 0.114 ms with at most
+// 256, 0.130 with 128, one image the same either way).
+template <int NT>
+rf_status conv3_direct(rf_cnn* c, int li, const CUtensorMap& map, int B, int H, int W, bf16* y,
+                       float* yf) {
+    const long long npos = (long long)B * (H + 2) * (W + 2);
+    auto fits = [&](int mt, size_t bytes) {
+        return npos >= 152ll * rf_tc::kTM * mt && bytes <= 113 * 1024;
+    };
+    if constexpr (NT <= 64) {
+        using S = rf_tc::ConvSmem<NT, 4>;
+        if (fits(4, S::bytes(S::nbox(W)))) return conv3_launch<NT, 4>(c, li, map, B, H, W, y, yf);
+    }
+    using S = rf_tc::ConvSmem<NT, 2>;
+    if (fits(2, S::bytes(S::nbox(W)))) return conv3_launch<NT, 2>(c, li, map, B, H, W, y, yf);
+    return conv3_launch<NT, 1>(c, li, map, B, H, W, y, yf);
 }
 
 // inference: padded activations (laid out for this call's frame size, up to
@@ -877,10 +898,10 @@ bool encode_positions_map(CUtensorMap* m, const bf16* base, int C, size_t npos) 
 
 // whether the direct kernel's shared memory fits rows of width W
 bool direct_fits(int W) {
-    const int nbox = (rf_tc::kTM + 2 * (W + 3) + rf_tc::kConvBox - 1) / rf_tc::kConvBox;
     const size_t lim = 227 * 1024;
-    return rf_tc::ConvSmem<32>::bytes(nbox) <= lim && rf_tc::ConvSmem<64>::bytes(nbox) <= lim &&
-           rf_tc::ConvSmem<96>::bytes(nbox) <= lim;
+    auto bytes = [&](auto smem) { return smem.bytes(smem.nbox(W)); };
+    return bytes(rf_tc::ConvSmem<32, 1>{}) <= lim && bytes(rf_tc::ConvSmem<64, 1>{}) <= lim &&
+           bytes(rf_tc::ConvSmem<96, 1>{}) <= lim;
 }
 
 }  // namespace rf_cnn_impl

@@ -519,15 +519,15 @@ __global__ void __launch_bounds__(kThreads) k_tc_wgrad(int M, int N, int K, int 
 // q + (dy - 1)(W + 2) + (dx - 1), so 128 consecutive output positions read
 // 128 consecutive input positions for every tap: each tap is one MMA whose
 // A operand is a shifted view of one staged slab, and no im2col copy exists.
-// A CTA computes positions [q0, q0 + 128) (border positions too; their
+// A CTA computes positions [q0, q0 + 128 MT) (border positions too; their
 // outputs are not stored, so borders stay zero).  Per stage of 16 input
 // channels it stages, by TMA, the slab of input positions
-// [q0 - (W + 3), q0 + 128 + (W + 3)) as two planes of 8 channels (16 bytes
+// [q0 - (W + 3), q0 + 128 MT + (W + 3)) as two planes of 8 channels (16 bytes
 // per position: the canonical no-swizzle K-major layout, core matrices of 8
 // positions, the two K halves one plane apart), and by a bulk copy the
 // stage's weights for all 9 taps in the same layout (host-prepared), then
-// one thread issues the 9 MMAs (M = 128, N = NT, K = 16) into the TMEM
-// accumulator.  kConvStages ring slots: loads of the next stages run while
+// one thread issues the 9 MT MMAs (M = 128, N = NT, K = 16) into the TMEM
+// accumulators.  kStages ring slots: loads of the next stages run while
 // a stage's MMAs do.  Out-of-range slab positions (before the first image,
 // past the buffer) are filled with zeros by the TMA unit and only reach
 // border outputs.
@@ -536,7 +536,7 @@ constexpr int kConvBox = 128;  // positions per TMA box (2 KB per 8-channel plan
 struct ConvGeom {
     int Wp;      // padded row length W + 2
     int npos;    // padded positions of this call: B (H + 2)(W + 2)
-    int nbox;    // TMA boxes per plane: ceil((128 + 2 (W + 3)) / 128)
+    int nbox;    // TMA boxes per plane: ceil((128 MT + 2 (W + 3)) / 128)
     int stages;  // input channels / 16
 };
 
@@ -566,12 +566,14 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t b
         : "memory");
 }
 
-template <int NT>
+template <int NT, int MT>
 struct ConvSmem {
-    static_assert(NT % 16 == 0 && NT >= 16 && NT <= 128, "N tile");
-    static constexpr int kStages = NT >= 96 ? 2 : 3;
+    static_assert(NT % 16 == 0 && NT >= 16 && NT <= 128 && NT * MT <= 256, "tile");
+    static constexpr int kStages = MT > 1 || NT >= 96 ? 2 : 3;
     static constexpr uint32_t kWBytes = 9u * NT * 32u;  // one stage's weights
-    static constexpr uint32_t kCols = NT <= 32 ? 32 : (NT <= 64 ? 64 : 128);
+    static constexpr uint32_t kN = NT * MT;
+    static constexpr uint32_t kCols = kN <= 32 ? 32 : (kN <= 64 ? 64 : (kN <= 128 ? 128 : 256));
+    static int nbox(int W) { return (kTM * MT + 2 * (W + 3) + kConvBox - 1) / kConvBox; }
     __host__ __device__ static uint32_t plane_bytes(int nbox) { return (uint32_t)nbox * kConvBox * 16u; }
     __host__ __device__ static uint32_t stage_bytes(int nbox) { return 2u * plane_bytes(nbox) + kWBytes; }
     static size_t bytes(int nbox) { return (size_t)kStages * stage_bytes(nbox) + 2048; }
@@ -584,13 +586,13 @@ struct ConvSmem {
 // caps the first slab wait of each CTA (a test hook, as for k_tc_gemm).
 // Every load issued is waited for (with the full limit) before the CTA
 // ends, and the last MMA commit before TMEM is released.
-template <int NT, class EP>
+template <int NT, int MT, class EP>
 __global__ void __launch_bounds__(kThreads) k_tc_conv3(const __grid_constant__ CUtensorMap xmap,
                                                       const __nv_bfloat16* __restrict__ wc,
                                                       ConvGeom g, EP ep, int* status,
                                                       int first_wait_polls) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
-    using S = ConvSmem<NT>;
+    using S = ConvSmem<NT, MT>;
     constexpr int kS = S::kStages;
     unsigned char* base = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     const uint32_t plane = S::plane_bytes(g.nbox);
@@ -603,7 +605,7 @@ __global__ void __launch_bounds__(kThreads) k_tc_conv3(const __grid_constant__ C
     int* committed = fail + 2;  // stages whose MMAs were committed
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int q0 = blockIdx.x * kTM;
+    const int q0 = blockIdx.x * kTM * MT;
     const int halo = g.Wp + 1;
     const int nst = g.stages;
 
@@ -652,9 +654,12 @@ __global__ void __launch_bounds__(kThreads) k_tc_conv3(const __grid_constant__ C
 #pragma unroll
             for (int t = 0; t < 9; t++) {
                 const int off = halo + (t / 3 - 1) * g.Wp + (t % 3 - 1);
-                const uint64_t da = smem_desc(a0 + (uint32_t)off * 16u, plane, 128);
                 const uint64_t db = smem_desc(b0 + (uint32_t)t * NT * 32u, 128, 256);
-                mma_bf16(tmem, da, db, idesc, (j > 0 || t > 0) ? 1u : 0u);
+#pragma unroll
+                for (int i = 0; i < MT; i++) {
+                    const uint64_t da = smem_desc(a0 + (uint32_t)(off + kTM * i) * 16u, plane, 128);
+                    mma_bf16(tmem + (uint32_t)(i * NT), da, db, idesc, (j > 0 || t > 0) ? 1u : 0u);
+                }
             }
             mma_commit(&empty[sl]);
             *committed = j + 1;
@@ -686,14 +691,17 @@ __global__ void __launch_bounds__(kThreads) k_tc_conv3(const __grid_constant__ C
     if (*fail) {
         if (tid == 0) atomicExch(status, 1);
     } else if (nst > 0) {
-        const int q = q0 + warp * 32 + lane;
-        const int p = ep.pos(q);  // < 0: a border position or past the call's positions
-        const uint32_t lane_addr = tmem + ((uint32_t)(warp * 32) << 16);
 #pragma unroll 1
-        for (int c = 0; c < NT; c += 8) {
-            float v[8];
-            tmem_ld8(lane_addr + (uint32_t)c, v);
-            if (p >= 0) ep.store(q, p, c, v);
+        for (int i = 0; i < MT; i++) {
+            const int q = q0 + i * kTM + warp * 32 + lane;
+            const int p = ep.pos(q);  // < 0: a border position or past the call's positions
+            const uint32_t lane_addr = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(i * NT);
+#pragma unroll 1
+            for (int c = 0; c < NT; c += 8) {
+                float v[8];
+                tmem_ld8(lane_addr + (uint32_t)c, v);
+                if (p >= 0) ep.store(q, p, c, v);
+            }
         }
     }
     tc_fence_before();
