@@ -413,15 +413,16 @@ __global__ void k_adam(float* w, const float* g, float* m, float* v, size_t n, f
 inline unsigned blocks_for(size_t n, int t = 256) { return (unsigned)((n + t - 1) / t); }
 
 // ---- inference path on padded activations (rf_tc::k_tc_conv3) -------------
-// A padded buffer holds [B][H + 2][W + 2][C] BF16 with a zero one-pixel
-// border; interior pixel (b, y, x) is at position (b (H + 2) + y + 1)(W + 2)
-// + x + 1.  Borders are zeroed once at creation and never written.
+// A padded buffer holds [C / 8] planes of [B][H + 2][W + 2] positions of 8 BF16
+// channels with a zero one-pixel border; interior pixel (b, y, x) is at position
+// (b (H + 2) + y + 1)(W + 2) + x + 1.  Borders are zeroed when a frame size is
+// first used and never written; planes are max_batch images apart.
 __device__ __forceinline__ size_t pad_pos(int b, int y, int x, int H, int W) {
     return ((size_t)b * (H + 2) + y + 1) * (W + 2) + x + 1;
 }
 
 // FP32 input [B][H][W][16] -> padded BF16 interior, 8 channels per thread
-__global__ void k_pad_input(const float* in, int B, int H, int W, bf16* xp) {
+__global__ void k_pad_input(const float* in, int B, int H, int W, size_t plane, bf16* xp) {
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     size_t n = (size_t)B * H * W * 2;
     if (i >= n) return;
@@ -432,23 +433,19 @@ __global__ void k_pad_input(const float* in, int B, int H, int W, bf16* xp) {
     bf16 v[8];
 #pragma unroll
     for (int e = 0; e < 8; e++) v[e] = __float2bfloat16(s[e]);
-    *(uint4*)(xp + pad_pos(b, y, x, H, W) * 16 + g * 8) = pack8(v);
+    *(uint4*)(xp + (g * plane + pad_pos(b, y, x, H, W)) * 8) = pack8(v);
 }
 
-// padded cat = [nearest 2x upsample of a (Ha x Wa x Ca), b (H x W x Cb)],
-// 8 channels per thread (Ca, Cb multiples of 8)
-__global__ void k_concat_up_pad(const bf16* a, int Ha, int Wa, int Ca, const bf16* bsrc, int Cb,
-                                int Bn, int H, int W, bf16* cat) {
-    const int C = Ca + Cb, G = C / 8;
-    size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    size_t n = (size_t)Bn * H * W * G;
-    if (i >= n) return;
-    const int c = (int)(i % G) * 8;
-    const size_t p = i / G;
-    const int x = (int)(p % W), r = (int)(p / W), y = r % H, bb = r / H;
-    uint4 v = c < Ca ? *(const uint4*)(a + pad_pos(bb, y / 2, x / 2, Ha, Wa) * Ca + c)
-                     : *(const uint4*)(bsrc + pad_pos(bb, y, x, H, W) * Cb + (c - Ca));
-    *(uint4*)(cat + pad_pos(bb, y, x, H, W) * C + c) = v;
+// nearest 2x upsample of the padded a (Ha x Wa), plane blockIdx.y, a pixel per
+// thread.  (What follows those planes in the concatenation, the convolution reads
+// where it is: ConvGeom::x2.)
+__global__ void k_up_pad(const bf16* a, int Ha, int Wa, size_t plane_a, int Bn, int H, int W,
+                         size_t plane, bf16* out) {
+    const size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= (size_t)Bn * H * W) return;
+    const int x = (int)(p % W), r = (int)(p / W), y = r % H, b = r / H;
+    const uint4 v = *(const uint4*)(a + (blockIdx.y * plane_a + pad_pos(b, y / 2, x / 2, Ha, Wa)) * 8);
+    *(uint4*)(out + (blockIdx.y * plane + pad_pos(b, y, x, H, W)) * 8) = v;
 }
 
 // weights [co][tap][ci] -> the direct kernel's [stage][tap][NT / 8][2][8][8]
@@ -471,10 +468,9 @@ __global__ void k_conv_wc(const bf16* w, int cin, int cout, int NT, bf16* wc) {
 struct ConvOutPadded {
     const float* bias;
     int nbias;
-    bf16* y;  // padded [pos][cout] or null
-    int cout;
+    bf16* y;  // padded or null
+    size_t plane;
     float* yf;  // unpadded FP32 or null
-    int cout_f;
     int relu, H, W, npos;
     __device__ int pos(int q) const {
         if (q >= npos) return -1;
@@ -483,23 +479,27 @@ struct ConvOutPadded {
         if (x < 1 || x > W || yy < 1 || yy > H) return -1;
         return (b * H + yy - 1) * W + (x - 1);
     }
-    __device__ void store(int q, int p, int c, const float (&v)[8]) const {
-        float o[8];
+    __device__ void store(int q, int p, int c0, const float (&v)[16]) const {
 #pragma unroll
-        for (int e = 0; e < 8; e++) {
-            float t = v[e] + (c + e < nbias ? bias[c + e] : 0.f);
-            o[e] = relu ? fmaxf(t, 0.f) : t;
+        for (int h = 0; h < 2; h++) {
+            const int c = c0 + 8 * h;
+            if (c >= nbias) return;  // a multiple of 8
+            const float4 b0 = *(const float4*)(bias + c), b1 = *(const float4*)(bias + c + 4);
+            const float b[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+            float o[8];
+#pragma unroll
+            for (int e = 0; e < 8; e++) {
+                const float t = v[8 * h + e] + b[e];
+                o[e] = relu ? fmaxf(t, 0.f) : t;
+            }
+            if (y) {
+                bf16 t[8];
+#pragma unroll
+                for (int e = 0; e < 8; e++) t[e] = __float2bfloat16(o[e]);
+                *(uint4*)(y + (c / 8 * plane + q) * 8) = pack8(t);
+            }
+            if (yf) store8(yf + (size_t)p * nbias + c, o);
         }
-        if (y && c < cout) {
-            bf16 h[8];
-#pragma unroll
-            for (int e = 0; e < 8; e++) h[e] = __float2bfloat16(o[e]);
-            *(uint4*)(y + (size_t)q * cout + c) = pack8(h);
-        }
-        if (yf)
-#pragma unroll
-            for (int e = 0; e < 8; e++)
-                if (c + e < cout_f) yf[(size_t)p * cout_f + c + e] = o[e];
     }
 };
 
@@ -507,28 +507,28 @@ struct ConvOutPadded {
 // border supplies the zeros of the padding)
 struct TcConvInPadded {
     const bf16* x;
-    int H, W, C, Ho, Wo, stride;
+    int H, W, C, Ho, Wo, stride, plane;
     __device__ const uint4* base() const { return units(x); }
     __device__ TcRow row(int m, int M) const {
         const int xo = m % Wo, r = m / Wo, yo = r % Ho, b = r / Ho;
-        return TcRow{((b * (H + 2) + yo * stride) * (W + 2) + xo * stride) * (C / 8),
-                     m < M ? 1u : 0u};
+        return TcRow{(b * (H + 2) + yo * stride) * (W + 2) + xo * stride, m < M ? 1u : 0u};
     }
     __device__ TcPos kpos(int k) const {
         const int ci = k % C, t = k / C;
-        return TcPos{(t / 3 * (W + 2) + t % 3) * (C / 8) + ci / 8, 0};
+        return TcPos{t / 3 * (W + 2) + t % 3 + ci / 8 * plane, 0};
     }
 };
 
 struct ConvOutToPadded {
     const float* bias;
     bf16* y;
-    int Cout, relu, Ho, Wo;
+    int relu, Ho, Wo;
+    size_t plane;
     __device__ void operator()(int m, int n, const float (&v)[8]) const {
         float o[8];
         bias_relu(bias + n, relu, v, o);
         const int xo = m % Wo, r = m / Wo, yo = r % Ho, b = r / Ho;
-        *(uint4*)(y + pad_pos(b, yo, xo, Ho, Wo) * Cout + n) = pack8(o);
+        *(uint4*)(y + (n / 8 * plane + pad_pos(b, yo, xo, Ho, Wo)) * 8) = pack8(o);
     }
 };
 
@@ -564,13 +564,13 @@ struct rf_cnn {
     uint64_t launches = 0;
     // inference on padded activations (rf_cnn_forward; training keeps the GEMMs)
     bool direct = false;
-    bf16 *xp = nullptr, *a1p = nullptr, *a2p = nullptr, *a3p = nullptr, *catp = nullptr,
-         *a4p = nullptr;
+    bf16* pad[6] = {};  // the allocations: kConvMargin positions, the planes, the margin
+    bf16 *xp = nullptr, *a1p = nullptr, *a2p = nullptr, *a3p = nullptr, *upp = nullptr,
+         *a4p = nullptr;  // their first planes
     int pad_h = -1, pad_w = -1;  // the frame size whose borders the padded buffers hold zero
     size_t pad_elems[6] = {};    // BF16 elements allocated per padded buffer
     bf16* wc[6] = {};  // per layer, the direct kernel's weight layout (null: c2)
     int nt[6] = {};    // per layer, the direct kernel's N tile
-    CUtensorMap map_x{}, map_a2{}, map_a3{}, map_cat{}, map_a4{};
 };
 
 namespace rf_cnn_impl {
@@ -728,18 +728,23 @@ rf_status sync_bf16_weights(rf_cnn* c) {
     return RF_OK;
 }
 
-// one stride-1 layer on the direct kernel: `map` covers its padded input
+// the input planes of a layer: `split` of them at x, the rest at x2
+struct ConvInput {
+    const bf16 *x, *x2;
+    int split;
+};
+size_t pad_plane(const rf_cnn* c, int H, int W) {
+    return (size_t)c->max_batch * (H + 2) * (W + 2);
+}
+
+// one stride-1 layer on the direct kernel
 template <int NT, int MT>
-rf_status conv3_launch(rf_cnn* c, int li, const CUtensorMap& map, int B, int H, int W, bf16* y,
-                       float* yf) {
+rf_status conv3_launch(rf_cnn* c, int li, ConvInput in, int B, int H, int W, bf16* y, float* yf) {
     const Layer& L = c->layers[li];
     using S = rf_tc::ConvSmem<NT, MT>;
-    rf_tc::ConvGeom g;
-    g.Wp = W + 2;
-    g.npos = B * (H + 2) * (W + 2);
-    g.nbox = S::nbox(W);
-    g.stages = L.cin / 16;
-    const size_t smem = S::bytes(g.nbox);
+    const rf_tc::ConvGeom g{W + 2, B * (H + 2) * (W + 2), L.cin / 16, in.x, in.x2, in.split,
+                            pad_plane(c, H, W)};
+    const size_t smem = S::bytes(g.Wp);
     static bool attr_set = false;
     if (!attr_set) {
         CN(cudaFuncSetAttribute(rf_tc::k_tc_conv3<NT, MT, ConvOutPadded>,
@@ -747,34 +752,25 @@ rf_status conv3_launch(rf_cnn* c, int li, const CUtensorMap& map, int B, int H, 
         attr_set = true;
     }
     if (smem > 227 * 1024) return cfail(RF_ERR_UNSUPPORTED, "cnn: row too long for the direct kernel");
-    ConvOutPadded ep{c->w + L.boff, L.cout, y, L.cout, yf, L.cout, L.relu, H, W, g.npos};
+    ConvOutPadded ep{c->w + L.boff, L.cout, y, g.plane, yf, L.relu, H, W, g.npos};
     const int tile = rf_tc::kTM * MT;
     rf_tc::k_tc_conv3<NT, MT, ConvOutPadded>
         <<<(unsigned)((g.npos + tile - 1) / tile), rf_tc::kThreads, smem, c->stream>>>(
-            map, c->wc[li], g, ep, c->d_status, c->test_first_wait_polls);
+            c->wc[li], g, ep, c->d_status, c->test_first_wait_polls);
     c->launches++;
     CN(cudaGetLastError());
     return RF_OK;
 }
-// The largest of 512, 256 and 128 positions per CTA with which every SM gets a CTA
-// and two fit on it.  Fewer, larger tiles load the weights and the two rows around a
-// tile less often (64 images of 160 x 90: 0.92 ms with 128, 0.72 with at most 256,
-// 0.71 with 512); with too few of them SMs idle (four images: 0.114 ms with at most
-// 256, 0.130 with 128, one image the same either way).
+// 256 positions per CTA where every SM gets one and two or more fit on it, otherwise
+// 128.  The larger tile loads the weights and the two rows around it half as often
+// (64 images of 160 x 90: 0.53 ms against 0.65, eight 0.133 and 0.143); with too few
+// of them SMs idle (one image: the same either way).
 template <int NT>
-rf_status conv3_direct(rf_cnn* c, int li, const CUtensorMap& map, int B, int H, int W, bf16* y,
-                       float* yf) {
+rf_status conv3_direct(rf_cnn* c, int li, ConvInput in, int B, int H, int W, bf16* y, float* yf) {
     const long long npos = (long long)B * (H + 2) * (W + 2);
-    auto fits = [&](int mt, size_t bytes) {
-        return npos >= 152ll * rf_tc::kTM * mt && bytes <= 113 * 1024;
-    };
-    if constexpr (NT <= 64) {
-        using S = rf_tc::ConvSmem<NT, 4>;
-        if (fits(4, S::bytes(S::nbox(W)))) return conv3_launch<NT, 4>(c, li, map, B, H, W, y, yf);
-    }
-    using S = rf_tc::ConvSmem<NT, 2>;
-    if (fits(2, S::bytes(S::nbox(W)))) return conv3_launch<NT, 2>(c, li, map, B, H, W, y, yf);
-    return conv3_launch<NT, 1>(c, li, map, B, H, W, y, yf);
+    if (npos >= 152ll * rf_tc::kTM * 2 && rf_tc::ConvSmem<NT, 2>::bytes(W + 2) <= 113 * 1024)
+        return conv3_launch<NT, 2>(c, li, in, B, H, W, y, yf);
+    return conv3_launch<NT, 1>(c, li, in, B, H, W, y, yf);
 }
 
 // inference: padded activations (laid out for this call's frame size, up to
@@ -786,30 +782,33 @@ rf_status forward_direct(rf_cnn* c, const float* input, int B, int H, int W) {
     if (H != c->pad_h || W != c->pad_w) {
         // a new frame size moves the borders: clear the buffers once (the
         // kernels never write a border position of the size they run at)
-        bf16* bufs[6] = {c->xp, c->a1p, c->a2p, c->a3p, c->catp, c->a4p};
         for (int k = 0; k < 6; k++)
-            CN(cudaMemsetAsync(bufs[k], 0, c->pad_elems[k] * 2, c->stream));
+            CN(cudaMemsetAsync(c->pad[k], 0, c->pad_elems[k] * 2, c->stream));
         c->pad_h = H;
         c->pad_w = W;
     }
-    k_pad_input<<<blocks_for((size_t)B * H * W * 2), 256, 0, c->stream>>>(input, B, H, W, c->xp);
+    const size_t plane = pad_plane(c, H, W), plane2 = pad_plane(c, H2, W2);
+    auto all = [](const bf16* x, const Layer& L) { return ConvInput{x, x, L.cin / 8}; };
+    k_pad_input<<<blocks_for((size_t)B * H * W * 2), 256, 0, c->stream>>>(input, B, H, W, plane,
+                                                                        c->xp);
     c->launches++;
-    rf_status rs = conv3_direct<32>(c, 0, c->map_x, B, H, W, c->a1p, nullptr);
+    rf_status rs = conv3_direct<32>(c, 0, all(c->xp, c1), B, H, W, c->a1p, nullptr);
     if (rs == RF_OK) {
         const int M = B * H2 * W2, K = 9 * c2.cin;
         rs = tc_gemm(c, M, c2.cout, K,
-                     TcConvInPadded{c->a1p, H, W, c2.cin, H2, W2, c2.stride},
+                     TcConvInPadded{c->a1p, H, W, c2.cin, H2, W2, c2.stride, (int)plane},
                      TcRows{c->wb + c2.woff, K},
-                     ConvOutToPadded{c->w + c2.boff, c->a2p, c2.cout, c2.relu, H2, W2});
+                     ConvOutToPadded{c->w + c2.boff, c->a2p, c2.relu, H2, W2, plane2});
     }
-    if (rs == RF_OK) rs = conv3_direct<96>(c, 2, c->map_a2, B, H2, W2, c->a3p, nullptr);
-    if (rs == RF_OK) rs = conv3_direct<16>(c, 3, c->map_a3, B, H2, W2, nullptr, c->o16);
+    if (rs == RF_OK) rs = conv3_direct<96>(c, 2, all(c->a2p, c3), B, H2, W2, c->a3p, nullptr);
+    if (rs == RF_OK)
+        rs = conv3_direct<16>(c, 3, all(c->a3p, c->layers[3]), B, H2, W2, nullptr, c->o16);
     if (rs != RF_OK) return rs;
-    k_concat_up_pad<<<blocks_for((size_t)B * H * W * ((c3.cout + c1.cout) / 8)), 256, 0,
-                      c->stream>>>(c->a3p, H2, W2, c3.cout, c->a1p, c1.cout, B, H, W, c->catp);
+    const dim3 up(blocks_for((size_t)B * H * W), c3.cout / 8);
+    k_up_pad<<<up, 256, 0, c->stream>>>(c->a3p, H2, W2, plane2, B, H, W, plane, c->upp);
     c->launches++;
-    rs = conv3_direct<64>(c, 4, c->map_cat, B, H, W, c->a4p, nullptr);
-    if (rs == RF_OK) rs = conv3_direct<16>(c, 5, c->map_a4, B, H, W, nullptr, c->o8);
+    rs = conv3_direct<64>(c, 4, ConvInput{c->upp, c->a1p, c3.cout / 8}, B, H, W, c->a4p, nullptr);
+    if (rs == RF_OK) rs = conv3_direct<16>(c, 5, all(c->a4p, c->layers[5]), B, H, W, nullptr, c->o8);
     if (rs != RF_OK) return rs;
     CN(cudaGetLastError());
     return RF_OK;
@@ -868,40 +867,12 @@ rf_status backward(rf_cnn* c, int B, int H, int W) {
     return RF_OK;
 }
 
-// cuTensorMapEncodeTiled through the runtime's driver entry point (no link
-// against libcuda): a 2D map over a padded buffer viewed as [positions][C]
-// BF16, boxes of 8 channels x kConvBox positions, zero fill outside
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*,
-                                  const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
-                                  const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-bool encode_positions_map(CUtensorMap* m, const bf16* base, int C, size_t npos) {
-    static EncodeTiledFn fn = nullptr;
-    if (!fn) {
-        void* p = nullptr;
-        cudaDriverEntryPointQueryResult q{};
-        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000,
-                                             cudaEnableDefault, &q) != cudaSuccess ||
-            q != cudaDriverEntryPointSuccess || !p)
-            return false;
-        fn = (EncodeTiledFn)p;
-    }
-    const cuuint64_t dims[2] = {(cuuint64_t)C, (cuuint64_t)npos};
-    const cuuint64_t strides[1] = {(cuuint64_t)C * 2};
-    const cuuint32_t box[2] = {8, (cuuint32_t)rf_tc::kConvBox};
-    const cuuint32_t es[2] = {1, 1};
-    return fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (void*)base, dims, strides, box, es,
-              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-              CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
 // whether the direct kernel's shared memory fits rows of width W
 bool direct_fits(int W) {
     const size_t lim = 227 * 1024;
-    auto bytes = [&](auto smem) { return smem.bytes(smem.nbox(W)); };
-    return bytes(rf_tc::ConvSmem<32, 1>{}) <= lim && bytes(rf_tc::ConvSmem<64, 1>{}) <= lim &&
-           bytes(rf_tc::ConvSmem<96, 1>{}) <= lim;
+    return W + 2 < rf_tc::kConvMargin / 2 && rf_tc::ConvSmem<32, 1>::bytes(W + 2) <= lim &&
+           rf_tc::ConvSmem<64, 1>::bytes(W + 2) <= lim &&
+           rf_tc::ConvSmem<96, 1>::bytes(W + 2) <= lim;
 }
 
 }  // namespace rf_cnn_impl
@@ -972,28 +943,21 @@ rf_status rf_cnn_create(int max_batch, int height, int width, unsigned long long
     const size_t PP = (size_t)(height + 2) * (width + 2);
     const size_t PP2 = (size_t)((height + 1) / 2 + 2) * ((width + 1) / 2 + 2);
     if (c->direct) {
-        alloc(&c->xp, B * PP * 16 * 2); alloc(&c->a1p, B * PP * 32 * 2);
-        alloc(&c->a2p, B * PP2 * 96 * 2); alloc(&c->a3p, B * PP2 * 96 * 2);
-        alloc(&c->catp, B * PP * 128 * 2); alloc(&c->a4p, B * PP * 64 * 2);
+        const size_t elems[6] = {B * PP * 16, B * PP * 32, B * PP2 * 96,
+                                 B * PP2 * 96, B * PP * 96, B * PP * 64};
+        bf16** first[6] = {&c->xp, &c->a1p, &c->a2p, &c->a3p, &c->upp, &c->a4p};
+        for (int k = 0; k < 6; k++) {
+            // cleared before the first call (forward_direct, per frame size)
+            c->pad_elems[k] = elems[k] + 2 * rf_tc::kConvMargin * 8;
+            alloc(&c->pad[k], c->pad_elems[k] * 2);
+            *first[k] = c->pad[k] + rf_tc::kConvMargin * 8;
+        }
         const int nts[6] = {32, 0, 96, 16, 64, 16};  // c2 (stride 2) keeps the GEMM
         for (int li = 0; li < 6; li++)
             if (nts[li]) {
                 c->nt[li] = nts[li];
                 alloc(&c->wc[li], (size_t)(c->layers[li].cin / 16) * 9 * nts[li] * 16 * 2);
             }
-        // cleared before the first call (forward_direct, per frame size)
-        const size_t elems[6] = {B * PP * 16, B * PP * 32, B * PP2 * 96,
-                                 B * PP2 * 96, B * PP * 128, B * PP * 64};
-        for (int k = 0; k < 6; k++) c->pad_elems[k] = elems[k];
-        if (e == cudaSuccess &&
-            !(encode_positions_map(&c->map_x, c->xp, 16, B * PP) &&
-              encode_positions_map(&c->map_a2, c->a2p, 96, B * PP2) &&
-              encode_positions_map(&c->map_a3, c->a3p, 96, B * PP2) &&
-              encode_positions_map(&c->map_cat, c->catp, 128, B * PP) &&
-              encode_positions_map(&c->map_a4, c->a4p, 64, B * PP))) {
-            rf_cnn_destroy(c);
-            return cfail(RF_ERR_CUDA, "rf_cnn_create: tensor map encoding failed");
-        }
     }
     if (e == cudaSuccess) e = cudaMemcpy(c->w, hw.data(), off * 4, cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemset(c->m, 0, off * 4);
@@ -1028,8 +992,8 @@ rf_status rf_cnn_destroy(rf_cnn* c) {
                     (void*)c->a1, (void*)c->a2, (void*)c->a3, (void*)c->cat, (void*)c->a4,
                     (void*)c->o16, (void*)c->o8, (void*)c->g_o16, (void*)c->g_o8, (void*)c->g_a4,
                     (void*)c->g_cat, (void*)c->g_a3, (void*)c->g_a2, (void*)c->g_a1, (void*)c->gb,
-                    (void*)c->part, (void*)c->d_loss, (void*)c->xp, (void*)c->a1p,
-                    (void*)c->a2p, (void*)c->a3p, (void*)c->catp, (void*)c->a4p})
+                    (void*)c->part, (void*)c->d_loss, (void*)c->pad[0], (void*)c->pad[1],
+                    (void*)c->pad[2], (void*)c->pad[3], (void*)c->pad[4], (void*)c->pad[5]})
         if (p) cudaFree(p);
     for (bf16* p : c->wc)
         if (p) cudaFree(p);

@@ -36,7 +36,6 @@
 
 #include <cstdint>
 
-#include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -146,6 +145,19 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8]) {
         : "memory");
 #pragma unroll
     for (int i = 0; i < 8; i++) v[i] = __uint_as_float(r[i]);
+}
+
+// 16 consecutive columns
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
+    uint32_t r[16];
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n"
+        "tcgen05.wait::ld.sync.aligned;\n"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr)
+        : "memory");
+#pragma unroll
+    for (int i = 0; i < 16; i++) v[i] = __uint_as_float(r[i]);
 }
 
 // An operand of k_tc_gemm hands out, in units of 16 bytes (8 elements) from base():
@@ -322,11 +334,12 @@ __global__ void __launch_bounds__(kThreads) k_tc_gemm(int M, int N, int K, LA la
     } else if (nchunks > 0) {
         const int m = m0 + warp * 32 + lane;
         const uint32_t lane_addr = tmem + ((uint32_t)(warp * 32) << 16);
-#pragma unroll 1
-        for (int j = 0; j < NT; j += 8) {
-            float v[8];
-            tmem_ld8(lane_addr + (uint32_t)j, v);
-            if (m < M && n0 + j < N) ep(m, n0 + j, v);
+#pragma unroll 2
+        for (int j = 0; j < NT; j += 16) {
+            float v[16];
+            tmem_ld16(lane_addr + (uint32_t)j, v);
+            if (m < M && n0 + j < N) ep(m, n0 + j, reinterpret_cast<const float(&)[8]>(v[0]));
+            if (m < M && n0 + j + 8 < N) ep(m, n0 + j + 8, reinterpret_cast<const float(&)[8]>(v[8]));
         }
     }
     tc_fence_before();
@@ -513,47 +526,47 @@ __global__ void __launch_bounds__(kThreads) k_tc_wgrad(int M, int N, int K, int 
 // ---------------------------------------------------------------------------
 // Direct 3x3 convolution (stride 1, padding 1) on padded activations
 // ---------------------------------------------------------------------------
-// Activations are NHWC with a one-pixel zero border: position
-// q = (b (H + 2) + y) (W + 2) + x of a [B][H + 2][W + 2][C] buffer.  For
+// Activations have a one-pixel zero border and are planar by groups of 8
+// channels: a plane holds position q = (b (H + 2) + y) (W + 2) + x of
+// [B][H + 2][W + 2], 16 bytes each, for channels 8 g .. 8 g + 7.  For
 // output position q, tap (dy, dx) reads input position
 // q + (dy - 1)(W + 2) + (dx - 1), so 128 consecutive output positions read
 // 128 consecutive input positions for every tap: each tap is one MMA whose
 // A operand is a shifted view of one staged slab, and no im2col copy exists.
 // A CTA computes positions [q0, q0 + 128 MT) (border positions too; their
 // outputs are not stored, so borders stay zero).  Per stage of 16 input
-// channels it stages, by TMA, the slab of input positions
-// [q0 - (W + 3), q0 + 128 MT + (W + 3)) as two planes of 8 channels (16 bytes
-// per position: the canonical no-swizzle K-major layout, core matrices of 8
-// positions, the two K halves one plane apart), and by a bulk copy the
-// stage's weights for all 9 taps in the same layout (host-prepared), then
-// one thread issues the 9 MT MMAs (M = 128, N = NT, K = 16) into the TMEM
-// accumulators.  kStages ring slots: loads of the next stages run while
-// a stage's MMAs do.  Out-of-range slab positions (before the first image,
-// past the buffer) are filled with zeros by the TMA unit and only reach
-// border outputs.
-constexpr int kConvBox = 128;  // positions per TMA box (2 KB per 8-channel plane)
+// channels it stages the slab of input positions
+// [q0 - (W + 3), q0 + 128 MT + (W + 3)) of two planes (the canonical no-swizzle
+// K-major layout: core matrices of 8 positions, the two K halves one plane
+// apart) and the stage's weights for all 9 taps in the same layout (prepared
+// on the device), each by one bulk copy of contiguous memory, then one thread
+// issues the 9 MT MMAs (M = 128, N = NT, K = 16) into the TMEM accumulators.
+// kStages ring slots: loads of the next stages run while a stage's MMAs do.
+// Slab positions before the first image and past the last only reach border
+// outputs; the buffers have kConvMargin positions before and after their planes
+// for them.
+//
+// What it waits for is its own prologue and epilogue, so three CTAs of 256 positions
+// fit on an SM rather than two of 512.  64 images of 160 x 90 through the network:
+// as [position][C], whose slabs came by 2D TMA boxes with rows of 16 bytes, 0.70
+// ms with at most 512 positions per CTA; planar 0.59, with the epilogue by 16
+// columns 0.55, with at most 256 positions 0.53, with 128 0.65.
+constexpr int kConvMargin = 4096;
 
 struct ConvGeom {
     int Wp;      // padded row length W + 2
     int npos;    // padded positions of this call: B (H + 2)(W + 2)
-    int nbox;    // TMA boxes per plane: ceil((128 MT + 2 (W + 3)) / 128)
     int stages;  // input channels / 16
+    // planes 0 .. split - 1 at x, the others at x2; `plane` positions apart
+    const __nv_bfloat16 *x, *x2;
+    int split;
+    size_t plane;
 };
 
 __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)),
                  "r"(bytes)
                  : "memory");
-}
-
-// 2D tile of the tensor map at (c0 = channel, c1 = position) into shared memory
-__device__ __forceinline__ void tma_load_2d(void* dst, const void* map, int c0, int c1,
-                                            uint64_t* bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-        " [%0], [%1, {%2, %3}], [%4];" ::"r"(smem_u32(dst)),
-        "l"(map), "r"(c0), "r"(c1), "r"(smem_u32(bar))
-        : "memory");
 }
 
 // contiguous bytes (16-byte aligned, a multiple of 16) into shared memory
@@ -573,30 +586,27 @@ struct ConvSmem {
     static constexpr uint32_t kWBytes = 9u * NT * 32u;  // one stage's weights
     static constexpr uint32_t kN = NT * MT;
     static constexpr uint32_t kCols = kN <= 32 ? 32 : (kN <= 64 ? 64 : (kN <= 128 ? 128 : 256));
-    static int nbox(int W) { return (kTM * MT + 2 * (W + 3) + kConvBox - 1) / kConvBox; }
-    __host__ __device__ static uint32_t plane_bytes(int nbox) { return (uint32_t)nbox * kConvBox * 16u; }
-    __host__ __device__ static uint32_t stage_bytes(int nbox) { return 2u * plane_bytes(nbox) + kWBytes; }
-    static size_t bytes(int nbox) { return (size_t)kStages * stage_bytes(nbox) + 2048; }
+    __host__ __device__ static uint32_t plane_bytes(int Wp) { return (kTM * MT + 2u * (Wp + 1)) * 16u; }
+    __host__ __device__ static uint32_t stage_bytes(int Wp) { return 2u * plane_bytes(Wp) + kWBytes; }
+    static size_t bytes(int Wp) { return (size_t)kStages * stage_bytes(Wp) + 2048; }
 };
 
-// `xmap`: CUtensorMap over the padded input viewed as [positions][C] BF16
-// (box: 8 channels x kConvBox positions); `wc`: weights as
+// `wc`: weights as
 // [stage][tap][NT / 8][2][8][8] BF16.  `status` is set to 1 if a wait gave
 // up (the launch's outputs are then not written); `first_wait_polls` >= 0
 // caps the first slab wait of each CTA (a test hook, as for k_tc_gemm).
 // Every load issued is waited for (with the full limit) before the CTA
 // ends, and the last MMA commit before TMEM is released.
 template <int NT, int MT, class EP>
-__global__ void __launch_bounds__(kThreads) k_tc_conv3(const __grid_constant__ CUtensorMap xmap,
-                                                      const __nv_bfloat16* __restrict__ wc,
+__global__ void __launch_bounds__(kThreads) k_tc_conv3(const __nv_bfloat16* __restrict__ wc,
                                                       ConvGeom g, EP ep, int* status,
                                                       int first_wait_polls) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     using S = ConvSmem<NT, MT>;
     constexpr int kS = S::kStages;
     unsigned char* base = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    const uint32_t plane = S::plane_bytes(g.nbox);
-    const uint32_t stage_bytes = S::stage_bytes(g.nbox);
+    const uint32_t plane = S::plane_bytes(g.Wp);
+    const uint32_t stage_bytes = S::stage_bytes(g.Wp);
     uint64_t* full = (uint64_t*)(base + kS * stage_bytes);
     uint64_t* empty = full + kS;
     uint32_t* tslot = (uint32_t*)(empty + kS);
@@ -630,10 +640,12 @@ __global__ void __launch_bounds__(kThreads) k_tc_conv3(const __grid_constant__ C
         const int sl = j % kS;
         unsigned char* st = base + sl * stage_bytes;
         mbar_expect_tx(&full[sl], stage_bytes);
-        for (int pl = 0; pl < 2; pl++)
-            for (int b = 0; b < g.nbox; b++)
-                tma_load_2d(st + pl * plane + b * (kConvBox * 16), &xmap, 16 * j + 8 * pl,
-                            q0 - halo + b * kConvBox, &full[sl]);
+        for (int pl = 0; pl < 2; pl++) {
+            const int c = 2 * j + pl;
+            const __nv_bfloat16* src = c < g.split ? g.x + c * g.plane * 8
+                                                   : g.x2 + (c - g.split) * g.plane * 8;
+            bulk_load(st + pl * plane, src + ((ptrdiff_t)q0 - halo) * 8, plane, &full[sl]);
+        }
         bulk_load(st + 2 * plane, wc + (size_t)j * 9 * NT * 16, S::kWBytes, &full[sl]);
         *produced = j + 1;
     };
@@ -696,10 +708,10 @@ __global__ void __launch_bounds__(kThreads) k_tc_conv3(const __grid_constant__ C
             const int q = q0 + i * kTM + warp * 32 + lane;
             const int p = ep.pos(q);  // < 0: a border position or past the call's positions
             const uint32_t lane_addr = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(i * NT);
-#pragma unroll 1
-            for (int c = 0; c < NT; c += 8) {
-                float v[8];
-                tmem_ld8(lane_addr + (uint32_t)c, v);
+#pragma unroll 2
+            for (int c = 0; c < NT; c += 16) {
+                float v[16];
+                tmem_ld16(lane_addr + (uint32_t)c, v);
                 if (p >= 0) ep.store(q, p, c, v);
             }
         }

@@ -1,5 +1,5 @@
-"""The warm-start network over a batch large enough for 256 and 512 positions per
-block against the same images one at a time (128 positions per block): each
+"""The warm-start network over a batch large enough for 256 positions per block
+against the same images one at a time (128 positions per block): each
 output is the same sum in the same order, so the bits are equal."""
 import numpy as np
 import pytest
