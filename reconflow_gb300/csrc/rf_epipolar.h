@@ -30,6 +30,12 @@ RF_HD inline double sampson2(const double* E, const double* a, const double* b) 
     return d > 0.0 ? r * r / d : (r == 0.0 ? 0.0 : INFINITY);
 }
 
+// Worker threads for the host loops below, kept while anyone holds them (one set
+// for the process, at most 15 threads; every pose handle holds them from creation
+// to destruction).  Calls without a holder start their own.
+void hold_workers();
+void release_workers();
+
 // Every five-point hypothesis (9 doubles each) of the seeded LMedS samples,
 // in sample order.
 std::vector<double> lmeds_hypotheses(const double* x0, const double* x1, int n, double conf,

@@ -38,6 +38,7 @@
 #include <cmath>
 #include <cstdint>
 #include <cstring>
+#include <exception>
 #include <string>
 #include <vector>
 
@@ -520,6 +521,7 @@ __global__ void __launch_bounds__(256) k_lmeds_median(const double* __restrict__
 using namespace rf_pose_impl;
 
 struct rf_pose {
+    bool holds_workers = false;
     rf_pose_params p{};
     int w = 0, h = 0, max_kp = 0, cand_cap = 0;
     cudaStream_t own = nullptr, stream = nullptr;
@@ -865,6 +867,11 @@ rf_status rf_pose_create(const rf_pose_params* p, int width, int height, rf_pose
         return pfail(RF_ERR_OOM, std::string("rf_pose_create: ") + cudaGetErrorString(e));
     }
     h->stream = h->own;
+    try {
+        rf_epi::hold_workers();
+        h->holds_workers = true;
+    } catch (const std::exception&) {  // no memory for them: solves start their own
+    }
     *out = h;
     return RF_OK;
 }
@@ -892,6 +899,7 @@ rf_status rf_pose_destroy(rf_pose* h) {
     cudaFree(h->d_hyp);
     cudaFree(h->d_med);
     if (h->own) cudaStreamDestroy(h->own);
+    if (h->holds_workers) rf_epi::release_workers();
     delete h;
     return RF_OK;
 }
