@@ -116,12 +116,9 @@ SOLVER = dict(method=14, lam=50.0, theta=0.33, tau=0.25, alpha_proj=60.0, lambda
               lambdams=100.0, fix_quirks=1)
 # algorithmic bytes per pixel per launch of the two inner-iteration kernels:
 # A reads u,v,duhat(2),p(4),uproj(2),sk(2),Ix,Iy,Iz,X,Y,Z = 18 floats, writes
-# duhat(2),uproj(2),X1,Y1,Z1 = 7; B reads duhat(2),p(4),X1(3),sk(2),u,v,uproj(2)
-# = 15, writes p(4),X,Y,Z,sk(2) = 9.
-ALG_BYTES = {"recon_a": 25 * 4, "recon_b": 24 * 4}
-# the batch's large levels (k_batch_a2 / k_batch_b2): A also updates and writes
-# sk (9 written), B reads duhat(2),p(4),X1(3) and writes p(4),X,Y,Z
-ALG_BYTES_BATCH = {"recon_a": 27 * 4, "recon_b": 16 * 4}
+# sk(2),duhat(2),uproj(2),X1,Y1,Z1 = 9; B reads duhat(2),p(4),X1(3) = 9, writes
+# p(4),X,Y,Z = 7.
+ALG_BYTES = {"recon_a": 27 * 4, "recon_b": 16 * 4}
 # compulsory bytes of one inner iteration per pixel (both kernels together)
 ITER_BYTES = 31 * 4
 L2_FLUSH_BYTES = 512 << 20
@@ -1825,7 +1822,7 @@ def roofline_of(ms, px, batched=False):
     """Roofline entry of the dominant level-0 kernel from per-launch times
     (`px` pixels per launch; `batched`: the batched solver's kernels)."""
     names = ["recon_a", "recon_b"]
-    alg = ALG_BYTES_BATCH if batched else ALG_BYTES
+    alg = ALG_BYTES
     dom = 0 if ms[0] >= ms[1] else 1
     achieved = alg[names[dom]] * px / (ms[dom] * 1e-3) / 1e9
     peak, peak_kind = load_peaks()
@@ -1840,7 +1837,7 @@ def roofline_of(ms, px, batched=False):
         # with the pixel count: one pass over every field per launch)
         traffic = None if per is None else per * px / tr["pixels"]
     return {"bound": "hbm", "kernel": ("k_batch_a2" if dom == 0 else "k_batch_b2")
-            if batched else ("k_recon_a" if dom == 0 else "k_recon_b"),
+            if batched else ("k_recon_a1" if dom == 0 else "k_recon_b1"),
             "achieved": achieved, "peak": peak,
             "peak_kind": peak_kind, "unit": "GB/s", "frac": achieved / peak, "traffic": traffic,
             "alg_bytes_per_launch": alg[names[dom]] * px,
