@@ -196,16 +196,6 @@ __global__ void __launch_bounds__(BX* BY) k_warp_deriv(const float* __restrict__
 #ifndef RF_MINB_B
 #define RF_MINB_B 4  // 64 registers: 4 blocks per SM (fewer registers spill; measured slower)
 #endif
-// Programmatic dependent launch: a kernel launched with the programmatic
-// stream-serialization attribute may start while its predecessor drains;
-// griddepcontrol.wait blocks until the predecessor has completed and its
-// writes are visible, and launch_dependents lets the successor be scheduled.
-// Both are no-ops for a normal launch.
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_release() {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
-
 template <int PRIOR>
 __global__ void __launch_bounds__(BX* BY, RF_MINB_A) k_recon_a(ReconFields f, const LevelConsts* __restrict__ lcp,
                                                     Weights wt, LevelDims d, int first,
@@ -717,7 +707,7 @@ bool use_pdl() {
 
 // Launch with the programmatic stream-serialization attribute (see pdl_wait).
 template <typename... KArgs, typename... Args>
-int launch_pdl(void (*kern)(KArgs...), dim3 g, dim3 b, cudaStream_t st, Args... args) {
+int launch_pdl(bool pdl, void (*kern)(KArgs...), dim3 g, dim3 b, cudaStream_t st, Args... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = g;
     cfg.blockDim = b;
@@ -725,7 +715,7 @@ int launch_pdl(void (*kern)(KArgs...), dim3 g, dim3 b, cudaStream_t st, Args... 
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = use_pdl() ? 1 : 0;
+    attr[0].val.programmaticStreamSerializationAllowed = pdl ? 1 : 0;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, args...);
@@ -737,15 +727,15 @@ int launch_recon_a(const ReconFields& f, const LevelConsts* lc, const Weights& w
                    bool first, bool uc_from_buffer, int prior, cudaStream_t st, dim3 b) {
     dim3 g((d.w + b.x - 1) / b.x, (d.h + b.y - 1) / b.y);
     int fi = first ? 1 : 0, ub = uc_from_buffer ? 1 : 0;
-    if (prior == 1) return launch_pdl(k_recon_a<1>, g, b, st, f, lc, wt, d, fi, ub);
-    if (prior == 2) return launch_pdl(k_recon_a<2>, g, b, st, f, lc, wt, d, fi, ub);
-    return launch_pdl(k_recon_a<0>, g, b, st, f, lc, wt, d, fi, ub);
+    if (prior == 1) return launch_pdl(use_pdl(), k_recon_a<1>, g, b, st, f, lc, wt, d, fi, ub);
+    if (prior == 2) return launch_pdl(use_pdl(), k_recon_a<2>, g, b, st, f, lc, wt, d, fi, ub);
+    return launch_pdl(use_pdl(), k_recon_a<0>, g, b, st, f, lc, wt, d, fi, ub);
 }
 
 int launch_recon_b(const ReconFields& f, const Weights& wt, LevelDims d, bool first,
                    cudaStream_t st, dim3 b) {
     dim3 g((d.w + b.x - 1) / b.x, (d.h + b.y - 1) / b.y);
-    return launch_pdl(k_recon_b, g, b, st, f, wt, d, first ? 1 : 0);
+    return launch_pdl(use_pdl(), k_recon_b, g, b, st, f, wt, d, first ? 1 : 0);
 }
 
 bool pair_weights(const Weights& wt) {
@@ -820,10 +810,10 @@ int recon_tiles(const ReconFields& f, const ReconState& b, const LevelConsts* lc
                   : prior == 2 ? k_recon_tile<2, ROWS, K>
                                : k_recon_tile<0, ROWS, K>;
     for (int i = 0; i < launches; i++) {
-        kernel<<<g, T::THREADS, 0, st>>>(f, i & 1 ? b : a, i & 1 ? a : b, lc, wt, d,
-                                         each + (i < more ? 1 : 0), i == 0, i + 1 == launches,
-                                         i == 0 && uc_from_buffer);
-        if (check_launch() != 0) return -1;
+        if (launch_pdl(i > 0, kernel, g, dim3(T::THREADS), st, f, i & 1 ? b : a, i & 1 ? a : b, lc,
+                       wt, d, each + (i < more ? 1 : 0), (int)(i == 0), (int)(i + 1 == launches),
+                       (int)(i == 0 && uc_from_buffer)) != 0)
+            return -1;
     }
     return launches;
 }
@@ -955,10 +945,10 @@ int plain_tiles(PlainState a, PlainState b, const float* Ix, const float* Iy, co
     int launches = 0;
     for (int done = 0; done < n_iters; done += K, launches++) {
         const int n = n_iters - done < K ? n_iters - done : K;
-        k_plain_tile<R, WARPS, K, SKIP><<<g, T::THREADS, 0, st>>>(
-            launches & 1 ? a : b, launches & 1 ? b : a, Ix, Iy, Iz, wt, d, n, done == 0,
-            done + n == n_iters);
-        if (check_launch() != 0) return -1;
+        if (launch_pdl(done > 0, k_plain_tile<R, WARPS, K, SKIP>, g, dim3(T::THREADS), st,
+                       launches & 1 ? a : b, launches & 1 ? b : a, Ix, Iy, Iz, PlainWeights(wt), d,
+                       n, (int)(done == 0), (int)(done + n == n_iters)) != 0)
+            return -1;
     }
     *in_b = launches & 1 ? 0 : 1;
     return launches;

@@ -30,6 +30,16 @@ __device__ __forceinline__ float deriv5(float m2, float m1, float p1, float p2) 
     return t;
 }
 
+// Programmatic dependent launch: a kernel launched with the programmatic
+// stream-serialization attribute may start while its predecessor drains;
+// griddepcontrol.wait blocks until the predecessor has completed and its
+// writes are visible, and launch_dependents lets the successor be scheduled.
+// Both are no-ops for a normal launch.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_release() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // What part A reads at a pixel; its results replace the values it updates.
 struct APoint {
     float u, v, dix, diy, dit, uproj, vproj, sku, skv, duhat, dvhat;

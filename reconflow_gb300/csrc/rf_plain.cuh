@@ -137,25 +137,32 @@ __global__ void __launch_bounds__(32 * WARPS)
 #pragma unroll
     for (int r = 0; r < R; r++) {
         const int y = y0 + r;
-        c[r].di = du[r] = dup2(0.0f);
+        c[r].di = dup2(0.0f);
         c[r].dit = 0.0f;
-        n1[r] = n2[r] = dup2(-0.0f);
         if (in_x && y >= 0 && y < d.h) {
             const int pos = x + y * d.s;
             c[r].di = f2{Ix[pos], Iy[pos]};
             c[r].dit = Iz[pos];
-            if (!first) {
-                du[r] = f2{in.du[pos], in.dv[pos]};
-                n1[r] = f2{in.pu1[pos], in.pv1[pos]};
-                n2[r] = f2{in.pu2[pos], in.pv2[pos]};
-            }
         }
-    }
-#pragma unroll
-    for (int r = 0; r < R; r++) {
         const float m = c[r].di.x * c[r].di.x + c[r].di.y * c[r].di.y;
         c[r].magi = m;
         c[r].nr = m >= 0x1p-50f && m <= 0x1p120f ? neg_recip(m) : __uint_as_float(0x7FC00000u);
+    }
+    // the derivatives do not change between the launches of a warp: they are read while
+    // the launch before drains; then the next one may start likewise
+    pdl_wait();
+    pdl_release();
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+        const int y = y0 + r;
+        du[r] = dup2(0.0f);
+        n1[r] = n2[r] = dup2(-0.0f);
+        if (!first && in_x && y >= 0 && y < d.h) {
+            const int pos = x + y * d.s;
+            du[r] = f2{in.du[pos], in.dv[pos]};
+            n1[r] = f2{in.pu1[pos], in.pv1[pos]};
+            n2[r] = f2{in.pu2[pos], in.pv2[pos]};
+        }
     }
     s_n2[warp][lane] = n2[R - 1];
     __syncthreads();

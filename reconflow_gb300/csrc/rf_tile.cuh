@@ -20,7 +20,9 @@
 // The arithmetic is that of the one-pixel half-steps (rf_pair.cuh): same bits.
 // Bound by a block's instruction issue (about 1000 per pixel and iteration):
 // 3 to 3.5 us per iteration, 5.2 to 6 by two launches.  Plain 640x480 pair 6.05 ->
-// 4.79 ms, 1280x720 35.2 -> 31.3, 451x333 with a prior 4.55 -> 3.44.
+// 4.79 ms, 1280x720 35.2 -> 31.3, 451x333 with a prior 4.55 -> 3.44.  With the next
+// launch's blocks coming in while one runs (programmatic launches) 640x480 4.72 -> 4.58
+// and the prior's 3.32 -> 3.22: there a launch has SMs to spare.
 #pragma once
 
 #include "rf_pair.cuh"
@@ -122,6 +124,17 @@ __global__ void __launch_bounds__(kTileW* ROWS)
         dix = RF_AT(f, Ix, pos);
         diy = RF_AT(f, Iy, pos);
         dit = RF_AT(f, Iz, pos);
+        if (PRIOR != 0) {
+            ufn = RF_AT(f, ufn, pos);
+            vfn = RF_AT(f, vfn, pos);
+            if (PRIOR == 2) mk = RF_AT(f, mask, pos);
+        }
+    }
+    // what comes before this does not change between the launches of a warp, so it is
+    // read while the launch before drains; then the next one may start likewise
+    pdl_wait();
+    pdl_release();
+    if (pixel) {
         uproj = RF_PT(in.uproj, pos, f.extent);
         vproj = RF_PT(in.vproj, pos, f.extent);
         sku = RF_PT(in.sku, pos, f.extent);
@@ -129,11 +142,6 @@ __global__ void __launch_bounds__(kTileW* ROWS)
         X = RF_PT(in.X, pos, f.extent);
         Y = RF_PT(in.Y, pos, f.extent);
         Z = RF_PT(in.Z, pos, f.extent);
-        if (PRIOR != 0) {
-            ufn = RF_AT(f, ufn, pos);
-            vfn = RF_AT(f, vfn, pos);
-            if (PRIOR == 2) mk = RF_AT(f, mask, pos);
-        }
         if (!first_launch) {
             duhat = RF_PT(in.duhat, pos, f.extent);
             dvhat = RF_PT(in.dvhat, pos, f.extent);
