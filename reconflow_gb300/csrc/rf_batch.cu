@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(kMaxTile) k_batch_rows2(BatchCtx ctx, int leve
 // A is bound by instruction issue and the latency of its first loads (461
 // warp instructions per 32 pixels at 54% issue, 20 warps per SM; DRAM at 60%),
 // B by the min / max pipe and its copies (346 at 69%): per launch of 64 720p
-// pairs (58 982 400 pixels) 1.28 and 0.79 ms against 1.40 and 1.11 ms for the
+// pairs (58 982 400 pixels) 1.15 and 0.77 ms against 1.40 and 1.11 ms for the
 // one-pixel kernels, 108 and 64 bytes per pixel.  Measured on 32 learned 720p
 // pairs (whole call, one-pixel kernels 24.8 ms): 5 / 10 blocks per SM of 4 rows
 // 20.4 ms; 8 rows 23.5 (waits at the block's barrier), 2 rows 21.3; A at 4
