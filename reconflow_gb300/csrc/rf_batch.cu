@@ -117,6 +117,7 @@ __global__ void __launch_bounds__(kMaxTile) k_batch(BatchCtx ctx, int level,
     const TileEntry t = ctx.tiles[blockIdx.x];
     const LevelDims d = ctx.pairs[t.pair].dims[level];
     const int ix = t.x0 + (int)threadIdx.x, iy = t.y0 + (int)threadIdx.y;
+    pdl_wait();
     if (ix >= d.w || iy >= d.h) return;
     op(ctx, t, level, d, ix, iy);
 }
@@ -173,6 +174,7 @@ __global__ void __launch_bounds__(kPairThreads, kPairBlocksA)
     const LevelDims d = ctx.pairs[t.pair].dims[level];
     const LevelConsts* lc = ctx.consts + t.pair * ctx.L + level;
     pair_consts(lc, wt, sc, threadIdx.x, kPairThreads);
+    pdl_wait();
     if (!first) prefetch_rows(ctx, level, f);
     const int x = t.x0 + 2 * (int)(threadIdx.x & 31), y = t.y0 + (int)(threadIdx.x >> 5);
     recon_a_pair<0>(f, lc, sc, wt, d, t.off, x, y, x < d.w && y < d.h, first != 0, ucb != 0);
@@ -184,6 +186,7 @@ __global__ void __launch_bounds__(kPairThreads, kPairBlocksB)
                const __grid_constant__ Weights wt, int first) {
     __shared__ __align__(16) float sm[StageB::FLOATS];
     const TileEntry t = ctx.tiles[blockIdx.x];
+    pdl_wait();
     recon_b_tile<LAST>(f, wt, sm, ctx.pairs[t.pair].dims[level], t.off, t.x0, t.y0,
                                   first != 0);
 }
@@ -733,12 +736,14 @@ ReconFields fields_of(rf_batch* b, const ReconIdx& r) {
     return f;
 }
 
+// `early`: the launch may start while the one before drains (the table and the level
+// constants, all it reads before, are written before a warp's first launch)
 template <class Op>
-int launch_op(rf_batch* b, int level, const Op& op) {
+int launch_op(rf_batch* b, int level, const Op& op, bool early = false) {
     int tiles = b->prefix[level * (b->n + 1) + b->n];
     if (tiles <= 0) return 0;
     const dim3 block(b->tile_w[level], b->tile_h[level]);
-    k_batch<Op><<<tiles, block, 0, b->stream>>>(ctx_of(b, level), level, op);
+    launch_early(early, k_batch<Op>, dim3(tiles), block, b->stream, ctx_of(b, level), level, op);
     b->enq++;
     return rf::launch_status();
 }
@@ -747,11 +752,12 @@ int launch_op(rf_batch* b, int level, const Op& op) {
 // level's pixel pairs or pixels; `last`: the warp's last B
 int launch_half_a(rf_batch* b, int level, const ReconFields& f, const Weights& wt, bool first,
                   bool ucb) {
-    if (b->pair_blocks[level] == 0) return launch_op(b, level, OpReconA1{f, wt, first, ucb});
+    if (b->pair_blocks[level] == 0) return launch_op(b, level, OpReconA1{f, wt, first, ucb}, !first);
     BatchCtx c = ctx_of(b, level);
     c.tiles = b->d_tiles + b->pair_start[level];
     c.prefetch = b->prefetch / 16 * kPairBlocksA / 2;  // half a wave of these blocks
-    k_batch_a2<<<b->pair_blocks[level], kPairThreads, 0, b->stream>>>(c, level, f, wt, first, ucb);
+    launch_early(!first, k_batch_a2, dim3(b->pair_blocks[level]), dim3(kPairThreads), b->stream, c,
+                 level, f, wt, (int)first, (int)ucb);
     b->enq++;
     return rf::launch_status();
 }
@@ -759,14 +765,12 @@ int launch_half_a(rf_batch* b, int level, const ReconFields& f, const Weights& w
 int launch_half_b(rf_batch* b, int level, const ReconFields& f, const Weights& wt, bool first,
                   bool last) {
     if (b->pair_blocks[level] == 0)
-        return last ? launch_op(b, level, OpReconB1<true>{f, wt, first})
-                    : launch_op(b, level, OpReconB1<false>{f, wt, first});
+        return last ? launch_op(b, level, OpReconB1<true>{f, wt, first}, true)
+                    : launch_op(b, level, OpReconB1<false>{f, wt, first}, true);
     BatchCtx c = ctx_of(b, level);
     c.tiles = b->d_tiles + b->pair_start[level];
-    if (last)
-        k_batch_b2<true><<<b->pair_blocks[level], kPairThreads, 0, b->stream>>>(c, level, f, wt, first);
-    else
-        k_batch_b2<false><<<b->pair_blocks[level], kPairThreads, 0, b->stream>>>(c, level, f, wt, first);
+    launch_early(true, last ? k_batch_b2<true> : k_batch_b2<false>, dim3(b->pair_blocks[level]),
+                 dim3(kPairThreads), b->stream, c, level, f, wt, (int)first);
     b->enq++;
     return rf::launch_status();
 }

@@ -220,13 +220,12 @@ __global__ void __launch_bounds__(BX* BY, RF_MINB_B) k_recon_b(ReconFields f, We
 
 // The half-steps of rf_pair.cuh, one pixel per thread: 632 and 371 warp
 // instructions per 32 pixels against 725 and 385 of k_recon_a / k_recon_b (a
-// plain 640x480 solve 6.49 -> 5.94 ms, 720p 37.0 -> 35.1).  Programmatic
-// dependent launches made them slower (6.17, 36.3): the launch is not what a
-// small level waits for, its longest thread is.
+// plain 640x480 solve 6.49 -> 5.94 ms, 720p 37.0 -> 35.1).
 template <int PRIOR>
 __global__ void __launch_bounds__(BX* BY)
     k_recon_a1(const __grid_constant__ ReconFields f, const LevelConsts* __restrict__ lcp,
                const __grid_constant__ Weights wt, LevelDims d, int first, int uc_from_buffer) {
+    pdl_wait();
     const int ix = blockIdx.x * blockDim.x + threadIdx.x;
     const int iy = blockIdx.y * blockDim.y + threadIdx.y;
     if (ix >= d.w || iy >= d.h) return;
@@ -237,6 +236,7 @@ template <bool LAST>
 __global__ void __launch_bounds__(BX* BY)
     k_recon_b1(const __grid_constant__ ReconFields f, const __grid_constant__ Weights wt,
                LevelDims d, int first) {
+    pdl_wait();
     const int ix = blockIdx.x * blockDim.x + threadIdx.x;
     const int iy = blockIdx.y * blockDim.y + threadIdx.y;
     if (ix >= d.w || iy >= d.h) return;
@@ -252,6 +252,7 @@ __global__ void __launch_bounds__(32 * kPairRows, 5)
     const int x = 2 * (int)(blockIdx.x * 32 + (threadIdx.x & 31));
     const int y = blockIdx.y * kPairRows + (threadIdx.x >> 5);
     pair_consts(lcp, wt, sc, threadIdx.x, 32 * kPairRows);
+    pdl_wait();
     recon_a_pair<PRIOR>(f, lcp, sc, wt, d, 0, x, y, x < d.w && y < d.h, first != 0,
                         uc_from_buffer != 0);
 }
@@ -261,6 +262,7 @@ __global__ void __launch_bounds__(32 * kPairRows, 10)
     k_recon_b2(const __grid_constant__ ReconFields f, const __grid_constant__ Weights wt,
                LevelDims d, int first) {
     __shared__ __align__(16) float sm[StageB::FLOATS];
+    pdl_wait();
     recon_b_tile<LAST>(f, wt, sm, d, 0, blockIdx.x * kPairW, blockIdx.y * kPairRows,
                                   first != 0);
 }
@@ -705,20 +707,9 @@ bool use_pdl() {
     return v == 1;
 }
 
-// Launch with the programmatic stream-serialization attribute (see pdl_wait).
 template <typename... KArgs, typename... Args>
-int launch_pdl(bool pdl, void (*kern)(KArgs...), dim3 g, dim3 b, cudaStream_t st, Args... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = g;
-    cfg.blockDim = b;
-    cfg.dynamicSmemBytes = 0;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = pdl ? 1 : 0;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, args...);
+int launch_pdl(bool early, void (*kern)(KArgs...), dim3 g, dim3 b, cudaStream_t st, Args... args) {
+    const cudaError_t e = launch_early(early, kern, g, b, st, args...);
     if (e != cudaSuccess) t_launch_error = e;
     return e == cudaSuccess ? 0 : 1;
 }
@@ -756,22 +747,22 @@ bool use_pairs(LevelDims d) {
 }
 }  // namespace
 
+// Every launch of a warp but its first starts while the one before drains (640x480
+// 4.58 -> 4.47 ms, 1280x720 30.8 -> 30.6, 451x333 with a prior 3.22 -> 3.10, one learned
+// 720p pair 1.37 -> 1.34; released from the blocks' start instead of their end, or with
+// A's fixed fields read before the wait: as fast).
 int launch_half_a(const ReconFields& f, const LevelConsts* lc, const Weights& wt, LevelDims d,
                   bool first, bool uc_from_buffer, int prior, cudaStream_t st, dim3 b) {
     const int fi = first ? 1 : 0, ub = uc_from_buffer ? 1 : 0;
-    if (use_pairs(d)) {
+    const bool pairs = use_pairs(d);
+    auto one = prior == 1 ? k_recon_a1<1> : prior == 2 ? k_recon_a1<2> : k_recon_a1<0>;
+    auto two = prior == 1 ? k_recon_a2<1> : prior == 2 ? k_recon_a2<2> : k_recon_a2<0>;
+    if (pairs) {
         const dim3 g((d.w + kPairW - 1) / kPairW, (d.h + kPairRows - 1) / kPairRows);
-        const int n = 32 * kPairRows;
-        if (prior == 1) k_recon_a2<1><<<g, n, 0, st>>>(f, lc, wt, d, fi, ub);
-        else if (prior == 2) k_recon_a2<2><<<g, n, 0, st>>>(f, lc, wt, d, fi, ub);
-        else k_recon_a2<0><<<g, n, 0, st>>>(f, lc, wt, d, fi, ub);
-    } else {
-        const dim3 g((d.w + b.x - 1) / b.x, (d.h + b.y - 1) / b.y);
-        if (prior == 1) k_recon_a1<1><<<g, b, 0, st>>>(f, lc, wt, d, fi, ub);
-        else if (prior == 2) k_recon_a1<2><<<g, b, 0, st>>>(f, lc, wt, d, fi, ub);
-        else k_recon_a1<0><<<g, b, 0, st>>>(f, lc, wt, d, fi, ub);
+        return launch_pdl(!first, two, g, dim3(32 * kPairRows), st, f, lc, wt, d, fi, ub);
     }
-    return check_launch();
+    const dim3 g((d.w + b.x - 1) / b.x, (d.h + b.y - 1) / b.y);
+    return launch_pdl(!first, one, g, b, st, f, lc, wt, d, fi, ub);
 }
 
 int launch_half_b(const ReconFields& f, const Weights& wt, LevelDims d, bool first, bool last,
@@ -779,14 +770,11 @@ int launch_half_b(const ReconFields& f, const Weights& wt, LevelDims d, bool fir
     const int fi = first ? 1 : 0;
     if (use_pairs(d)) {
         const dim3 g((d.w + kPairW - 1) / kPairW, (d.h + kPairRows - 1) / kPairRows);
-        if (last) k_recon_b2<true><<<g, 32 * kPairRows, 0, st>>>(f, wt, d, fi);
-        else k_recon_b2<false><<<g, 32 * kPairRows, 0, st>>>(f, wt, d, fi);
-    } else {
-        const dim3 g((d.w + b.x - 1) / b.x, (d.h + b.y - 1) / b.y);
-        if (last) k_recon_b1<true><<<g, b, 0, st>>>(f, wt, d, fi);
-        else k_recon_b1<false><<<g, b, 0, st>>>(f, wt, d, fi);
+        return launch_pdl(true, last ? k_recon_b2<true> : k_recon_b2<false>, g,
+                          dim3(32 * kPairRows), st, f, wt, d, fi);
     }
-    return check_launch();
+    const dim3 g((d.w + b.x - 1) / b.x, (d.h + b.y - 1) / b.y);
+    return launch_pdl(true, last ? k_recon_b1<true> : k_recon_b1<false>, g, b, st, f, wt, d, fi);
 }
 
 namespace {

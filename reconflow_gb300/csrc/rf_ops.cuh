@@ -40,6 +40,24 @@ __device__ __forceinline__ void pdl_release() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// Launch a kernel that calls pdl_wait before it reads what the launch before writes;
+// `early`: it may start while that one drains.
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_early(bool early, void (*kern)(KArgs...), dim3 g, dim3 b,
+                                cudaStream_t st, Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = g;
+    cfg.blockDim = b;
+    cfg.dynamicSmemBytes = 0;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = early ? 1 : 0;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, args...);
+}
+
 // What part A reads at a pixel; its results replace the values it updates.
 struct APoint {
     float u, v, dix, diy, dit, uproj, vproj, sku, skv, duhat, dvhat;
