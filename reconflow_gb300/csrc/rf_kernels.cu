@@ -143,6 +143,7 @@ struct UpscaleArgs {
 };
 
 __global__ void k_upscale_fields(UpscaleArgs a, LevelDims c, LevelDims f) {
+    pdl_wait();
     int ix = blockIdx.x * blockDim.x + threadIdx.x;
     int iy = blockIdx.y * blockDim.y + threadIdx.y;
     if (ix >= f.w || iy >= f.h) return;
@@ -176,14 +177,13 @@ __global__ void k_derivatives(const float* __restrict__ I0, const float* __restr
 }
 
 // the two fused (warp_deriv_tile): one BX x BY tile per block
-__global__ void __launch_bounds__(BX* BY) k_warp_deriv(const float* __restrict__ I0,
-                                                       const float* __restrict__ I1,
-                                                       const float* __restrict__ u,
-                                                       const float* __restrict__ v, LevelDims d,
-                                                       float* __restrict__ Ix,
-                                                       float* __restrict__ Iy,
-                                                       float* __restrict__ Iz) {
+// (u, v without __restrict__: what the launch before writes must not be read ahead of
+// the wait, as the compiler may with inputs it takes for constant)
+__global__ void __launch_bounds__(BX* BY) k_warp_deriv(const float* I0, const float* I1,
+                                                       const float* u, const float* v, LevelDims d,
+                                                       float* Ix, float* Iy, float* Iz) {
     __shared__ float sm[2 * (BX + 4) * (BY + 4)];
+    pdl_wait();
     warp_deriv_tile(I0, I1, u, v, d, blockIdx.x * BX, blockIdx.y * BY, BX, BY, sm, Ix, Iy, Iz);
 }
 
@@ -353,10 +353,11 @@ __device__ __noinline__ float median25_tile(const float* t, bool net) {
 
 template <bool ADD>
 __global__ void __launch_bounds__(kMedW* kMedH / 2)
-    k_median_tile(const float* __restrict__ in0, const float* __restrict__ in1, const float* add0,
-                  const float* add1, float* out0, float* out1, LevelDims d) {
+    k_median_tile(const float* in0, const float* in1, const float* add0, const float* add1,
+                  float* out0, float* out1, LevelDims d) {
     __shared__ float tile[(kMedH + 4) * kMedPitch];
-    const float* __restrict__ in = blockIdx.z ? in1 : in0;
+    pdl_wait();
+    const float* in = blockIdx.z ? in1 : in0;
     const float* add = blockIdx.z ? add1 : add0;
     float* out = blockIdx.z ? out1 : out0;
     const int x0 = blockIdx.x * kMedW, y0 = blockIdx.y * kMedH;
@@ -652,6 +653,13 @@ __global__ void k_energy_final_jobs(const EnergyJob* jobs) {
 // ---------------------------------------------------------------------------
 // Launchers
 // ---------------------------------------------------------------------------
+template <typename... KArgs, typename... Args>
+int launch_pdl(bool early, void (*kern)(KArgs...), dim3 g, dim3 b, cudaStream_t st, Args... args) {
+    const cudaError_t e = launch_early(early, kern, g, b, st, args...);
+    if (e != cudaSuccess) t_launch_error = e;
+    return e == cudaSuccess ? 0 : 1;
+}
+
 int launch_status() { return check_launch(); }
 
 cudaError_t last_launch_error() {
@@ -687,8 +695,8 @@ int launch_warp(const float* I1, const float* u, const float* v, LevelDims d, fl
 
 int launch_warp_deriv(const float* I0, const float* I1, const float* u, const float* v,
                       LevelDims d, float* Ix, float* Iy, float* Iz, cudaStream_t st) {
-    k_warp_deriv<<<grid_for(d.w, d.h), dim3(BX, BY), 0, st>>>(I0, I1, u, v, d, Ix, Iy, Iz);
-    return check_launch();
+    return launch_pdl(true, k_warp_deriv, grid_for(d.w, d.h), dim3(BX, BY), st, I0, I1, u, v, d, Ix,
+                      Iy, Iz);
 }
 
 int launch_derivatives(const float* I0, const float* I1w, LevelDims d, float* Ix, float* Iy,
@@ -705,13 +713,6 @@ bool use_pdl() {
         v = (e && e[0] == '1') ? 1 : 0;
     }
     return v == 1;
-}
-
-template <typename... KArgs, typename... Args>
-int launch_pdl(bool early, void (*kern)(KArgs...), dim3 g, dim3 b, cudaStream_t st, Args... args) {
-    const cudaError_t e = launch_early(early, kern, g, b, st, args...);
-    if (e != cudaSuccess) t_launch_error = e;
-    return e == cudaSuccess ? 0 : 1;
 }
 
 int launch_recon_a(const ReconFields& f, const LevelConsts* lc, const Weights& wt, LevelDims d,
@@ -978,15 +979,15 @@ int launch_plain_tv(const float* duhat, const float* dvhat, float* pu1, float* p
 int launch_median_add(const float* duhat, const float* dvhat, const float* u, const float* v,
                       float* ou, float* ov, LevelDims d, cudaStream_t st) {
     const dim3 g((d.w + kMedW - 1) / kMedW, (d.h + kMedH - 1) / kMedH, 2);
-    k_median_tile<true><<<g, kMedW * kMedH / 2, 0, st>>>(duhat, dvhat, u, v, ou, ov, d);
-    return check_launch();
+    return launch_pdl(true, k_median_tile<true>, g, dim3(kMedW * kMedH / 2), st, duhat, dvhat, u, v,
+                      ou, ov, d);
 }
 
 int launch_median5(const float* u, const float* v, float* ou, float* ov, LevelDims d,
                    cudaStream_t st) {
     const dim3 g((d.w + kMedW - 1) / kMedW, (d.h + kMedH - 1) / kMedH, 2);
-    k_median_tile<false><<<g, kMedW * kMedH / 2, 0, st>>>(u, v, u, v, ou, ov, d);
-    return check_launch();
+    return launch_pdl(true, k_median_tile<false>, g, dim3(kMedW * kMedH / 2), st, u, v, u, v, ou, ov,
+                      d);
 }
 
 int launch_median3d(const float* X, const float* Y, const float* Z, float* X1, float* Y1,
@@ -1011,8 +1012,8 @@ int launch_upscale_fields(int n, const float* const* src, float* const* dst, con
         a.dst[i] = dst[i];
         a.scale[i] = scales[i];
     }
-    k_upscale_fields<<<grid_for(fine.w, fine.h), dim3(BX, BY), 0, st>>>(a, coarse, fine);
-    return check_launch();
+    return launch_pdl(true, k_upscale_fields, grid_for(fine.w, fine.h), dim3(BX, BY), st, a, coarse,
+                      fine);
 }
 
 int launch_upscale(const float* src, LevelDims coarse, LevelDims fine, float scale, float* out,
