@@ -24,11 +24,12 @@
 #include <list>
 #include <memory>
 #include <mutex>
+#include <new>
 #include <system_error>
 #include <thread>
 #include <vector>
 
-#include <unistd.h>
+#include <pthread.h>
 
 #include "../../include/reconflow_gb300.h"
 #include "rf_epipolar.h"
@@ -170,8 +171,6 @@ int uniform_below(uint64_t& s, int n) {
     return (int)(v % (uint64_t)n);
 }
 
-// Least-median-of-squares essential matrix over n >= 5 normalized matches.
-// Returns false when no sample gave a model.
 // Threads that wait for loops to share.  Whoever runs a loop works on it too, so it
 // ends whether or not a worker is free, and several callers' loops run side by
 // side.  Starting 16 threads for each pose took longer than its 134 five-point
@@ -188,7 +187,7 @@ class Workers {
     static constexpr int kChunk = 2;
 
 public:
-    explicit Workers(int n) : pid_(getpid()) {
+    explicit Workers(int n) {
         threads_.reserve(n);
         try {
             for (int i = 0; i < n; i++) threads_.emplace_back([this] { work(); });
@@ -196,10 +195,6 @@ public:
         }
     }
     ~Workers() {
-        if (!here()) {  // a forked child has none of the threads
-            for (auto& t : threads_) t.detach();
-            return;
-        }
         {
             std::lock_guard<std::mutex> lock(mutex_);
             stop_ = true;
@@ -207,7 +202,6 @@ public:
         wake_.notify_all();
         for (auto& t : threads_) t.join();
     }
-    bool here() const { return getpid() == pid_; }
     void run(int n, void (*call)(void*, int), void* loop) {
         Job job;
         job.call = call;
@@ -251,7 +245,6 @@ private:
         }
     }
 
-    const pid_t pid_;
     std::mutex mutex_;
     std::condition_variable wake_, done_;
     std::list<Job*> jobs_;
@@ -266,14 +259,28 @@ std::shared_ptr<Workers>& workers() {  // (never destroyed: no thread outlives i
     return *w;
 }
 
+// A forked child has none of the threads, and destroying what they wait on would wait
+// for them: it forgets the set (never destroyed there) and starts its own when asked.
+// No fork falls into a change of the set.
+void keep_across_forks() {
+    static const int registered = pthread_atfork(
+        [] { g_workers_mutex.lock(); }, [] { g_workers_mutex.unlock(); },
+        [] {
+            ::new (static_cast<void*>(&workers())) std::shared_ptr<Workers>;
+            g_workers_mutex.unlock();
+        });
+    (void)registered;
+}
+
 int host_threads() {
     const unsigned hw = std::thread::hardware_concurrency();
     return std::min((int)(hw ? hw : 1), 16);
 }
 
 void hold_workers() {
+    keep_across_forks();
     std::lock_guard<std::mutex> lock(g_workers_mutex);
-    if (g_holders == 0) workers() = std::make_shared<Workers>(host_threads() - 1);
+    if (!workers()) workers() = std::make_shared<Workers>(host_threads() - 1);
     g_holders++;
 }
 
@@ -296,7 +303,7 @@ void parallel_for(int n, F&& f) {
         std::lock_guard<std::mutex> lock(g_workers_mutex);
         w = workers();
     }
-    if (w && w->here()) {
+    if (w) {
         w->run(n, [](void* loop, int i) { (*static_cast<std::remove_reference_t<F>*>(loop))(i); },
                &f);
         return;
@@ -404,6 +411,7 @@ bool lmeds_select(const std::vector<double>& hyp, const std::vector<double>& med
 }
 
 // Least-median-of-squares essential matrix over n >= 5 normalized matches.
+// Returns false when no sample gave a model.
 bool lmeds(const double* x0, const double* x1, int n, double conf, uint64_t seed, double* E,
            unsigned char* mask) {
     const std::vector<double> hyp = lmeds_hypotheses(x0, x1, n, conf, seed);
