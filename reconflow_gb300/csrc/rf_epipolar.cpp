@@ -21,11 +21,11 @@
 #include <cstring>
 #include <atomic>
 #include <condition_variable>
+#include <exception>
 #include <list>
 #include <memory>
 #include <mutex>
 #include <new>
-#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -182,7 +182,8 @@ class Workers {
         void* loop;
         int n;
         std::atomic<int> next{0};
-        int users = 0;  // workers inside, under mutex_
+        int users = 0;             // workers inside, under mutex_
+        std::exception_ptr error;  // the first of the loop's, under mutex_
     };
     static constexpr int kChunk = 2;
 
@@ -191,7 +192,7 @@ public:
         threads_.reserve(n);
         try {
             for (int i = 0; i < n; i++) threads_.emplace_back([this] { work(); });
-        } catch (const std::system_error&) {  // fewer threads will do
+        } catch (const std::exception&) {  // fewer threads will do
         }
     }
     ~Workers() {
@@ -216,14 +217,22 @@ public:
         std::unique_lock<std::mutex> lock(mutex_);
         jobs_.remove(&job);
         done_.wait(lock, [&] { return job.users == 0; });
+        if (job.error) std::rethrow_exception(job.error);
     }
 
 private:
-    static void take(Job& job) {
-        for (;;) {
-            const int lo = job.next.fetch_add(kChunk);
-            if (lo >= job.n) return;
-            for (int i = lo; i < std::min(job.n, lo + kChunk); i++) job.call(job.loop, i);
+    // (an exception ends the loop, and leaves it by its caller)
+    void take(Job& job) {
+        try {
+            for (;;) {
+                const int lo = job.next.fetch_add(kChunk);
+                if (lo >= job.n) return;
+                for (int i = lo; i < std::min(job.n, lo + kChunk); i++) job.call(job.loop, i);
+            }
+        } catch (...) {
+            job.next = job.n;
+            std::lock_guard<std::mutex> lock(mutex_);
+            if (!job.error) job.error = std::current_exception();
         }
     }
     Job* open() {  // a loop with something left, under mutex_

@@ -4,6 +4,7 @@
 
 #include <chrono>
 #include <cstdio>
+#include <string>
 
 #include <signal.h>
 #include <sys/wait.h>
@@ -83,11 +84,39 @@ int forked_busy() {
     return st == 0 ? 0 : fail(st == -1 ? "the child hangs" : "the child's loop");
 }
 
+// a loop whose body throws, in the caller's share and in the workers', with other
+// callers' loops running beside it
+int throwing() {
+    hold_workers();
+    std::atomic<bool> stop{false}, bad{false};
+    std::thread other([&] {
+        while (!stop)
+            if (!loop_runs(64)) bad = true;
+    });
+    for (int k = 0; k < 500; k++) {
+        bool caught = false;
+        try {
+            parallel_for(64, [&](int i) {
+                if (i % 8 == k % 8) throw std::bad_alloc();
+            });
+        } catch (const std::bad_alloc&) {
+            caught = true;
+        }
+        if (!caught) return fail("the exception is lost");
+        if (!loop_runs(64)) return fail("the loop after it");
+    }
+    stop = true;
+    other.join();
+    release_workers();
+    return bad ? fail("another caller's loop") : 0;
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
     const std::string what = argc > 1 ? argv[1] : "";
     if (what == "forked") return forked();
     if (what == "forked_busy") return forked_busy();
+    if (what == "throwing") return throwing();
     return fail("unknown situation");
 }
