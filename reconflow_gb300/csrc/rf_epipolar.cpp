@@ -263,23 +263,24 @@ private:
 
 std::mutex g_workers_mutex;
 int g_holders = 0;
-std::shared_ptr<Workers>& workers() {  // (never destroyed: no thread outlives its state)
-    static auto* w = new std::shared_ptr<Workers>;
-    return *w;
-}
+// the set, if someone holds it (never destroyed: no thread outlives its state)
+union Slot {
+    std::shared_ptr<Workers> workers;
+    constexpr Slot() : workers() {}
+    ~Slot() {}
+};
+Slot g_slot;
 
 // A forked child has none of the threads, and destroying what they wait on would wait
 // for them: it forgets the set (never destroyed there) and starts its own when asked.
-// No fork falls into a change of the set.
-void keep_across_forks() {
-    static const int registered = pthread_atfork(
-        [] { g_workers_mutex.lock(); }, [] { g_workers_mutex.unlock(); },
-        [] {
-            ::new (static_cast<void*>(&workers())) std::shared_ptr<Workers>;
-            g_workers_mutex.unlock();
-        });
-    (void)registered;
-}
+// No fork falls into a change of the set.  (Registered when the library is loaded: a
+// first use could be under way in another thread at the fork.)
+const int g_across_forks = pthread_atfork(
+    [] { g_workers_mutex.lock(); }, [] { g_workers_mutex.unlock(); },
+    [] {
+        ::new (static_cast<void*>(&g_slot)) Slot;
+        g_workers_mutex.unlock();
+    });
 
 int host_threads() {
     const unsigned hw = std::thread::hardware_concurrency();
@@ -287,16 +288,15 @@ int host_threads() {
 }
 
 void hold_workers() {
-    keep_across_forks();
     std::lock_guard<std::mutex> lock(g_workers_mutex);
-    if (!workers()) workers() = std::make_shared<Workers>(host_threads() - 1);
+    if (!g_slot.workers) g_slot.workers = std::make_shared<Workers>(host_threads() - 1);
     g_holders++;
 }
 
 void release_workers() {
     std::shared_ptr<Workers> last;  // destroyed after the lock: joins outside it
     std::lock_guard<std::mutex> lock(g_workers_mutex);
-    if (--g_holders == 0) last.swap(workers());
+    if (--g_holders == 0) last.swap(g_slot.workers);
 }
 
 // calls of parallel_for without workers running at once
@@ -310,7 +310,7 @@ void parallel_for(int n, F&& f) {
     std::shared_ptr<Workers> w;
     if (n >= 16) {
         std::lock_guard<std::mutex> lock(g_workers_mutex);
-        w = workers();
+        w = g_slot.workers;
     }
     if (w) {
         w->run(n, [](void* loop, int i) { (*static_cast<std::remove_reference_t<F>*>(loop))(i); },
