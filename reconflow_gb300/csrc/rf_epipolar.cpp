@@ -30,6 +30,7 @@
 #include <vector>
 
 #include <pthread.h>
+#include <sched.h>
 
 #include "../../include/reconflow_gb300.h"
 #include "rf_epipolar.h"
@@ -188,7 +189,7 @@ class Workers {
     static constexpr int kChunk = 2;
 
 public:
-    explicit Workers(int n) {
+    explicit Workers(int n) : cpus_(own_cpus()) {
         threads_.reserve(n);
         try {
             for (int i = 0; i < n; i++) threads_.emplace_back([this] { work(); });
@@ -202,6 +203,12 @@ public:
         }
         wake_.notify_all();
         for (auto& t : threads_) t.join();
+    }
+    // Whether a caller's loops may run here: threads of its own would inherit the CPUs
+    // that it is bound to, and the workers have those of whoever started them.
+    bool serves_caller() const {
+        const cpu_set_t own = own_cpus();
+        return CPU_EQUAL(&own, &cpus_);
     }
     void run(int n, void (*call)(void*, int), void* loop) {
         Job job;
@@ -221,6 +228,12 @@ public:
     }
 
 private:
+    static cpu_set_t own_cpus() {
+        cpu_set_t s;
+        CPU_ZERO(&s);
+        if (sched_getaffinity(0, sizeof s, &s) != 0) CPU_ZERO(&s);
+        return s;
+    }
     // (an exception ends the loop, and leaves it by its caller)
     void take(Job& job) {
         try {
@@ -254,6 +267,7 @@ private:
         }
     }
 
+    const cpu_set_t cpus_;
     std::mutex mutex_;
     std::condition_variable wake_, done_;
     std::list<Job*> jobs_;
@@ -303,7 +317,7 @@ void release_workers() {
 std::atomic<int> g_active{0};
 
 // f(i) for i in [0, n) on host threads, every i computed exactly as on one thread:
-// on the workers if someone holds them, otherwise on threads of its own (the cores
+// on the workers if someone holds them and they may run where the caller may, otherwise on threads of its own (the cores
 // shared among the calls running at once).
 template <class F>
 void parallel_for(int n, F&& f) {
@@ -312,7 +326,7 @@ void parallel_for(int n, F&& f) {
         std::lock_guard<std::mutex> lock(g_workers_mutex);
         w = g_slot.workers;
     }
-    if (w) {
+    if (w && w->serves_caller()) {
         w->run(n, [](void* loop, int i) { (*static_cast<std::remove_reference_t<F>*>(loop))(i); },
                &f);
         return;

@@ -6,6 +6,7 @@
 #include <cstdio>
 #include <string>
 
+#include <sched.h>
 #include <signal.h>
 #include <sys/wait.h>
 
@@ -111,6 +112,36 @@ int throwing() {
     return bad ? fail("another caller's loop") : 0;
 }
 
+// a handle made by a thread bound to one CPU: the loops of a thread that is not run
+// where that one may run (and the other way round)
+int affinity() {
+    cpu_set_t all, one;
+    CPU_ZERO(&all);
+    if (sched_getaffinity(0, sizeof all, &all) != 0) return fail("sched_getaffinity");
+    CPU_ZERO(&one);
+    for (int c = 0; c < CPU_SETSIZE && CPU_COUNT(&one) == 0; c++)
+        if (CPU_ISSET(c, &all)) CPU_SET(c, &one);
+    if (CPU_EQUAL(&one, &all)) return 0;  // a single CPU: nothing to tell apart
+    for (int k = 0; k < 2; k++) {
+        const cpu_set_t *maker = k ? &all : &one, *caller = k ? &one : &all;
+        sched_setaffinity(0, sizeof *maker, maker);
+        hold_workers();
+        sched_setaffinity(0, sizeof *caller, caller);
+        std::atomic<int> elsewhere{0};
+        for (int r = 0; r < 20; r++)
+            parallel_for(256, [&](int) {
+                cpu_set_t mine;
+                CPU_ZERO(&mine);
+                sched_getaffinity(0, sizeof mine, &mine);
+                if (!CPU_EQUAL(&mine, caller)) elsewhere++;
+                std::this_thread::sleep_for(std::chrono::microseconds(20));
+            });
+        release_workers();
+        if (elsewhere) return fail(k ? "on other CPUs than the caller's" : "bound to the maker's CPU");
+    }
+    return 0;
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
@@ -118,5 +149,6 @@ int main(int argc, char** argv) {
     if (what == "forked") return forked();
     if (what == "forked_busy") return forked_busy();
     if (what == "throwing") return throwing();
+    if (what == "affinity") return affinity();
     return fail("unknown situation");
 }

@@ -18,7 +18,7 @@ def tool(tmp_path_factory):
     return str(exe)
 
 
-@pytest.mark.parametrize("situation", ["forked", "forked_busy", "throwing"])
+@pytest.mark.parametrize("situation", ["forked", "forked_busy", "throwing", "affinity"])
 def test_workers(tool, situation):
     r = subprocess.run([tool, situation], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stderr
