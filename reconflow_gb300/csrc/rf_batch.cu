@@ -680,7 +680,7 @@ cudaError_t fill_tiles(rf_batch* b) {
         bool fits = pair_weights(solver_weights(&b->p));
         long long px = 0;
         for (int i = 0; i < b->n; i++) {
-            fits = fits && pair_stride(b->dims[i][l]);
+            fits = fits && pair_stride(b->dims[i][l].s);
             px += (long long)b->dims[i][l].w * b->dims[i][l].h;
         }
         if (!fits || px < kPairMinPixels) continue;

@@ -317,8 +317,8 @@ void release_workers() {
 std::atomic<int> g_active{0};
 
 // f(i) for i in [0, n) on host threads, every i computed exactly as on one thread:
-// on the workers if someone holds them and they may run where the caller may, otherwise on threads of its own (the cores
-// shared among the calls running at once).
+// on the workers if someone holds them and they may run where the caller may, otherwise
+// on threads of its own (the cores shared among the calls running at once).
 template <class F>
 void parallel_for(int n, F&& f) {
     std::shared_ptr<Workers> w;

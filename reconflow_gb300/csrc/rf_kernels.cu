@@ -27,6 +27,7 @@
 #include "rf_ops.cuh"
 #include "rf_pair.cuh"
 #include "rf_plain.cuh"
+#include "rf_rules.h"
 #include "rf_tile.cuh"
 
 namespace {
@@ -737,17 +738,6 @@ bool pair_weights(const Weights& wt) {
            wt.alpha_proj >= 0.0f && wt.alpha_fn >= 0.0f;
 }
 
-namespace {
-// whether a level takes two pixels per thread
-bool use_pairs(LevelDims d) {
-    // A 720p pair's level 0 (0.92 million pixels, under two waves of blocks, its
-    // state in L2) takes as long either way (37.2 against 37.0 ms a solve), a
-    // 1080p pair's (2.1 million) is faster by pairs (67.5 against 73.0 ms).
-    constexpr long long kMinPixels = 1500000;
-    return pair_stride(d) && (long long)d.w * d.h >= kMinPixels;
-}
-}  // namespace
-
 // Every launch of a warp but its first starts while the one before drains (640x480
 // 4.58 -> 4.47 ms, 1280x720 30.8 -> 30.6, 451x333 with a prior 3.22 -> 3.10, one learned
 // 720p pair 1.37 -> 1.34; released from the blocks' start instead of their end, or with
@@ -755,7 +745,7 @@ bool use_pairs(LevelDims d) {
 int launch_half_a(const ReconFields& f, const LevelConsts* lc, const Weights& wt, LevelDims d,
                   bool first, bool uc_from_buffer, int prior, cudaStream_t st, dim3 b) {
     const int fi = first ? 1 : 0, ub = uc_from_buffer ? 1 : 0;
-    const bool pairs = use_pairs(d);
+    const bool pairs = use_pairs(d.w, d.h, d.s);
     auto one = prior == 1 ? k_recon_a1<1> : prior == 2 ? k_recon_a1<2> : k_recon_a1<0>;
     auto two = prior == 1 ? k_recon_a2<1> : prior == 2 ? k_recon_a2<2> : k_recon_a2<0>;
     if (pairs) {
@@ -769,7 +759,7 @@ int launch_half_a(const ReconFields& f, const LevelConsts* lc, const Weights& wt
 int launch_half_b(const ReconFields& f, const Weights& wt, LevelDims d, bool first, bool last,
                   cudaStream_t st, dim3 b) {
     const int fi = first ? 1 : 0;
-    if (use_pairs(d)) {
+    if (use_pairs(d.w, d.h, d.s)) {
         const dim3 g((d.w + kPairW - 1) / kPairW, (d.h + kPairRows - 1) / kPairRows);
         return launch_pdl(true, last ? k_recon_b2<true> : k_recon_b2<false>, g,
                           dim3(32 * kPairRows), st, f, wt, d, fi);

@@ -30,6 +30,7 @@
 
 #include "rf_ops.cuh"
 #include "rf_packed.cuh"
+#include "rf_rules.h"
 
 namespace rf {
 
@@ -77,11 +78,7 @@ __device__ __forceinline__ float2 ld2_at(const float* p, int i, long long) {
 // occupancy with direct loads, 48 and 57% with copies, 0.95 -> 0.79 ms per 59
 // million pixels).  Column 0 of the tile is at column 4 of a row in shared
 // memory, so that every copy is aligned.
-constexpr int kPairRows = 4;
-constexpr int kPairW = 64, kPitch = kPairW + 8;
-
-// rows whose pixel pairs and groups of four are aligned
-inline bool pair_stride(LevelDims d) { return d.s % 4 == 0; }
+constexpr int kPitch = kPairW + 8;
 
 // the fields A reads, as ReconFields has them in a row: u, v, duhat, dvhat,
 // pu1, pu2, pv1, pv2, uproj, vproj, sku, skv, Ix, Iy, Iz, X, Y, Z
