@@ -37,6 +37,7 @@
 #include "rf_alloc.h"
 #include "rf_nvtx.h"
 #include "rf_kernels.cuh"
+#include "rf_rules.h"
 #include "rf_tc.cuh"
 
 namespace rf_cnn_impl {
@@ -761,14 +762,10 @@ rf_status conv3_launch(rf_cnn* c, int li, ConvInput in, int B, int H, int W, bf1
     CN(cudaGetLastError());
     return RF_OK;
 }
-// 256 positions per CTA where every SM gets one and two or more fit on it, otherwise
-// 128.  The larger tile loads the weights and the two rows around it half as often
-// (64 images of 160 x 90: 0.53 ms against 0.65, eight 0.133 and 0.143); with too few
-// of them SMs idle (one image: the same either way).
 template <int NT>
 rf_status conv3_direct(rf_cnn* c, int li, ConvInput in, int B, int H, int W, bf16* y, float* yf) {
     const long long npos = (long long)B * (H + 2) * (W + 2);
-    if (npos >= 152ll * rf_tc::kTM * 2 && rf_tc::ConvSmem<NT, 2>::bytes(W + 2) <= 113 * 1024)
+    if (rf::conv_wide_tile(npos, rf_tc::ConvSmem<NT, 2>::bytes(W + 2), rf::sm_count()))
         return conv3_launch<NT, 2>(c, li, in, B, H, W, y, yf);
     return conv3_launch<NT, 1>(c, li, in, B, H, W, y, yf);
 }

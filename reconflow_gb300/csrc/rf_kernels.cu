@@ -17,9 +17,10 @@
 // All pixel-local state (duhat, p, uproj, sk) is updated in place: each is
 // read at a neighbour only by the other kernel of the pair.
 #include <atomic>
-#include <cooperative_groups.h>
 #include <cstdint>
 #include <cstdlib>
+
+#include <cooperative_groups.h>
 
 #include "../../include/reconflow_gb300.h"
 #include "rf_alloc.h"
@@ -768,13 +769,17 @@ int launch_half_b(const ReconFields& f, const Weights& wt, LevelDims d, bool fir
     return launch_pdl(true, last ? k_recon_b1<true> : k_recon_b1<false>, g, b, st, f, wt, d, fi);
 }
 
-namespace {
-template <int ROWS, int K>
-long long tile_blocks(LevelDims d) {
-    using T = ReconTile<ROWS, K>;
-    return (long long)((d.w + T::W - 1) / T::W) * ((d.h + T::H - 1) / T::H);
+int sm_count() {
+    static std::atomic<int> known[64];  // by device
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+    if (dev < 64 && (sms = known[dev]) > 0) return sms;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
+    if (dev < 64) known[dev] = sms;
+    return sms;
 }
 
+namespace {
 template <int ROWS, int K>
 int recon_tiles(const ReconFields& f, const ReconState& b, const LevelConsts* lc, const Weights& wt,
                 LevelDims d, int n_iters, bool uc_from_buffer, int prior, cudaStream_t st) {
@@ -796,38 +801,19 @@ int recon_tiles(const ReconFields& f, const ReconState& b, const LevelConsts* lc
     }
     return launches;
 }
-
-// Which tile a level takes, 0 for none: the first of those below with no more
-// than a block per SM.
-int recon_tile_kind(LevelDims d) {
-    // An iteration of a block is bound by the instructions of its warps, so the
-    // smallest tile is the fastest while every block has an SM to itself; two
-    // blocks on one take twice as long.  Solves of 96x72 .. 640x480, the level in
-    // question with one tile and the next larger: 80x60 with 24 x 2 (10 rows) and
-    // 24 x 8 (16): 2.44 and 2.56 ms (of a 160x120 solve); 112x83 with 24 x 4 and
-    // 20 x 8: 3.74 and 3.82 (451x333); 160x120 with 20 x 8, three iterations, and
-    // 24 x 12, two: 2.42 and 2.51; 225x166 with 24 x 12 and with two launches per
-    // iteration: 3.52 and 3.75.  320x240, 280 blocks of 24 x 12, is as fast by two
-    // launches per iteration (4.95 against 5.01, 640x480).
-    constexpr int kSms = 152;
-    if (tile_blocks<10, 2>(d) <= kSms) return 1;
-    if (tile_blocks<12, 2>(d) <= kSms) return 2;
-    if (tile_blocks<20, 3>(d) <= kSms) return 3;
-    if (tile_blocks<20, 2>(d) <= kSms) return 4;
-    return 0;
-}
 }  // namespace
 
 bool use_recon_tiles(const Weights& wt, LevelDims d, int n_iters) {
     // (a row that ends where the next begins has that one's first pixels to its
     // right: a tile's region must not reach a second row)
-    return n_iters >= 2 && pair_weights(wt) && (d.s > d.w || d.w >= kTileW) && recon_tile_kind(d);
+    return n_iters >= 2 && pair_weights(wt) && (d.s > d.w || d.w >= kTileW) &&
+           recon_tile_kind(d.w, d.h, sm_count()) != 0;
 }
 
 int launch_recon_tiles(const ReconFields& f, const ReconState& b, const LevelConsts* lc,
                        const Weights& wt, LevelDims d, int n_iters, bool uc_from_buffer, int prior,
                        cudaStream_t st) {
-    switch (recon_tile_kind(d)) {
+    switch (recon_tile_kind(d.w, d.h, sm_count())) {
         case 1: return recon_tiles<10, 2>(f, b, lc, wt, d, n_iters, uc_from_buffer, prior, st);
         case 2: return recon_tiles<12, 2>(f, b, lc, wt, d, n_iters, uc_from_buffer, prior, st);
         case 3: return recon_tiles<20, 3>(f, b, lc, wt, d, n_iters, uc_from_buffer, prior, st);

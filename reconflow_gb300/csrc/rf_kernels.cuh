@@ -163,6 +163,8 @@ int launch_half_a(const ReconFields& f, const LevelConsts* lc, const Weights& wt
                   bool first, bool uc_from_buffer, int prior, cudaStream_t st, dim3 block);
 int launch_half_b(const ReconFields& f, const Weights& wt, LevelDims d, bool first, bool last,
                   cudaStream_t st, dim3 block);
+// Multiprocessors of the current device.
+int sm_count();
 // All inner iterations of a ReconFlow warp, several per launch (rf_tile.cuh),
 // between f's state and `b`, f's at the end.  Whether a level takes them
 // (`n_iters` of them), and the launches; returns their number, < 0 if one failed.

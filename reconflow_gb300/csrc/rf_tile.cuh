@@ -26,6 +26,7 @@
 #pragma once
 
 #include "rf_pair.cuh"
+#include "rf_rules.h"
 
 namespace rf {
 
@@ -35,8 +36,6 @@ struct ReconState {
 };
 
 namespace {
-
-constexpr int kTileW = 32;  // a region's columns, one per lane
 
 // what a block's threads show each other: p for part A, the points for A and
 // (their triangulated form) for B, duhat for B; a ring around each

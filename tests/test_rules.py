@@ -30,3 +30,25 @@ def test_pairs_fit_a_grid(ask, w, h, align):
     s = align_up(w, align)
     want = s % 4 == 0 and w * h >= 1500000 and -(-h // 4) <= 65535
     assert ask([f"pairs {w} {h} {s}"]) == [int(want)]
+
+
+# the region's columns and rows that a block's tile keeps, in the order they are tried
+TILES = [(24, 2), (24, 4), (20, 8), (24, 12)]
+
+
+@pytest.mark.parametrize("sms", [1, 20, 148, 152, 160])
+def test_tiles_have_an_sm_each(ask, sms):
+    sizes = [(w, h) for w in (1, 24, 25, 96, 97, 160, 225, 240, 288, 289, 320)
+             for h in (1, 2, 38, 61, 72, 84, 120, 144, 145, 152, 166, 168, 240)]
+    got = ask([f"tile {w} {h} {sms}" for w, h in sizes])
+    for (w, h), kind, blocks in zip(sizes, got[::2], got[1::2]):
+        need = [-(-w // tw) * -(-h // th) for tw, th in TILES]
+        fits = [i for i, n in enumerate(need) if n <= sms]
+        assert (kind, blocks) == ((fits[0] + 1, need[fits[0]]) if fits else (0, 0)), (w, h)
+
+
+@pytest.mark.parametrize("sms", [1, 148, 152])
+def test_wide_convolution_tiles(ask, sms):
+    n = 256 * sms
+    q = [(n - 1, 1000), (n, 1000), (n, 113 * 1024), (n, 113 * 1024 + 1)]
+    assert ask([f"conv {a} {b} {sms}" for a, b in q]) == [0, 1, 1, 0]
