@@ -216,10 +216,16 @@ RF_API rf_status rf_debug_bounds_selftest(void);
 /* Tile shape of the inner-iteration kernels at each pyramid level
  * (tile_w[l] x tile_h[l] pixels, one thread each; 32 .. 256 threads, a
  * multiple of 32; default 32 x 8), as reconflow_gb300/autotune.py picks
- * them.  No reference counterpart (the reference's BlockWidth / BlockHeight
+ * them, where these kernels take one (rf_level_takes_tile).  No reference counterpart (the reference's BlockWidth / BlockHeight
  * constructor arguments, Reconflow.h:12, play this role for all kernels).
  * Results do not depend on it. */
 RF_API rf_status rf_set_tiles(rf_handle* h, const int* tile_w, const int* tile_h);
+/* Whether the inner iterations of a solve at pyramid level `level` run kernels
+ * of the shape that rf_set_tiles gives: 1; or ones with a tile of their own
+ * (several iterations per launch on small levels, two pixels per thread on
+ * large ones, a cluster, plain TV-L1): 0.  Negative: bad argument.  No
+ * reference counterpart. */
+RF_API int rf_level_takes_tile(const rf_handle* h, int level);
 
 /* Use a caller's CUDA stream (cudaStream_t passed as void*; NULL = the
  * handle's own stream). */
@@ -233,11 +239,12 @@ RF_API rf_status rf_host_free(void* ptr);
 /* Timing hook (no reference counterpart): after a solve, time each of the
  * two inner-iteration kernels at pyramid level `level` on the handle's
  * stream: `n_iters` launches of one kernel back to back, captured in a CUDA
- * graph as the solve captures them, the graph replay timed with CUDA events;
+ * graph, the graph replay timed with CUDA events;
  * returns the mean time per launch in milliseconds (ms[0] = data /
  * projection / triangulation kernel, ms[1] = dual / median / clean-up
- * kernel; plain TV-L1: data, dual as launches of their own, where its solve
- * runs several iterations per launch).  Changes the solver state; results of
+ * kernel; plain TV-L1: data, dual).  Where a solve runs several iterations per
+ * launch (plain TV-L1, small ReconFlow levels) these are not its launches but
+ * the two half-steps as launches of their own.  Changes the solver state; results of
  * the last solve are no longer valid afterwards. */
 RF_API rf_status rf_profile_iterations(rf_handle* h, int level, int n_iters, float* ms);
 
@@ -308,10 +315,16 @@ RF_API rf_status rf_batch_energies_async(rf_batch* b, double* out);
 RF_API rf_status rf_batch_solve_warm_levels(rf_batch* b, const double* R0, const double* t0,
                                             const double* R1, const double* t1, int level,
                                             const int* warps, const int* iters);
-/* Tile shape of each pyramid level (tile_w[l] x tile_h[l] pixels, one
- * thread each; 32 .. 256 threads, a multiple of 32; default 32 x 8), as
- * reconflow_gb300/autotune.py picks them.  Results do not depend on it. */
+/* Tile shape of each pyramid level's kernels (tile_w[l] x tile_h[l] pixels,
+ * one thread each; 32 .. 256 threads, a multiple of 32; default 32 x 8), as
+ * reconflow_gb300/autotune.py picks them: warp, derivatives, medians,
+ * upscale, and the inner iterations unless they take two pixels per thread
+ * (rf_batch_level_takes_tile).  Results do not depend on it. */
 RF_API rf_status rf_batch_set_tiles(rf_batch* b, const int* tile_w, const int* tile_h);
+/* Whether the inner iterations at `level` run with the level's tile shape: 1;
+ * or, two pixels per thread, with a tile of their own: 0.  Negative: bad
+ * argument.  No reference counterpart. */
+RF_API int rf_batch_level_takes_tile(const rf_batch* b, int level);
 /* Timing hook (no reference counterpart): after a ReconFlow solve, the mean
  * time in milliseconds of one launch of each inner-iteration kernel over
  * every pair at `level` with the current tiles (ms[0] data / projection /

@@ -87,6 +87,7 @@ _SIGS = [
     ("rf_debug_bounds_selftest", _I, []),
     ("rf_set_cluster_pixels", _I, [ctypes.c_longlong]),
     ("rf_set_tiles", _I, [_VP, _VP, _VP]),
+    ("rf_level_takes_tile", _I, [_VP, _I]),
     ("rf_set_stream", _I, [_VP, _VP]),
     ("rf_synchronize", _I, [_VP]),
     ("rf_host_alloc", _I, [ctypes.c_size_t, ctypes.POINTER(_VP)]),
@@ -110,6 +111,7 @@ _SIGS = [
     ("rf_batch_warm_planes", _I, [_VP, _I, _VP, _VP, _VP, _VP, _VP]),
     ("rf_batch_image_planes", _I, [_VP, _I, _I, _VP, _VP]),
     ("rf_batch_set_tiles", _I, [_VP, _VP, _VP]),
+    ("rf_batch_level_takes_tile", _I, [_VP, _I]),
     ("rf_batch_profile_level", _I, [_VP, _I, _I, _VP]),
     ("rf_batch_download_flow", _I, [_VP, _I, _VP, _VP, _I]),
     ("rf_batch_download_points", _I, [_VP, _I, _VP, _VP, _VP, _I]),

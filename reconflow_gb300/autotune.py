@@ -4,17 +4,20 @@ Every step of a batched solve is one launch over the tiles of every pair at
 one pyramid level (``rf_batch.cu``); the tile shape decides how pixels map
 to blocks (and so the wave count, the tail of the last wave and how well
 neighbouring pixels share cache lines), never the arithmetic, so results are
-identical for every shape.  ``autotune`` times the two inner-iteration
-kernels of each level (``rf_batch_profile_level``: launches back to back in a
-CUDA graph, CUDA events) for every candidate shape and keeps the fastest per
-level.  ``tiles_for`` turns a saved table into per-level shapes for a batch
+identical for every shape.  ``autotune`` times, for every candidate shape,
+what the shape decides at a level, and keeps the fastest: the two
+inner-iteration kernels (``rf_batch_profile_level``: launches back to back in
+a CUDA graph, CUDA events), or, where these take two pixels per thread and a
+tile of their own, the warp, derivative and median passes around them (solves
+of that level that run several warps of one iteration).  ``tiles_for`` turns a saved table into per-level shapes for a batch
 of any size by the pixel count of the level (summed over pairs).
 
     python -m reconflow_gb300.autotune --size 1280x720 --pairs 64 --out table.json
 
 The tile candidates span 2 to 8 warps per block (32 x 2 .. 16 x 16), so the
-shape search also picks the warps per block.  For one ReconFlow handle a
-second dimension is searched: iterations per launch.  The two-launch loop
+shape search also picks the warps per block.  For one ReconFlow handle the
+levels whose kernels take no shape (small ones: several iterations per
+launch) keep the default, and a second dimension is searched: iterations per launch.  The two-launch loop
 runs one inner iteration per pair of launches (a CUDA graph); the
 thread-block-cluster kernel runs all of a warp's iterations at a level in
 one launch (rf_set_cluster_pixels: every level of at most n pixels).
@@ -28,30 +31,54 @@ from __future__ import annotations
 import json
 import os
 
+DEFAULT = (32, 8)
 CANDIDATES = [(32, 8), (64, 4), (128, 2), (32, 4), (64, 2), (16, 16), (32, 2), (16, 8)]
+
+
+def _passes_ms(batch, R1s, t1s, level, warps=20, solves=5):
+    """What one more warp of one iteration at `level` takes in a solve that
+    starts there (the fastest of `solves` solves with `warps` more).  (With no
+    iteration the medians would see only zeros, which they take more time for.)"""
+    import time
+
+    def fastest(n):
+        best = float("inf")
+        for k in range(1 + solves):  # the first one captures the graph
+            batch.synchronize()
+            t0 = time.perf_counter()
+            batch.solveWarm(level, R1s, t1s, [0] * level + [n], [0] * level + [1])
+            batch.synchronize()
+            if k:
+                best = min(best, (time.perf_counter() - t0) * 1000.0)
+        return best
+
+    return (fastest(1 + warps) - fastest(1)) / warps
 
 
 def autotune(batch, R1s, t1s, candidates=CANDIDATES, iters=20, log=None):
     """Pick the fastest tile per level of `batch` (images and cameras set).
-    Returns [{"level", "pixels", "tile", "ms": {shape: ms}}] and leaves the
-    batch set to the chosen tiles."""
+    Returns [{"level", "pixels", "tile", "timed", "ms": {shape: ms}}] and leaves
+    the batch set to the chosen tiles; "timed" says what the shape was chosen
+    for: "iterations", or "passes" where these take no shape."""
     L = int(batch.params.n_levels)
-    best = [(32, 8)] * L
+    best = [DEFAULT] * L
     table = []
     for level in range(L):
         px = sum(batch.levelDims(i, level)[0] * batch.levelDims(i, level)[1]
                  for i in range(batch.n))
+        inner = batch.levelTakesTile(level)
         times = {}
         for shape in candidates:
             trial = list(best)
             trial[level] = shape
             batch.setTiles([s[0] for s in trial], [s[1] for s in trial])
             batch.solveR(R1s, t1s)
-            a, b = batch.profileLevel(level, iters)
-            times[f"{shape[0]}x{shape[1]}"] = a + b
+            times[f"{shape[0]}x{shape[1]}"] = (sum(batch.profileLevel(level, iters)) if inner else
+                                               _passes_ms(batch, R1s, t1s, level))
         pick = min(times, key=times.get)
         best[level] = tuple(int(x) for x in pick.split("x"))
-        table.append({"level": level, "pixels": px, "tile": list(best[level]), "ms": times})
+        table.append({"level": level, "pixels": px, "tile": list(best[level]),
+                      "timed": "iterations" if inner else "passes", "ms": times})
         if log:
             log(f"level {level} ({px} px): {pick}  " +
                 " ".join(f"{k} {v * 1e3:.1f}us" for k, v in sorted(times.items(), key=lambda x: x[1])))
@@ -61,11 +88,17 @@ def autotune(batch, R1s, t1s, candidates=CANDIDATES, iters=20, log=None):
 
 def autotune_single(flow, R1, t1, n_levels, candidates=CANDIDATES, iters=20, log=None):
     """The same search for one ReconFlow handle (rf_set_tiles,
-    rf_profile_iterations); images and cameras must be set."""
-    best = [(32, 8)] * n_levels
+    rf_profile_iterations); images and cameras must be set.  Levels whose
+    kernels take no shape keep the default."""
+    best = [DEFAULT] * n_levels
     table = []
     for level in range(n_levels):
         times = {}
+        if not flow.levelTakesTile(level):
+            table.append({"level": level, "tile": list(DEFAULT), "ms": times})
+            if log:
+                log(f"level {level}: kernels with a tile of their own")
+            continue
         for shape in candidates:
             trial = list(best)
             trial[level] = shape

@@ -899,8 +899,8 @@ rf_status enqueue_batch(rf_batch* b, int kind) {
             NvtxRange warp_range("batch level %d warp %d", level, warp);
             // WarpImage and ComputeDerivatives as two launches: the fused
             // shared-memory form recomputes its halo's warped values, which at
-            // the tuned level-0 tile (32 x 2) costs more than the warped
-            // image's round trip (0.312 vs 0.196 ms for 8 720p pairs)
+            // a 32 x 2 tile costs more than the warped image's round trip
+            // (0.312 vs 0.196 ms for 8 720p pairs)
             BL(launch_op(b, level, OpWarp{b->pI1(level), u, v, P(P_I1W)}));
             BL(launch_op(b, level, OpDeriv{b->pI0(level), P(P_I1W), P(P_IX), P(P_IY), P(P_IZ)}));
             const ReconFields r = fields_of(
@@ -1324,6 +1324,11 @@ rf_status rf_batch_set_tiles(rf_batch* b, const int* tile_w, const int* tile_h) 
     return RF_OK;
 }
 
+int rf_batch_level_takes_tile(const rf_batch* b, int level) {
+    if (!b || level < 0 || level >= b->L) return -1;
+    return b->p.method == RF_METHOD_TVL1 || b->split > 0 || b->pair_blocks[level] == 0 ? 1 : 0;
+}
+
 rf_status rf_batch_profile_level(rf_batch* b, int level, int n_iters, float* ms) {
     if (!b || !ms || n_iters < 1 || level < 0 || level >= b->L)
         return bfail(RF_ERR_INVALID_ARG, "rf_batch_profile_level: bad argument");
@@ -1345,7 +1350,7 @@ rf_status rf_batch_profile_level(rf_batch* b, int level, int n_iters, float* ms)
         BC(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
         int bad = 0;
         for (int i = 0; i < n_iters && !bad; i++)
-            if (pair_weights(wt))
+            if (pair_weights(wt) && b->split == 0)
                 bad = k == 0 ? launch_half_a(b, level, r, wt, false, false)
                              : launch_half_b(b, level, r, wt, false, false);
             else

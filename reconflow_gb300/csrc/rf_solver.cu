@@ -22,6 +22,7 @@
 #include "rf_nvtx.h"
 #include "rf_kernels.cuh"
 #include "rf_plain.cuh"
+#include "rf_rules.h"
 #include "rf_tile.cuh"
 
 using namespace rf;
@@ -1063,6 +1064,16 @@ rf_status rf_host_alloc(size_t bytes, void** ptr) {
 rf_status rf_host_free(void* ptr) {
     if (ptr) RF_CUDA(cudaFreeHost(ptr));
     return RF_OK;
+}
+
+int rf_level_takes_tile(const rf_handle* h, int level) {
+    if (!h || level < 0 || level >= h->L) return -1;
+    if (h->p.method == RF_METHOD_TVL1) return 0;
+    const LevelDims d{h->W[level], h->H[level], h->S[level]};
+    const Weights wt = make_weights(h->p);
+    if (h->p.n_solver_iters > 0 && use_cluster_at(h, d)) return 0;
+    if (use_recon_tiles(wt, d, h->p.n_solver_iters)) return 0;
+    return pair_weights(wt) && use_pairs(d.w, d.h, d.s) ? 0 : 1;
 }
 
 rf_status rf_profile_iterations(rf_handle* h, int level, int n_iters, float* ms) {

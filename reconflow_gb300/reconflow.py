@@ -207,8 +207,16 @@ class CudaFlow:
                                        (ctypes.c_int * n)(*map(int, tile_h))))
         return 0
 
+    def levelTakesTile(self, level) -> bool:
+        """Whether the inner iterations at `level` run in setTiles' shape
+        (rf_level_takes_tile)."""
+        r = self._lib.rf_level_takes_tile(self._handle(), int(level))
+        if r < 0:
+            raise ValueError("no such level")
+        return r != 0
+
     def profileLevel(self, level, nIters=20):
-        """Mean ms per launch of the two inner-iteration kernels at `level`
+        """Mean ms per launch of the two inner half-steps at `level`
         (rf_profile_iterations); needs a prior solve and invalidates it."""
         ms = (ctypes.c_float * 2)()
         N.check(self._lib.rf_profile_iterations(self._handle(), int(level), int(nIters), ms))
@@ -500,6 +508,14 @@ class ReconFlowBatch:
             raise ValueError("one tile shape per level")
         N.check(self._lib.rf_batch_set_tiles(self._h, (ctypes.c_int * n)(*map(int, tile_w)),
                                              (ctypes.c_int * n)(*map(int, tile_h))))
+
+    def levelTakesTile(self, level) -> bool:
+        """Whether the inner iterations at `level` run in setTiles' shape
+        (rf_batch_level_takes_tile)."""
+        r = self._lib.rf_batch_level_takes_tile(self._h, int(level))
+        if r < 0:
+            raise ValueError("no such level")
+        return r != 0
 
     def profileLevel(self, level, nIters=20):
         """Mean ms per launch of the two inner-iteration kernels at `level`
