@@ -366,12 +366,13 @@ __global__ void __launch_bounds__(kMedW* kMedH / 2)
     const int lx = threadIdx.x & 31, ly = 2 * (int)(threadIdx.x >> 5);
     const int ix = x0 + lx, iy = y0 + ly, pos = ix + iy * d.s;
     const bool in_0 = ix < d.w && iy < d.h, in_1 = ix < d.w && iy + 1 < d.h;
+    const long long end = (long long)d.s * d.h;  // of the level's planes
     float a0 = 0.0f, a1 = 0.0f;
-    if (ADD && in_0) a0 = add[pos];
-    if (ADD && in_1) a1 = add[pos + d.s];
+    if (ADD && in_0) a0 = RF_PT(add, pos, end);
+    if (ADD && in_1) a1 = RF_PT(add, pos + d.s, end);
     for (int i = threadIdx.x; i < (kMedH + 4) * kMedPitch; i += kMedW * kMedH / 2) {
         const int at = median5_tap(x0 + i % kMedPitch - 2, y0 + i / kMedPitch - 2, d.w, d.h, d.s);
-        tile[i] = at >= 0 ? in[at] : 0.0f;
+        tile[i] = at >= 0 ? RF_PT(in, at, end) : 0.0f;
     }
     __syncthreads();
     if (!in_0) return;
@@ -381,10 +382,10 @@ __global__ void __launch_bounds__(kMedW* kMedH / 2)
     for (int k = 0; k < 30; k++) w[k] = t[k / 5 * kMedPitch + k % 5];
     const bool ok = median25_two(w, m0, m1);
     if (!ok || m0 == 0.0f) m0 = median25_tile(t, !ok);
-    out[pos] = ADD ? a0 + m0 : m0;
+    RF_PT(out, pos, end) = ADD ? a0 + m0 : m0;
     if (!in_1) return;
     if (!ok || m1 == 0.0f) m1 = median25_tile(t + kMedPitch, !ok);
-    out[pos + d.s] = ADD ? a1 + m1 : m1;
+    RF_PT(out, pos + d.s, end) = ADD ? a1 + m1 : m1;
 }
 
 __global__ void k_median3d(const float* __restrict__ X, const float* __restrict__ Y,

@@ -92,6 +92,8 @@ __device__ __forceinline__ const float& rf_checked(const float* p, long long i, 
     return p[i];
 }
 #define RF_AT(f, name, idx) rf_checked((f).name, (long long)(idx), (f).extent)
+// element `idx` of a plane of `n` elements that is not a field
+#define RF_PT(p, idx, n) rf_checked(p, (long long)(idx), n)
 
 // this translation unit's counts (and reset them)
 static inline unsigned long long rf_oob_take(long long* first) {
@@ -107,6 +109,7 @@ static inline unsigned long long rf_oob_take(long long* first) {
 }
 #else
 #define RF_AT(f, name, idx) (f).name[idx]
+#define RF_PT(p, idx, n) ((void)(n), (p)[idx])
 #endif
 
 // Per-level camera constants of one pair (K pyramid, P = K0 [R0|t0],

@@ -39,7 +39,6 @@ namespace {
 // elements i, i + 1 of a field (i even)
 #ifdef RF_BOUNDS_CHECK
 #define RF_LD2(f, name, i) mk2(RF_AT(f, name, i), RF_AT(f, name, (i) + 1))
-#define RF_PT(p, i, n) rf_checked(p, (long long)(i), n)
 __device__ __forceinline__ float2 ld2_at(const float* p, long long i, long long n) {
     return make_float2(rf_checked(p, i, n), rf_checked(p, i + 1, n));
 }
@@ -49,7 +48,6 @@ __device__ __forceinline__ f2 ld2(const float* p) {
     return f2{t.x, t.y};
 }
 #define RF_LD2(f, name, i) ld2((f).name + (i))
-#define RF_PT(p, i, n) (p)[i]
 __device__ __forceinline__ float2 ld2_at(const float* p, int i, long long) {
     return *reinterpret_cast<const float2*>(p + i);
 }

@@ -130,6 +130,7 @@ __global__ void __launch_bounds__(32 * WARPS)
     const int first_row = warp * R;
     const bool any_y = y0 < d.h && y0 + R > 0;
     const bool in_x = x >= 0 && x < d.w;
+    const long long end = (long long)d.s * d.h;  // of the level's planes
     const int above = warp > 0 ? warp - 1 : 0, below = warp < WARPS - 1 ? warp + 1 : warp;
 
     PlainPx c[R];
@@ -141,8 +142,8 @@ __global__ void __launch_bounds__(32 * WARPS)
         c[r].dit = 0.0f;
         if (in_x && y >= 0 && y < d.h) {
             const int pos = x + y * d.s;
-            c[r].di = f2{Ix[pos], Iy[pos]};
-            c[r].dit = Iz[pos];
+            c[r].di = f2{RF_PT(Ix, pos, end), RF_PT(Iy, pos, end)};
+            c[r].dit = RF_PT(Iz, pos, end);
         }
         const float m = c[r].di.x * c[r].di.x + c[r].di.y * c[r].di.y;
         c[r].magi = m;
@@ -159,9 +160,9 @@ __global__ void __launch_bounds__(32 * WARPS)
         n1[r] = n2[r] = dup2(-0.0f);
         if (!first && in_x && y >= 0 && y < d.h) {
             const int pos = x + y * d.s;
-            du[r] = f2{in.du[pos], in.dv[pos]};
-            n1[r] = f2{in.pu1[pos], in.pv1[pos]};
-            n2[r] = f2{in.pu2[pos], in.pv2[pos]};
+            du[r] = f2{RF_PT(in.du, pos, end), RF_PT(in.dv, pos, end)};
+            n1[r] = f2{RF_PT(in.pu1, pos, end), RF_PT(in.pv1, pos, end)};
+            n2[r] = f2{RF_PT(in.pu2, pos, end), RF_PT(in.pv2, pos, end)};
         }
     }
     s_n2[warp][lane] = n2[R - 1];
@@ -234,13 +235,13 @@ __global__ void __launch_bounds__(32 * WARPS)
         const int row = warp * R + r, y = y0 + r;
         if (row < K || row >= R * WARPS - K || y >= d.h) continue;
         const int pos = x + y * d.s;
-        out.du[pos] = du[r].x;
-        out.dv[pos] = du[r].y;
+        RF_PT(out.du, pos, end) = du[r].x;
+        RF_PT(out.dv, pos, end) = du[r].y;
         if (!last) {
-            out.pu1[pos] = n1[r].x;
-            out.pv1[pos] = n1[r].y;
-            out.pu2[pos] = n2[r].x;
-            out.pv2[pos] = n2[r].y;
+            RF_PT(out.pu1, pos, end) = n1[r].x;
+            RF_PT(out.pv1, pos, end) = n1[r].y;
+            RF_PT(out.pu2, pos, end) = n2[r].x;
+            RF_PT(out.pv2, pos, end) = n2[r].y;
         }
     }
 }
