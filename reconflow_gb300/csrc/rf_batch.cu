@@ -47,8 +47,9 @@ constexpr int kMaxLevels = 16;
 // half-steps: below, a launch is shorter than the chain of one pixel's
 // instructions and the one-pixel kernels' is the shorter chain.  Measured, 2 / 4
 // learned 720p pairs (levels 0.46 and 1.84 / 0.92 and 3.7 million pixels): from
-// 0.4 million 2.00 / 3.21 ms, from 1.5 million 2.06 / 3.53, never 2.13 / 3.65;
-// from 0.05 million the mixed batch loses 1%.
+// 0.4 million 1.82 / 3.04 ms, from 1.5 million 1.94 / 3.48, never 2.03 / 3.66; from
+// 0.2 million one learned pair (0.23 and 0.92) 1.19 against 1.19, from 0.05 million
+// the mixed batch of 12 251.1 against 251.4.
 constexpr long long kPairMinPixels = 400000;
 
 struct BatchPair {

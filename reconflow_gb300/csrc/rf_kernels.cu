@@ -930,8 +930,9 @@ int launch_plain_warp(PlainState a, PlainState b, const float* Ix, const float* 
     // fewer pixels per block, more iterations per launch (solve of 64x48, all
     // five levels small: 0.90 ms against 1.22; K = 4, 5 and 8: 0.94, 1.00, 0.91;
     // 0.81 with used-up rows sitting out).
-    // Between them, 320x240 within a 640x480 solve: 1.49 ms as a large level, 1.67
-    // as a small one; 200x150: 0.98 as a small one, 1.27 as a large one.
+    // Between them, 320x240 within a 640x480 solve: 1.30 ms as a large level, 1.41
+    // as a small one; 200x150 within one of 400x300: 0.556 as a small one, 0.567 as a
+    // large one.
     if ((long long)d.w * d.h >= 60000)
         return plain_tiles<2, 16, 4, false>(a, b, Ix, Iy, Iz, wt, d, n_iters, st, in_b);
     return plain_tiles<1, 20, 6, true>(a, b, Ix, Iy, Iz, wt, d, n_iters, st, in_b);

@@ -16,9 +16,10 @@ inline bool pair_stride(int s) { return s % 4 == 0; }
 
 // Whether a level of a single pair takes two pixels per thread.
 inline bool use_pairs(int w, int h, int s) {
-    // A 720p pair's level 0 (0.92 million pixels, under two waves of blocks, its
-    // state in L2) takes as long either way (37.2 against 37.0 ms a solve), a
-    // 1080p pair's (2.1 million) is faster by pairs (67.5 against 73.0 ms).
+    // A 1080p pair's level 0 (2.1 million pixels) is faster by pairs: 59.6 against
+    // 68.9 ms a solve (6 levels, 5 x 100 iterations). The gain ends below: a 720p
+    // pair's (0.92 million, under two waves of blocks, its state in L2) would take
+    // 29.6 against 30.2.
     constexpr long long kMinPixels = 1500000;
     // the one-pixel kernels' blocks have twice the rows, so a level can be too tall
     // for a grid of these alone
@@ -39,13 +40,13 @@ constexpr long long recon_tile_blocks(int w, int h, int rows, int k) {
 inline int recon_tile_kind(int w, int h, int sms) {
     // An iteration of a block is bound by the instructions of its warps, so the
     // smallest tile is the fastest while every block has an SM to itself; two
-    // blocks on one take twice as long.  Solves of 96x72 .. 640x480, the level in
-    // question with one tile and the next larger: 80x60 with 24 x 2 (10 rows) and
-    // 24 x 8 (16): 2.44 and 2.56 ms (of a 160x120 solve); 112x83 with 24 x 4 and
-    // 20 x 8: 3.74 and 3.82 (451x333); 160x120 with 20 x 8, three iterations, and
-    // 24 x 12, two: 2.42 and 2.51; 225x166 with 24 x 12 and with two launches per
-    // iteration: 3.52 and 3.75.  320x240, 280 blocks of 24 x 12, is as fast by two
-    // launches per iteration (4.95 against 5.01, 640x480).
+    // blocks on one take twice as long.  Solves on 152 SMs, the level in question
+    // with its tile and the next: 80x60 with 24 x 2 and 24 x 4: 2.55 and 2.66 ms
+    // (of a 160x120 solve, 5 x 100); 112x83 with 24 x 4 and 20 x 8: 2.85 and 2.93
+    // (451x333, 3 x 50); 160x120 with 20 x 8, three iterations, and 24 x 12, two:
+    // 2.55 and 2.79; 225x166 with 24 x 12 and with two launches per iteration: 2.85
+    // and 3.15.  320x240, 280 blocks of 24 x 12, is faster by two launches per
+    // iteration (4.30 against 4.44, 640x480).
     if (recon_tile_blocks(w, h, 10, 2) <= sms) return 1;
     if (recon_tile_blocks(w, h, 12, 2) <= sms) return 2;
     if (recon_tile_blocks(w, h, 20, 3) <= sms) return 3;

@@ -546,8 +546,10 @@ __global__ void __launch_bounds__(kThreads) k_tc_wgrad(int M, int N, int K, int 
 // outputs; the buffers have kConvMargin positions before and after their planes
 // for them.
 //
-// What it waits for is its own prologue and epilogue, so three CTAs of 256 positions
-// fit on an SM rather than two of 512.  64 images of 160 x 90 through the network:
+// What it waits for is its own prologue and epilogue, so CTAs are kept small enough that
+// several fit on an SM (of 256 positions, 64 images of 160 x 90: three for 32 and 64
+// channels, four or five for the heads, two for 96, whose accumulators take 256 of 512
+// TMEM columns) rather than one or two of 512.  64 images of 160 x 90 through the network:
 // as [position][C], whose slabs came by 2D TMA boxes with rows of 16 bytes, 0.70
 // ms with at most 512 positions per CTA; planar 0.59, with the epilogue by 16
 // columns 0.55, with at most 256 positions 0.53, with 128 0.65.
